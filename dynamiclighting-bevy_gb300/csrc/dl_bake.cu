@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "dl_bvh.hpp"
+#include "dl_bvh_rules.hpp"
 #include "dl_kernels.cuh"
 
 namespace dl {
@@ -2033,7 +2034,14 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
             std::memcpy(&occ, &h.tris[k * 12 + 3], 4);
             occ_leaf[occ] = k;
         }
-        up(h.nodes.data(), h.nodes.size() * sizeof(BvhNode), sc.nodes);
+        std::vector<TravNode> nodes(h.nodes.size());
+        for (size_t i = 0; i < nodes.size(); ++i) {
+            const BvhNode &b = h.nodes[i];
+            const float lo0[3] = {b.c0[0], b.c0[2], b.c2[0]}, hi0[3] = {b.c0[1], b.c0[3], b.c2[1]};
+            const float lo1[3] = {b.c1[0], b.c1[2], b.c2[2]}, hi1[3] = {b.c1[1], b.c1[3], b.c2[3]};
+            nodes[i] = trav_node(lo0, hi0, lo1, hi1, b.ref[0], b.ref[1]);
+        }
+        up(nodes.data(), nodes.size() * sizeof(TravNode), sc.nodes);
         up(h.tris.data(), h.tris.size() * 4, sc.tris);
         up(occ_leaf.data(), N * 4ull, sc.occ_leaf);
     } else {
@@ -2056,11 +2064,11 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
         }
         h.bvh_depth = db.depth;
         h.bvh_node_count = db.node_count;
-        sc.nodes = reinterpret_cast<const float4 *>(db.nodes);
+        sc.nodes = db.nodes;
         sc.tris = db.tris;
         sc.occ_leaf = db.occ_leaf;
         if (N == 0) {  // no occluders: small placeholders, which traversal never reads
-            sc.nodes = dev_alloc<float4>(s->owned, s->stream, 4, bytes, &s->budget);
+            sc.nodes = dev_alloc<TravNode>(s->owned, s->stream, 1, bytes, &s->budget);
             sc.tris = dev_alloc<float4>(s->owned, s->stream, 3, bytes, &s->budget);
             sc.occ_leaf = dev_alloc<uint32_t>(s->owned, s->stream, 1, bytes, &s->budget);
         }
@@ -3246,6 +3254,79 @@ dl_status encode_device(dl_session &s, uint8_t *&bytes, uint64_t &length, uint32
     return DL_OK;
 }
 
+// The occluder BVH's nodes with their boxes as planes, for dl_session_occluder_bvh. The device
+// holds centres and half extents, from which the planes do not follow exactly; they are minima and
+// maxima over the triangles below (padded), so they are taken again from the resident triangles,
+// children before parents (a node's index is below its children's).
+std::vector<BvhNode> plane_nodes(dl_session &s) {
+    const DevScene &sc = s.sc;
+    const HostScene &h = s.host;
+    const uint32_t count = h.bvh_node_count, M = sc.mesh_count;
+    std::vector<TravNode> dev(count);
+    std::vector<float> tris((size_t)sc.occluders * 12);
+    std::vector<uint32_t> vbase(M + 1), ibase(M + 1);
+    CK(cudaMemcpy(dev.data(), sc.nodes, count * sizeof(TravNode), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(tris.data(), sc.tris, tris.size() * 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(vbase.data(), sc.mesh_vertex_base, (M + 1) * 4ull, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(ibase.data(), sc.mesh_index_base, (M + 1) * 4ull, cudaMemcpyDeviceToHost));
+    std::vector<float> pos((size_t)vbase[M] * 3);
+    std::vector<uint32_t> idx(ibase[M]);
+    CK(cudaMemcpy(pos.data(), sc.positions, pos.size() * 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(idx.data(), sc.indices, idx.size() * 4, cudaMemcpyDeviceToHost));
+    struct Box {
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        void add(const float *l, const float *u) {
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = bvh_min(lo[a], l[a]);
+                hi[a] = bvh_max(hi[a], u[a]);
+            }
+        }
+    };
+    std::vector<Box> all(count);  // each node's children together
+    std::vector<BvhNode> out(count);
+    for (uint32_t i = count; i-- > 0;) {
+        Box b[2];
+        for (int c = 0; c < 2; ++c) {
+            const int32_t ref = dev[i].ref[c];
+            if (ref >= 0) {
+                b[c] = all[ref];
+            } else {
+                const uint32_t packed = (uint32_t)~ref;
+                for (uint32_t k = packed >> 3; k < (packed >> 3) + (packed & 7u); ++k) {
+                    uint32_t occ;
+                    std::memcpy(&occ, &tris[(size_t)k * 12 + 3], 4);
+                    const uint32_t m = h.occ_mesh[occ], *v = &idx[ibase[m] + (size_t)h.occ_tri[occ] * 3];
+                    for (int j = 0; j < 3; ++j) {
+                        const float *p = &pos[(size_t)(vbase[m] + v[j]) * 3];
+                        b[c].add(p, p);
+                    }
+                }
+            }
+            all[i].add(b[c].lo, b[c].hi);
+            if (ref == ~0) {
+                for (int a = 0; a < 3; ++a) {
+                    b[c].lo[a] = 1e30f;
+                    b[c].hi[a] = -1e30f;
+                }
+            } else {
+                bvh_pad_box(b[c].lo, b[c].hi);
+            }
+        }
+        BvhNode &n = out[i];
+        n = BvhNode{};
+        for (int a = 0; a < 2; ++a) {
+            n.c0[2 * a] = b[0].lo[a];
+            n.c0[2 * a + 1] = b[0].hi[a];
+            n.c1[2 * a] = b[1].lo[a];
+            n.c1[2 * a + 1] = b[1].hi[a];
+            n.c2[2 * a] = b[a].lo[2];
+            n.c2[2 * a + 1] = b[a].hi[2];
+            n.ref[a] = dev[i].ref[a];
+        }
+    }
+    return out;
+}
+
 dl_status result(dl_session &s, dl_baked_scene *&out) {
     std::unique_ptr<HostResult> r;
     dl_status st = assemble(s, r, true);
@@ -3424,7 +3505,11 @@ dl_status dl_session_occluder_bvh(dl_session *s, void *nodes, uint64_t node_cap,
     DL_GUARD({
         CK(cudaSetDevice(s->device));
         uint64_t n = std::min<uint64_t>(node_cap, h.bvh_node_count);
-        if (n) CK(cudaMemcpy(nodes, s->sc.nodes, n * sizeof(BvhNode), cudaMemcpyDeviceToHost));
+        if (n && !h.nodes.empty()) std::memcpy(nodes, h.nodes.data(), n * sizeof(BvhNode));
+        else if (n) {
+            const std::vector<BvhNode> boxes = plane_nodes(*s);
+            std::memcpy(nodes, boxes.data(), n * sizeof(BvhNode));
+        }
         uint64_t t = std::min<uint64_t>(tri_cap, s->sc.occluders);
         if (t) CK(cudaMemcpy(triangles, s->sc.tris, t * 3 * sizeof(float4), cudaMemcpyDeviceToHost));
         return DL_OK;

@@ -633,7 +633,7 @@ __device__ __forceinline__ int32_t child_ref(const Layout &L, int32_t kid) {
     return c.inner ? (int32_t)L.pos[kid] : ~(int32_t)((c.first << 3) | c.count);
 }
 
-__global__ void k_emit(Layout L, BvhNode *out) {
+__global__ void k_emit(Layout L, TravNode *out) {
     uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= L.total) return;
     const TNode &n = L.nodes[id];
@@ -641,13 +641,8 @@ __global__ void k_emit(Layout L, BvhNode *out) {
         // the whole set is one leaf: the root holds it and an empty second child
         float lo[3] = {n.lo[0], n.lo[1], n.lo[2]}, hi[3] = {n.hi[0], n.hi[1], n.hi[2]};
         bvh_pad_box(lo, hi);
-        BvhNode r{};
-        r.c0[0] = lo[0]; r.c0[1] = hi[0]; r.c0[2] = lo[1]; r.c0[3] = hi[1];
-        r.c1[0] = 1e30f; r.c1[1] = -1e30f; r.c1[2] = 1e30f; r.c1[3] = -1e30f;
-        r.c2[0] = lo[2]; r.c2[1] = hi[2]; r.c2[2] = 1e30f; r.c2[3] = -1e30f;
-        r.ref[0] = ~(int32_t)((n.first << 3) | n.count);
-        r.ref[1] = ~0;
-        out[0] = r;
+        const float elo[3] = {1e30f, 1e30f, 1e30f}, ehi[3] = {-1e30f, -1e30f, -1e30f};
+        out[0] = trav_node(lo, hi, elo, ehi, ~(int32_t)((n.first << 3) | n.count), ~0);
         return;
     }
     if (!n.inner) return;
@@ -656,13 +651,7 @@ __global__ void k_emit(Layout L, BvhNode *out) {
     float rlo[3] = {r.lo[0], r.lo[1], r.lo[2]}, rhi[3] = {r.hi[0], r.hi[1], r.hi[2]};
     bvh_pad_box(llo, lhi);
     bvh_pad_box(rlo, rhi);
-    BvhNode b{};
-    b.c0[0] = llo[0]; b.c0[1] = lhi[0]; b.c0[2] = llo[1]; b.c0[3] = lhi[1];
-    b.c1[0] = rlo[0]; b.c1[1] = rhi[0]; b.c1[2] = rlo[1]; b.c1[3] = rhi[1];
-    b.c2[0] = llo[2]; b.c2[1] = lhi[2]; b.c2[2] = rlo[2]; b.c2[3] = rhi[2];
-    b.ref[0] = child_ref(L, n.kid[0]);
-    b.ref[1] = child_ref(L, n.kid[1]);
-    out[L.pos[id]] = b;
+    out[L.pos[id]] = trav_node(llo, lhi, rlo, rhi, child_ref(L, n.kid[0]), child_ref(L, n.kid[1]));
 }
 
 // Triangles in leaf order: v0 (occluder index bits in w), e1 = v1 - v0, e2 = v2 - v0.
@@ -843,7 +832,7 @@ void build_bvh_device(const DeviceBvhInput &in, const std::function<void *(size_
         BK(cudaStreamSynchronize(stream));
     }
     out.node_count = inner;
-    out.nodes = static_cast<BvhNode *>(alloc((size_t)inner * sizeof(BvhNode)));
+    out.nodes = static_cast<TravNode *>(alloc((size_t)inner * sizeof(TravNode)));
     out.tris = static_cast<float4 *>(alloc((size_t)n * 3 * sizeof(float4)));
     out.occ_leaf = static_cast<uint32_t *>(alloc((size_t)n * 4));
     k_emit<<<g, kThreads, 0, stream>>>(L, out.nodes);

@@ -9,6 +9,7 @@
 #include <functional>
 
 #include "dl_host.hpp"
+#include "dl_slab.hpp"
 
 namespace dl {
 
@@ -24,7 +25,7 @@ struct DeviceBvhInput {
 };
 
 struct DeviceBvh {
-    BvhNode *nodes = nullptr;  // depth-first, the root first, each left subtree before its right one
+    TravNode *nodes = nullptr;  // depth-first, the root first, each left subtree before its right one
     float4 *tris = nullptr;    // leaf order, 3 per triangle: v0 (w: occluder bits), e1, e2
     uint32_t *occ_leaf = nullptr;  // occluder -> its slot in leaf order
     uint32_t node_count = 0;

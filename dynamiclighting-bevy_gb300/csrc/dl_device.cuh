@@ -11,13 +11,14 @@
 
 #include "dl_host.hpp"
 #include "dl_math.cuh"
+#include "dl_slab.hpp"
 
 namespace dl {
 
 // Everything the kernels read, as device pointers (one struct passed by value).
 struct DevScene {
     // BVH and triangles in leaf order
-    const float4 *nodes;  // 4 float4 per node
+    const TravNode *nodes;
     // triangles as 3 float4 each, one 48-byte record per triangle (a leaf's triangles are
     // contiguous): v0 (w: occluder index bits), e1 = v1 - v0, e2 = v2 - v0
     const float4 *tris;
@@ -197,34 +198,22 @@ __device__ __forceinline__ bool tri_test_refined(const DevScene &sc, float4 v0, 
 
 constexpr int kStack = 64;  // >= BVH depth; the host refuses deeper trees
 
-// Slab test of both children of a node against the ray [0, tmax]. Boxes are padded on the host
-// and the exit distance gets a relative slack, so the test only ever errs towards visiting.
-__device__ __forceinline__ void box2(const float4 &a, const float4 &b, const float4 &c, f3 inv, f3 oinv, float tmax,
-                                     bool &h0, bool &h1, float &n0, float &n1) {
-    float lx0 = __fmaf_rn(a.x, inv.x, -oinv.x), hx0 = __fmaf_rn(a.y, inv.x, -oinv.x);
-    float ly0 = __fmaf_rn(a.z, inv.y, -oinv.y), hy0 = __fmaf_rn(a.w, inv.y, -oinv.y);
-    float lz0 = __fmaf_rn(c.x, inv.z, -oinv.z), hz0 = __fmaf_rn(c.y, inv.z, -oinv.z);
-    float lx1 = __fmaf_rn(b.x, inv.x, -oinv.x), hx1 = __fmaf_rn(b.y, inv.x, -oinv.x);
-    float ly1 = __fmaf_rn(b.z, inv.y, -oinv.y), hy1 = __fmaf_rn(b.w, inv.y, -oinv.y);
-    float lz1 = __fmaf_rn(c.z, inv.z, -oinv.z), hz1 = __fmaf_rn(c.w, inv.z, -oinv.z);
-    float en0 = fmaxf(fmaxf(fminf(lx0, hx0), fminf(ly0, hy0)), fmaxf(fminf(lz0, hz0), 0.0f));
-    float ex0 = fminf(fminf(fmaxf(lx0, hx0), fmaxf(ly0, hy0)), fminf(fmaxf(lz0, hz0), tmax));
-    float en1 = fmaxf(fmaxf(fminf(lx1, hx1), fminf(ly1, hy1)), fmaxf(fminf(lz1, hz1), 0.0f));
-    float ex1 = fminf(fminf(fmaxf(lx1, hx1), fmaxf(ly1, hy1)), fminf(fmaxf(lz1, hz1), tmax));
-    const float slack = 1.0f + 2.0e-6f;
-    h0 = en0 <= ex0 * slack;
-    h1 = en1 <= ex1 * slack;
-    n0 = en0;
-    n1 = en1;
-}
-
-// The reciprocal direction for the slab tests. It only prunes, so the fast reciprocal (within
-// 2 ulp) serves: each axis' slab distances all scale by one factor within 2^-22 of 1, so entry
-// and exit move by under 5e-7 of their value, inside box2's relative exit slack (2e-6).
-__device__ __forceinline__ f3 safe_inv(f3 d) {
-    return f3{__fdividef(1.0f, d.x == 0.0f ? copysignf(1e-30f, d.x) : d.x),
-              __fdividef(1.0f, d.y == 0.0f ? copysignf(1e-30f, d.y) : d.y),
-              __fdividef(1.0f, d.z == 0.0f ? copysignf(1e-30f, d.z) : d.z)};
+// A node's 64 bytes in two 32-byte loads.
+struct NodeData {
+    Pair c0, c1, h0, h1, cz, hz;
+    int ref0, ref1;
+};
+__device__ __forceinline__ NodeData load_node(const TravNode *n) {
+    NodeData d;
+    Pair refs, zero;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(d.c0), "=l"(d.c1), "=l"(d.h0), "=l"(d.h1)
+        : "l"(n));
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(d.cz), "=l"(d.hz), "=l"(refs), "=l"(zero)
+        : "l"(reinterpret_cast<const char *>(n) + 32));
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(d.ref0), "=r"(d.ref1) : "l"(refs));
+    return d;
 }
 
 // Any-hit (ANY) or closest-hit traversal of the BVH2. Child references: >= 0 an inner node,
@@ -240,8 +229,7 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
     hit.occluder = 0xFFFFFFFFu;
     if (sc.occluders == 0) return false;
     f3 d{dir.x + 0.0f, dir.y + 0.0f, dir.z + 0.0f};  // -0 -> +0 (occluder.rs:171-178)
-    f3 inv = safe_inv(d);
-    f3 oinv{o.x * inv.x, o.y * inv.y, o.z * inv.z};
+    const RaySlabs slabs = ray_slabs(o, d);
     float tmax = fmaxf(max, 0.0f);
     bool found = false;
     int sp = 0;
@@ -251,14 +239,14 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
     // loop body together instead of alternating node and leaf work per lane.
     for (;;) {
         while (ref >= 0) {
-            const float4 *nd = sc.nodes + (size_t)ref * 4;
-            float4 a = ldg4(nd), b = ldg4(nd + 1), c = ldg4(nd + 2), r = ldg4(nd + 3);
+            const NodeData nd = load_node(sc.nodes + ref);
             if (COUNT) ++vis->nodes;
             bool h0, h1;
             float n0, n1;
-            box2(a, b, c, inv, oinv, ANY ? tmax : fminf(tmax, hit.t), h0, h1, n0, n1);
+            slab_pair(nd.c0, nd.c1, nd.h0, nd.h1, nd.cz, nd.hz, slabs, ANY ? tmax : fminf(tmax, hit.t), h0, h1, n0,
+                      n1);
             // an empty child (~0, only beside a root leaf) reads as a leaf of no triangles
-            int r0 = __float_as_int(r.x), r1 = __float_as_int(r.y);
+            const int r0 = nd.ref0, r1 = nd.ref1;
             if (h0 && h1) {
                 bool swap = n1 < n0;
                 stack[sp * stride] = swap ? r0 : r1;

@@ -44,7 +44,8 @@ enum : uint32_t {
     kLightArea = 16,
 };
 
-// Aila–Laine style BVH2 node: both children's boxes in the parent, 64 bytes.
+// Aila–Laine style BVH2 node: both children's boxes in the parent, 64 bytes, as the host builder
+// makes it and dl_session_occluder_bvh returns it (the traversal reads TravNode, dl_slab.hpp).
 // c0 = (l0.lo.x, l0.hi.x, l0.lo.y, l0.hi.y), c1 = same for child 1,
 // c2 = (l0.lo.z, l0.hi.z, l1.lo.z, l1.hi.z), c3 = (ref0, ref1, 0, 0) as int bits.
 // ref >= 0: inner node; ref < 0: leaf ~(first << 3 | count) over triangles [first, first + count);
