@@ -118,109 +118,136 @@ __global__ void k_region_words(const uint32_t *region_rect, const DevLight *ligh
     words[e] = lights[e % L].shadow_bits == 1 ? (uint32_t)((n + 31) / 32) : (uint32_t)((n + 3) / 4);
 }
 
+// Index i of a row-major grid of width w as column and row; grids beyond 2^32 texels are rare, so
+// the division is a 32-bit one where it can be (the 64-bit one takes several times the instructions).
+__device__ __forceinline__ void grid_xy(uint64_t i, uint32_t w, uint32_t &x, uint32_t &y) {
+    if (i <= 0xFFFFFFFFull) {
+        y = (uint32_t)i / w;
+        x = (uint32_t)i - y * w;
+    } else {
+        y = (uint32_t)(i / w);
+        x = (uint32_t)(i % w);
+    }
+}
+
+// The kernels below take a warp (or a block) per triangle, pair, entry or region. With few of them
+// (a room of large walls) most of the chip would wait for a few warps that walk thousands of texels
+// each, so the launch adds a second grid dimension: part y of gridDim.y takes every gridDim.y-th
+// run of the job's texels (grid_parts). On the small room (72 triangles, 8 texels/m) k_crop took 367 us
+// with one part and 19 us so, k_pad_seams 152 us and 8 us, the three k_texels passes 208 us and 26 us,
+// the two k_unburied passes 80 us and 9 us (also from 32-bit index divisions).
+
 // ================================ texels ===============================================
 
+// Slots for a warp's `n` texels of triangle t: parts of a triangle share a cursor. The order of a
+// triangle's texels does not matter to any result (a texel's streams are keyed by its coordinates).
+__device__ __forceinline__ uint32_t take_slots(uint32_t *cursor, uint32_t t, uint32_t n, uint32_t &local) {
+    if (gridDim.y == 1) {
+        const uint32_t at = local;
+        local += n;
+        return at;
+    }
+    uint32_t at = 0;
+    if (lane_id() == 0 && n) at = atomicAdd(cursor + t, n);
+    return __shfl_sync(0xFFFFFFFFu, at, 0);
+}
+
 // MODE 0: count centered texels and set the owned grid; MODE 1: count touched texels;
-// MODE 2: write centered then touched texels at tex_off[t]. One warp per triangle.
+// MODE 2: write centered and touched texels from tex_off[t]. A warp per triangle and part; counts are
+// added to `count`, which starts at 0, as do the cursors.
 template <int MODE>
 __global__ void k_texels(DevScene sc, const float4 *tri_face, uint32_t *owned, const uint64_t *grid_off,
-                         uint32_t *count, const uint32_t *tex_off, uint32_t *tex_xy, float4 *tex_pos, float4 *tex_nrm,
-                         uint32_t *tex_tri) {
+                         uint32_t *count, uint32_t *cursor, const uint32_t *tex_off, uint32_t *tex_xy, float4 *tex_pos,
+                         float4 *tex_nrm, uint32_t *tex_tri) {
     uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     unsigned lane = lane_id();
     if (t >= sc.triangles) return;
     float4 f = tri_face[t];
-    if (f.w == 0.0f) {
-        if (MODE != 2 && lane == 0) count[t] = 0;
-        return;
-    }
+    if (f.w == 0.0f) return;
     f3 face{f.x, f.y, f.z};
     TriData d;
     load_tri(sc, t, d);
     uint32_t res = d.res;
     uint32_t *own = owned + grid_off[d.mesh];
-    uint32_t written = 0;
-    uint32_t out = MODE == 2 ? tex_off[t] : 0;
+    const uint64_t first = (uint64_t)blockIdx.y * 32, stride = (uint64_t)gridDim.y * 32;
+    uint32_t counted = 0, local = 0;
+    const uint32_t out = MODE == 2 ? tex_off[t] : 0;
+    auto write = [&](bool take, unsigned ballot, uint32_t x, uint32_t y, f3 wts) {
+        const uint32_t at = take_slots(cursor, t, __popc(ballot), local);
+        if (!take) return;
+        const uint32_t o = out + at + __popc(ballot & ((1u << lane) - 1u));
+        f3 pos, nrm;
+        surface_at(d, face, wts, pos, nrm);
+        tex_xy[o] = x | (y << 16);
+        tex_pos[o] = make_float4(pos.x, pos.y, pos.z, 0.0f);
+        tex_nrm[o] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
+        tex_tri[o] = t;
+    };
     if (MODE == 0 || MODE == 2) {
         Rect r = center_rect(d.uv, res, 0.0f);
         uint32_t w = r.max_x - r.min_x + 1;
         uint64_t n = (uint64_t)w * (r.max_y - r.min_y + 1);
-        for (uint64_t base = 0; base < n; base += 32) {
+        for (uint64_t base = first; base < n; base += stride) {
             uint64_t i = base + lane;
             bool inside = false;
             uint32_t x = 0, y = 0;
             f3 wts;
             if (i < n) {
-                x = r.min_x + (uint32_t)(i % w);
-                y = r.min_y + (uint32_t)(i / w);
+                grid_xy(i, w, x, y);
+                x += r.min_x;
+                y += r.min_y;
                 inside = uv_barycentrics(d.uv, texel_center(x, y, res), wts);
             }
             unsigned ballot = __ballot_sync(0xFFFFFFFFu, inside);
-            if (inside) {
-                if (MODE == 0) {
+            if (MODE == 0) {
+                if (inside) {
                     uint64_t bit = (uint64_t)x + (uint64_t)y * res;
                     atomicOr(own + bit / 32, 1u << (bit % 32));
-                } else {
-                    uint32_t o = out + written + __popc(ballot & ((1u << lane) - 1u));
-                    f3 pos, nrm;
-                    surface_at(d, face, wts, pos, nrm);
-                    tex_xy[o] = x | (y << 16);
-                    tex_pos[o] = make_float4(pos.x, pos.y, pos.z, 0.0f);
-                    tex_nrm[o] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
-                    tex_tri[o] = t;
                 }
+                counted += __popc(ballot);
+            } else {
+                write(inside, ballot, x, y, wts);
             }
-            written += __popc(ballot);
-        }
-        if (MODE == 0) {
-            if (lane == 0) count[t] = written;
-            return;
         }
     }
     // touched texels (texels.rs:78-121)
-    float s = (float)res;
-    f2 mn, mx;
-    uv_bounds(d.uv, mn, mx);
-    uint32_t x0 = f2u(fmaxf(floorf(mn.x * s), 0.0f)), y0 = f2u(fmaxf(floorf(mn.y * s), 0.0f));
-    uint32_t x1 = f2u(fminf(floorf(mx.x * s), s - 1.0f)), y1 = f2u(fminf(floorf(mx.y * s), s - 1.0f));
-    float half = 0.5f / s;
-    uint32_t touched = 0;
-    if (x1 >= x0 && y1 >= y0) {
-        uint32_t w = x1 - x0 + 1;
-        uint64_t n = (uint64_t)w * (y1 - y0 + 1);
-        for (uint64_t base = 0; base < n; base += 32) {
-            uint64_t i = base + lane;
-            bool take = false;
-            uint32_t x = 0, y = 0;
-            f3 wts;
-            if (i < n) {
-                x = x0 + (uint32_t)(i % w);
-                y = y0 + (uint32_t)(i / w);
-                uint64_t bit = (uint64_t)x + (uint64_t)y * res;
-                bool is_owned = (own[bit / 32] >> (bit % 32)) & 1u;
-                if (!is_owned) {
-                    f2 center = texel_center(x, y, res);
-                    if (nearest_weights(d.uv, center, wts)) {
-                        float nx = d.uv[0].x * wts.x + d.uv[1].x * wts.y + d.uv[2].x * wts.z;
-                        float ny = d.uv[0].y * wts.x + d.uv[1].y * wts.y + d.uv[2].y * wts.z;
-                        take = fmaxf(fabsf(nx - center.x), fabsf(ny - center.y)) <= half;
+    if (MODE != 0) {
+        float s = (float)res;
+        f2 mn, mx;
+        uv_bounds(d.uv, mn, mx);
+        uint32_t x0 = f2u(fmaxf(floorf(mn.x * s), 0.0f)), y0 = f2u(fmaxf(floorf(mn.y * s), 0.0f));
+        uint32_t x1 = f2u(fminf(floorf(mx.x * s), s - 1.0f)), y1 = f2u(fminf(floorf(mx.y * s), s - 1.0f));
+        float half = 0.5f / s;
+        if (x1 >= x0 && y1 >= y0) {
+            uint32_t w = x1 - x0 + 1;
+            uint64_t n = (uint64_t)w * (y1 - y0 + 1);
+            for (uint64_t base = first; base < n; base += stride) {
+                uint64_t i = base + lane;
+                bool take = false;
+                uint32_t x = 0, y = 0;
+                f3 wts;
+                if (i < n) {
+                    grid_xy(i, w, x, y);
+                    x += x0;
+                    y += y0;
+                    uint64_t bit = (uint64_t)x + (uint64_t)y * res;
+                    bool is_owned = (own[bit / 32] >> (bit % 32)) & 1u;
+                    if (!is_owned) {
+                        f2 center = texel_center(x, y, res);
+                        if (nearest_weights(d.uv, center, wts)) {
+                            float nx = d.uv[0].x * wts.x + d.uv[1].x * wts.y + d.uv[2].x * wts.z;
+                            float ny = d.uv[0].y * wts.x + d.uv[1].y * wts.y + d.uv[2].y * wts.z;
+                            take = fmaxf(fabsf(nx - center.x), fabsf(ny - center.y)) <= half;
+                        }
                     }
                 }
+                unsigned ballot = __ballot_sync(0xFFFFFFFFu, take);
+                if (MODE == 1) counted += __popc(ballot);
+                else write(take, ballot, x, y, wts);
             }
-            unsigned ballot = __ballot_sync(0xFFFFFFFFu, take);
-            if (MODE == 2 && take) {
-                uint32_t o = out + written + touched + __popc(ballot & ((1u << lane) - 1u));
-                f3 pos, nrm;
-                surface_at(d, face, wts, pos, nrm);
-                tex_xy[o] = x | (y << 16);
-                tex_pos[o] = make_float4(pos.x, pos.y, pos.z, 0.0f);
-                tex_nrm[o] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
-                tex_tri[o] = t;
-            }
-            touched += __popc(ballot);
         }
     }
-    if (MODE == 1 && lane == 0) count[t] = touched;
+    if (MODE != 2 && lane == 0 && counted) atomicAdd(count + t, counted);
 }
 
 // Burial test per texel (mesh_texels.rs:57-88). Buried texels are dropped from tracing.
@@ -248,37 +275,33 @@ __global__ void __launch_bounds__(kBlock) k_burial(DevScene sc, uint32_t texels,
     if (REFINE) add_retests(ctr, vis.retests);
 }
 
-__global__ void k_add_u32(const uint32_t *a, const uint32_t *b, uint32_t *c, uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) c[i] = a[i] + b[i];
-    if (i == n) c[i] = 0;
-}
-
-
-// Per triangle: how many of its texels are not buried (warp per triangle).
+// Per triangle: how many of its texels are not buried, then those texels (a warp per triangle and part).
 template <bool WRITE>
 __global__ void k_unburied(uint32_t triangles, const uint32_t *tex_off, const uint8_t *buried, uint32_t *count,
-                           const uint32_t *ctex_off, const uint32_t *tex_xy, const float4 *tex_pos,
+                           uint32_t *cursor, const uint32_t *ctex_off, const uint32_t *tex_xy, const float4 *tex_pos,
                            const float4 *tex_nrm, uint32_t *c_xy, float4 *c_pos, float4 *c_nrm) {
     uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     unsigned lane = lane_id();
     if (t >= triangles) return;
     uint32_t b = tex_off[t], e = tex_off[t + 1];
-    uint32_t kept = 0;
+    uint32_t kept = 0, local = 0;
     uint32_t out = WRITE ? ctex_off[t] : 0;
-    for (uint32_t base = b; base < e; base += 32) {
-        uint32_t i = base + lane;
+    for (uint64_t base = b + (uint64_t)blockIdx.y * 32; base < e; base += (uint64_t)gridDim.y * 32) {
+        const uint64_t i = base + lane;
         bool keep = i < e && !buried[i];
         unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
-        if (WRITE && keep) {
-            uint32_t o = out + kept + __popc(ballot & ((1u << lane) - 1u));
-            c_xy[o] = tex_xy[i];
-            c_pos[o] = tex_pos[i];
-            c_nrm[o] = tex_nrm[i];
+        if (WRITE) {
+            const uint32_t at = take_slots(cursor, t, __popc(ballot), local);
+            if (keep) {
+                uint32_t o = out + at + __popc(ballot & ((1u << lane) - 1u));
+                c_xy[o] = tex_xy[i];
+                c_pos[o] = tex_pos[i];
+                c_nrm[o] = tex_nrm[i];
+            }
         }
         kept += __popc(ballot);
     }
-    if (!WRITE && lane == 0) count[t] = kept;
+    if (!WRITE && lane == 0 && kept) atomicAdd(count + t, kept);
 }
 
 // ================================ visibility ===========================================
@@ -942,61 +965,130 @@ __global__ void k_bounce_scatter(DevScene sc, BounceArgs a, const uint32_t *regi
         map[idx] = make_float4(v.x, v.y, v.z, 0.0f);
 }
 
-// dilate then separable blur (bounce_map.rs:67-112) of one window per block; A holds the
-// scattered map on entry and B the filtered map on exit.
-__global__ void __launch_bounds__(256) k_bounce_filter(DevScene sc, const uint32_t *region_rect, const uint32_t *woff,
-                                                       const uint32_t *wsize, float4 *A, float4 *B, float w0, float w1,
-                                                       float w2, float w3, float w4, float w5, float w6, float wsum) {
-    size_t e = blockIdx.x;
-    if (!wsize[e]) return;
-    uint32_t m = (uint32_t)(e / sc.light_count);
-    uint32_t res = sc.mesh_res[m];
-    Rect w = bounce_window(region_rect + e * 4, res);
-    uint32_t ww = w.max_x - w.min_x + 1, wh = w.max_y - w.min_y + 1, n = ww * wh;
-    float4 *a = A + woff[e], *b = B + woff[e];
-    auto get = [&](const float4 *g, int64_t x, int64_t y) -> float4 {
-        if (x < (int64_t)w.min_x || y < (int64_t)w.min_y || x > (int64_t)w.max_x || y > (int64_t)w.max_y)
-            return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        return g[(size_t)(y - w.min_y) * ww + (x - w.min_x)];
-    };
-    const int order[9][2] = {{0, 0}, {-1, -1}, {0, -1}, {1, -1}, {-1, 0}, {1, 0}, {-1, 1}, {0, 1}, {1, 1}};
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        int64_t x = w.min_x + i % ww, y = w.min_y + i / ww;
-        float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (int k = 0; k < 9; ++k) {
-            float4 v = get(a, x + order[k][0], y + order[k][1]);
-            if (fmaxf(fmaxf(v.x, v.y), v.z) > 0.0f) {
-                out = v;
-                break;
-            }
-        }
-        b[i] = out;
+struct BlurWeights {
+    float w[7];
+    float sum;
+};
+
+// The bounce map's filter (bounce_map.rs:67-112) on a tile of kTileW x kTileH texels of a window of
+// w x h: the tile and a halo of 4 (3 of the blur, 1 of the dilation) into shared memory, the dilation
+// (:67-87: the first positive texel among itself and its 8 neighbours in a fixed order; outside the window
+// reads 0), then one blur pass across and one down (:92-112: sample coordinates clamped to the map,
+// reads outside the window are 0, sum in tap order, divided by the weights' sum). `clamp` holds the map's
+// first and last column (x, y) and row (z, w) in window coordinates. A window is read once, so
+// small ones are bound by launch latency and large ones by the passes' shared-memory reads: which
+// texels are positive is worked out once, as a bit mask per row, so that the dilation reads one
+// texel instead of nine, and a thread blurs kRun outputs in a row from one set of taps in registers.
+// For callers of the filter alone (k_noalloc_filter), three launches with their intermediates in global
+// memory took 12.3 us a call for 61 x 45 texels and 18.4 us for 512 x 512; one launch of tiles takes
+// 6.1 us and 12.3 us (3.9 us and 10.2 us on the device). Tiles of 16 rows took 5.7 us and 10.3 us on
+// the device: a small window then has too few blocks. In the bake (k_bounce_filter) a block per window,
+// its passes in global memory, took 397 us on a room of large walls and 643 us on a terrain tile;
+// tiles take 23 us and 40 us.
+constexpr int kTileW = 32, kTileH = 8, kTileThreads = 256, kRun = 4;
+constexpr int kRawW = kTileW + 8, kRawH = kTileH + 8, kWideW = kTileW + 6, kWideH = kTileH + 6;
+struct FilterTile {
+    float raw[kRawH][kRawW * 3], wide[kWideH][kWideW * 3], across[kWideH][kTileW * 3];
+    unsigned long long lit[kRawH];  // bit c: texel c of the row has a positive channel
+};
+template <class Load, class Store>
+__device__ __forceinline__ void filter_tile(FilterTile &s, int tx, int ty, int w, int h, int4 clamp,
+                                            const BlurWeights &bw, Load load, Store store) {
+    const int tid = threadIdx.x;
+#pragma unroll 3
+    for (int i = tid; i < kRawH * kRawW; i += kTileThreads) {
+        const int row = i / kRawW, c = i % kRawW, x = tx - 4 + c, y = ty - 4 + row;
+        float v[3] = {0.0f, 0.0f, 0.0f};
+        if (x >= 0 && x < w && y >= 0 && y < h) load(x, y, v);
+        for (int j = 0; j < 3; ++j) s.raw[row][c * 3 + j] = v[j];
     }
     __syncthreads();
-    const float wt[7] = {w0, w1, w2, w3, w4, w5, w6};
-    int64_t last = (int64_t)res - 1;
-    for (int pass = 0; pass < 2; ++pass) {
-        const float4 *src = pass == 0 ? b : a;
-        float4 *dst = pass == 0 ? a : b;
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            int64_t x = w.min_x + i % ww, y = w.min_y + i / ww;
-            float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-            for (int k = -3; k <= 3; ++k) {
-                int64_t qx = pass == 0 ? min(max(x + k, (int64_t)0), last) : x;
-                int64_t qy = pass == 0 ? y : min(max(y + k, (int64_t)0), last);
-                float4 v = get(src, qx, qy);
-                sx = sx + v.x * wt[k + 3];
-                sy = sy + v.y * wt[k + 3];
-                sz = sz + v.z * wt[k + 3];
-            }
-            dst[i] = make_float4(sx / wsum, sy / wsum, sz / wsum, 0.0f);
+    for (int row = tid >> 5; row < kRawH; row += kTileThreads / 32) {
+        const int lane = tid & 31;
+        const float *v = &s.raw[row][lane * 3], *u = &s.raw[row][(32 + (lane & 7)) * 3];
+        const unsigned low = __ballot_sync(0xFFFFFFFFu, fmaxf(fmaxf(v[0], v[1]), v[2]) > 0.0f);
+        const unsigned high = __ballot_sync(0xFFFFFFFFu, fmaxf(fmaxf(u[0], u[1]), u[2]) > 0.0f);
+        if (lane == 0) s.lit[row] = low | (unsigned long long)(high & 0xFFu) << 32;
+    }
+    __syncthreads();
+    for (int i = tid; i < kWideH * kWideW; i += kTileThreads) {
+        const int row = i / kWideW, c = i % kWideW;
+        const unsigned top = (unsigned)(s.lit[row] >> c) & 7u, mid = (unsigned)(s.lit[row + 1] >> c) & 7u,
+                       low = (unsigned)(s.lit[row + 2] >> c) & 7u;
+        // itself, the row above, left and right, the row below: the lowest bit is the first in order
+        const unsigned order = (mid >> 1 & 1u) | top << 1 | (mid & 1u) << 4 | (mid >> 2) << 5 | low << 6;
+        const int k = __ffs(order) - 1;  // -1: none
+        const int dy = k <= 0 ? 1 : k < 4 ? 0 : k < 6 ? 1 : 2;
+        const int dx = k <= 0 ? 1 : k < 4 ? k - 1 : k == 4 ? 0 : k == 5 ? 2 : k - 6;
+        const float *v = &s.raw[row + dy][(c + dx) * 3];
+        // zero outside the window too, so that the blur only clamps its taps to the map
+        const int x = tx - 3 + c, y = ty - 3 + row;
+        const bool none = k < 0 || x < 0 || x >= w || y < 0 || y >= h;
+        for (int j = 0; j < 3; ++j) s.wide[row][c * 3 + j] = none ? 0.0f : v[j];
+    }
+    __syncthreads();
+    // across: a thread takes kRun texels of one channel of a row, down: kRun rows of one column's channel
+    for (int i = tid; i < kWideH * 3 * (kTileW / kRun); i += kTileThreads) {
+        const int run = i % (kTileW / kRun), j = i / (kTileW / kRun) % 3, row = i / (kTileW / kRun * 3), c0 = run * kRun;
+        float tap[kRun + 6];
+#pragma unroll
+        for (int k = 0; k < kRun + 6; ++k)
+            tap[k] = s.wide[row][(min(max(tx + c0 + k - 3, clamp.x), clamp.y) - tx + 3) * 3 + j];
+#pragma unroll
+        for (int o = 0; o < kRun; ++o) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 7; ++k) sum = sum + tap[o + k] * bw.w[k];
+            s.across[row][(c0 + o) * 3 + j] = sum / bw.sum;
         }
+    }
+    __syncthreads();
+    for (int i = tid; i < kTileW * 3 * (kTileH / kRun); i += kTileThreads) {
+        const int c = i % (kTileW * 3), r0 = i / (kTileW * 3) * kRun;
+        if (tx + c / 3 >= w) continue;
+        float tap[kRun + 6];
+#pragma unroll
+        for (int k = 0; k < kRun + 6; ++k) tap[k] = s.across[min(max(ty + r0 + k - 3, clamp.z), clamp.w) - ty + 3][c];
+#pragma unroll
+        for (int o = 0; o < kRun; ++o) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 7; ++k) sum = sum + tap[o + k] * bw.w[k];
+            if (ty + r0 + o < h) store(tx + c / 3, ty + r0 + o, c % 3, sum / bw.sum);
+        }
+    }
+}
+
+// The filter of every (mesh, light) window: the scattered map A into the filtered map B, a block per
+// window and part, tile by tile.
+__global__ void __launch_bounds__(kTileThreads) k_bounce_filter(DevScene sc, const uint32_t *region_rect,
+                                                                const uint32_t *woff, const uint32_t *wsize,
+                                                                const float4 *A, float4 *B, BlurWeights bw) {
+    __shared__ FilterTile tile;
+    const size_t e = blockIdx.x;
+    if (!wsize[e]) return;
+    const uint32_t res = sc.mesh_res[e / sc.light_count];
+    const Rect r = bounce_window(region_rect + e * 4, res);
+    const int w = (int)(r.max_x - r.min_x + 1), h = (int)(r.max_y - r.min_y + 1);
+    const int4 clamp = make_int4(-(int)r.min_x, (int)(res - 1 - r.min_x), -(int)r.min_y, (int)(res - 1 - r.min_y));
+    const float4 *a = A + woff[e];
+    float4 *b = B + woff[e];
+    const uint32_t across = (w + kTileW - 1) / kTileW, tiles = across * ((h + kTileH - 1) / kTileH);
+    for (uint32_t k = blockIdx.y; k < tiles; k += gridDim.y) {
+        filter_tile(tile, (int)(k % across) * kTileW, (int)(k / across) * kTileH, w, h, clamp, bw,
+                    [&](int x, int y, float v[3]) {
+                        const float4 q = a[(size_t)y * w + x];
+                        v[0] = q.x;
+                        v[1] = q.y;
+                        v[2] = q.z;
+                    },
+                    [&](int x, int y, int j, float v) { reinterpret_cast<float *>(b + (size_t)y * w + x)[j] = v; });
         __syncthreads();
     }
 }
 
-// BounceMap::crop's "lit" test (bounce_map.rs:124-136) per bounce pair: a warp scans the
-// triangle's crop in the filtered window.
+// BounceMap::crop's "lit" test (bounce_map.rs:124-136) per bounce pair: a warp per part scans the
+// triangle's crop in the filtered window; `pair_bounce` starts at 0.
 __global__ void k_bounce_lit(DevScene sc, BounceArgs a, const uint4 *tri_crop, const uint32_t *region_rect,
                              const uint32_t *woff, const float4 *map, uint8_t *pair_bounce) {
     uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1012,17 +1104,18 @@ __global__ void k_bounce_lit(DevScene sc, BounceArgs a, const uint4 *tri_crop, c
     uint32_t cw = c.z - c.x + 1;
     uint64_t n = (uint64_t)cw * (c.w - c.y + 1);
     bool lit = false;
-    for (uint64_t base = 0; base < n && !lit; base += 32) {
+    for (uint64_t base = (uint64_t)blockIdx.y * 32; base < n && !lit; base += (uint64_t)gridDim.y * 32) {
         uint64_t i = base + lane;
         bool l = false;
         if (i < n) {
-            uint32_t x = c.x + (uint32_t)(i % cw), y = c.y + (uint32_t)(i / cw);
-            float4 v = map[woff[e] + (size_t)(y - w.min_y) * ww + (x - w.min_x)];
+            uint32_t x, y;
+            grid_xy(i, cw, x, y);
+            float4 v = map[woff[e] + (size_t)(c.y + y - w.min_y) * ww + (c.x + x - w.min_x)];
             l = fmaxf(fmaxf(v.x, v.y), v.z) > 0.0f;
         }
         lit = __any_sync(0xFFFFFFFFu, l);
     }
-    if (lane == 0) pair_bounce[p] = lit;
+    if (lane == 0 && lit) pair_bounce[p] = 1;
 }
 
 __device__ __forceinline__ uint64_t bounce_words(uint4 crop, uint32_t bits, bool colored) {
@@ -1099,8 +1192,8 @@ __global__ void k_pack_bounce(DevScene sc, uint32_t entries, const uint32_t *ent
 }
 
 // pack_bounce(_rgb) for 8-bit bounce (bounce_pack.rs:28-86), which has no dither (its amplitude
-// is 0, so no random draw is taken): every pixel quantizes on its own, so a warp packs one entry,
-// each lane four consecutive pixels — one word of four 8-bit pixels, or three words of four
+// is 0, so no random draw is taken): every pixel quantizes on its own, so a warp packs an entry's
+// part, each lane four consecutive pixels — one word of four 8-bit pixels, or three words of four
 // 24-bit RGB pixels — in the padded crop grid's row-major order, as the sequential packer does.
 __global__ void k_pack_bounce8(DevScene sc, uint32_t entries, const uint32_t *entry_pair,
                                const unsigned long long *entry_bdst, const uint32_t *pair_tri,
@@ -1122,12 +1215,14 @@ __global__ void k_pack_bounce8(DevScene sc, uint32_t entries, const uint32_t *en
     const bool colored = sc.colored_bounce != 0;
     const uint64_t nwords = colored ? (n * 24 + 31) / 32 : (n + 3) / 4;
     Pcg none{0, 0};  // never drawn from at 8 bits
-    for (uint64_t g = lane; g * 4 < n; g += 32) {
+    for (uint64_t g = lane + (uint64_t)blockIdx.y * 32; g * 4 < n; g += (uint64_t)gridDim.y * 32) {
         uint32_t px[4];
         for (int k = 0; k < 4; ++k) {
             const uint64_t i = g * 4 + k;
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const int gx = (int)(i % gw), gy = (int)(i / gw);
+            uint32_t ux, uy;
+            grid_xy(i, (uint32_t)gw, ux, uy);
+            const int gx = (int)ux, gy = (int)uy;
             if (i < n && gx >= 2 && gy >= 2 && gx < gw - 2 && gy < gh - 2) {
                 const uint32_t x = c.x + gx - 2, y = c.y + gy - 2;
                 v = map[base + (size_t)(y - w.min_y) * ww + (x - w.min_x)];
@@ -1159,22 +1254,20 @@ __device__ __forceinline__ uint32_t region_get(const uint32_t *pool, uint32_t of
     return (pool[off + idx / 4] >> ((idx % 4) * 8)) & 0xFFu;
 }
 
-// LightEntries::optimize (shadows.rs:54-73) + any_light (:136-144): a warp per pair scans the
-// triangle's optimize rect within the light's region for any lit texel; marks used regions and
-// counts kept entries per triangle.
+// LightEntries::optimize (shadows.rs:54-73) + any_light (:136-144): a warp per pair and part scans the
+// triangle's optimize rect within the light's region for any lit texel; `keep` starts at 0.
 __global__ void k_optimize(DevScene sc, uint32_t pairs, const uint32_t *pair_tri, const uint32_t *pair_light,
                            const uint32_t *region_rect, const uint32_t *region_off, const uint32_t *region_pool,
-                           const uint8_t *pair_bounce, uint8_t *keep, uint32_t *kept_count, uint8_t *used,
-                           Counters *ctr) {
+                           const uint8_t *pair_bounce, uint8_t *keep) {
     uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     unsigned lane = lane_id();
     if (p >= pairs) return;
     uint32_t t = pair_tri[p], s = pair_light[p];
-    TriData d;
-    load_tri(sc, t, d);
-    size_t e = (size_t)d.mesh * sc.light_count + s;
     bool k = pair_bounce && pair_bounce[p];
     if (!k) {
+        TriData d;
+        load_tri(sc, t, d);
+        size_t e = (size_t)d.mesh * sc.light_count + s;
         Rect o = center_rect(d.uv, d.res, 1.0f);
         const uint32_t *r = region_rect + e * 4;
         uint32_t min_x = max(o.min_x, r[0]), max_x = min(o.max_x, r[2]);
@@ -1183,26 +1276,33 @@ __global__ void k_optimize(DevScene sc, uint32_t pairs, const uint32_t *pair_tri
             uint32_t w = max_x - min_x + 1;
             uint64_t n = (uint64_t)w * (max_y - min_y + 1);
             uint32_t bits = sc.lights[s].shadow_bits, roff = region_off[e];
-            for (uint64_t base = 0; base < n && !k; base += 32) {
+            for (uint64_t base = (uint64_t)blockIdx.y * 32; base < n && !k; base += (uint64_t)gridDim.y * 32) {
                 uint64_t i = base + lane;
-                bool lit = i < n && region_get(region_pool, roff, r, bits, min_x + (uint32_t)(i % w),
-                                               min_y + (uint32_t)(i / w)) != 0;
+                uint32_t x = 0, y = 0;
+                if (i < n) grid_xy(i, w, x, y);
+                bool lit = i < n && region_get(region_pool, roff, r, bits, min_x + x, min_y + y) != 0;
                 k = __any_sync(0xFFFFFFFFu, lit);
             }
         }
     }
-    if (lane == 0) {
-        keep[p] = k;
-        if (k) {
-            used[e] = 1;
-            atomicAdd(kept_count + t, 1u);
-        } else {
-            atomicAdd(&ctr->lights_removed, 1ull);
-        }
+    if (lane == 0 && k) keep[p] = 1;
+}
+// Marks the kept pairs' regions as used and counts the kept entries per triangle.
+__global__ void k_kept(DevScene sc, uint32_t pairs, const uint32_t *pair_tri, const uint32_t *pair_light,
+                       const uint8_t *keep, uint32_t *kept_count, uint8_t *used, Counters *ctr) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = p < pairs, kept = in && keep[p];
+    if (kept) {
+        const uint32_t t = pair_tri[p];
+        used[(size_t)sc.tri_mesh[t] * sc.light_count + pair_light[p]] = 1;
+        atomicAdd(kept_count + t, 1u);
     }
+    const unsigned removed = __ballot_sync(0xFFFFFFFFu, in && !kept);
+    if (lane_id() == 0 && removed) atomicAdd(&ctr->lights_removed, (unsigned long long)__popc(removed));
 }
 
-// pad_seams (seams.rs:15-39) on every used region; a block per (mesh, light) entry.
+// pad_seams (seams.rs:15-39) on every used region; a block per (mesh, light) entry and part. It reads
+// visited texels and writes the others, so parts do not meet.
 __global__ void k_pad_seams(DevScene sc, const uint8_t *used, const uint32_t *region_rect, const uint32_t *region_off,
                             uint32_t *region_pool, const uint32_t *visited, const uint64_t *grid_off) {
     size_t e = blockIdx.x;
@@ -1220,8 +1320,11 @@ __global__ void k_pad_seams(DevScene sc, const uint8_t *used, const uint32_t *re
         return (vis[bit / 32] >> (bit % 32)) & 1u;
     };
     const int dxs[4] = {-1, 1, 0, 0}, dys[4] = {0, 0, -1, 1};
-    for (uint64_t i = threadIdx.x; i < (uint64_t)w * h; i += blockDim.x) {
-        int64_t x = r[0] + (int64_t)(i % w), y = r[1] + (int64_t)(i / w);
+    const uint64_t n = (uint64_t)w * h, stride = (uint64_t)gridDim.y * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += stride) {
+        uint32_t ux, uy;
+        grid_xy(i, w, ux, uy);
+        int64_t x = (int64_t)r[0] + ux, y = (int64_t)r[1] + uy;
         if (visited_at(x, y)) continue;
         uint32_t level = 0;
         for (int k = 0; k < 4; ++k) {
@@ -1366,9 +1469,19 @@ __device__ __forceinline__ uint32_t crop_level(const uint32_t *pool, uint32_t of
 constexpr int kCropBytes = 2048;  // per-warp staging grid in shared memory (texels)
 
 // 1-bit words LSB first (bits.rs:40-46): word w holds texels 32w .. 32w + 31, so lane j's texel of
-// word w is bit j of a warp ballot. Each round of 32 words ends with one coalesced store per lane.
+// word w is bit j of a warp ballot. A warp alone ends each round of 32 words with one coalesced store
+// per lane; parts take single words, every parts-th one.
 template <class Texel>
-__device__ __forceinline__ void ballot_words(uint64_t n, uint64_t nw, uint32_t *out, unsigned lane, Texel texel) {
+__device__ __forceinline__ void ballot_words(uint64_t n, uint64_t nw, uint32_t *out, unsigned lane, uint32_t part,
+                                             uint32_t parts, Texel texel) {
+    if (parts > 1) {
+        for (uint64_t w = part; w < nw; w += parts) {
+            const uint64_t i = w * 32 + lane;
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, i < n && texel(i) != 0);
+            if (lane == 0) out[w] = b;
+        }
+        return;
+    }
     for (uint64_t base = 0; base < nw; base += 32) {
         uint32_t mine = 0;
         for (uint32_t k = 0; k < 32 && base + k < nw; ++k) {
@@ -1404,25 +1517,30 @@ __global__ void __launch_bounds__(kBlock) k_crop(DevScene sc, uint32_t entries, 
     uint64_t nw = (n + per - 1) / per;
     unsigned long long dst = entry_dst[e];
     if (n > (uint64_t)kCropBytes) {
-        // large crops: every texel straight from the region
+        // large crops: every texel straight from the region, the words shared by the parts
         if (bits == 1) {
-            ballot_words(n, nw, words + dst, lane, [&](uint64_t i) {
-                return crop_level(region_pool, off, r, bits, c, gw, gh, (int)(i % gw), (int)(i / gw));
+            ballot_words(n, nw, words + dst, lane, blockIdx.y, gridDim.y, [&](uint64_t i) {
+                uint32_t x, y;
+                grid_xy(i, (uint32_t)gw, x, y);
+                return crop_level(region_pool, off, r, bits, c, gw, gh, (int)x, (int)y);
             });
             return;
         }
-        for (uint64_t wi = lane; wi < nw; wi += 32) {
-            uint32_t word = 0;
-            for (uint32_t j = 0; j < per; ++j) {
-                uint64_t i = wi * per + j;
-                if (i >= n) break;
-                uint32_t v = crop_level(region_pool, off, r, bits, c, gw, gh, (int)(i % gw), (int)(i / gw));
-                word |= (bits == 1 ? (v != 0) : v) << (j * bits);
+        for (uint64_t wi = (uint64_t)blockIdx.y * 32 + lane; wi < nw; wi += (uint64_t)gridDim.y * 32) {
+            uint32_t word = 0, x, y;
+            grid_xy(wi * per, (uint32_t)gw, x, y);
+            for (uint32_t j = 0; j < per && wi * per + j < n; ++j) {
+                word |= crop_level(region_pool, off, r, bits, c, gw, gh, (int)x, (int)y) << (j * bits);
+                if (++x == (uint32_t)gw) {
+                    x = 0;
+                    ++y;
+                }
             }
             words[dst + wi] = word;
         }
         return;
     }
+    if (blockIdx.y) return;  // one part takes a small crop whole
     auto interior = [&](int x, int y) { return x >= 2 && y >= 2 && x < gw - 2 && y < gh - 2; };
     auto outer = [&](int x, int y) { return x == 0 || y == 0 || x == gw - 1 || y == gh - 1; };
     // the crop: interior texels from the region, padding rings zero
@@ -1459,7 +1577,7 @@ __global__ void __launch_bounds__(kBlock) k_crop(DevScene sc, uint32_t entries, 
     }
     __syncwarp();
     if (bits == 1) {
-        ballot_words(n, nw, words + dst, lane, [&](uint64_t i) { return (uint32_t)g[i]; });
+        ballot_words(n, nw, words + dst, lane, 0, 1, [&](uint64_t i) { return (uint32_t)g[i]; });
         return;
     }
     for (uint64_t wi = lane; wi < nw; wi += 32) {
@@ -1743,6 +1861,15 @@ T read_back(dl_session &s, const T *p) {
     return v;
 }
 unsigned grid_for(size_t n, unsigned block = kBlock) { return (unsigned)std::max<size_t>(1, (n + block - 1) / block); }
+// Grid of `jobs` jobs of `threads` threads each, with parts (second dimension) while the jobs alone
+// leave the chip short of warps: up to kParts, aiming at kPartThreads threads (a few times what
+// the SMs hold: parts of jobs that turn out small end at once).
+// Most (mesh, light) entries have no region: for them the parts are counted as if a warp took an entry.
+constexpr size_t kParts = 64, kPartThreads = 1u << 20;
+dim3 grid_parts(size_t jobs, unsigned threads = 32, unsigned block = kBlock) {
+    const size_t want = kPartThreads / std::max<size_t>(1, jobs * threads);
+    return dim3(grid_for(jobs * threads, block), (unsigned)std::min(kParts, std::max<size_t>(1, want)));
+}
 
 // Blocks the caller until the stream drains, forwarding a cancel request to the device flag. A
 // forwarded request's copy (on the side stream) is waited for too, so that it cannot land after
@@ -2581,23 +2708,19 @@ dl_status run(dl_session &s, dl_progress *progress) {
     uint32_t *visited = P.get<uint32_t>("visited", s.grid_words);
     CK(cudaMemsetAsync(owned, 0, s.grid_words * 4, st));
     CK(cudaMemsetAsync(visited, 0, s.grid_words * 4, st));
-    uint32_t *cen = P.get<uint32_t>("cen", T + 1);
-    uint32_t *tou = P.get<uint32_t>("tou", T + 1);
+    uint32_t *cursor = P.get<uint32_t>("cursor", T + 1);
     uint32_t *tex_cnt = P.get<uint32_t>("tex_cnt", T + 1);
     uint32_t *tex_off = P.get<uint32_t>("tex_off", T + 1);
-    const unsigned warp_grid = grid_for((size_t)T * 32);
-    if (T) {
-        k_texels<0><<<warp_grid, kBlock, 0, st>>>(sc, tri_face, owned, grid_off, cen, nullptr, nullptr, nullptr,
-                                                  nullptr, nullptr);
-        LAUNCHED("k_texels");
-        k_texels<1><<<warp_grid, kBlock, 0, st>>>(sc, tri_face, owned, grid_off, tou, nullptr, nullptr, nullptr,
-                                                  nullptr, nullptr);
-        LAUNCHED("k_texels");
-        s.launches += 2;
-    }
-    k_add_u32<<<grid_for(T + 1), kBlock, 0, st>>>(cen, tou, tex_cnt, T);
-    LAUNCHED("k_add_u32");
-    ++s.launches;
+    const dim3 warp_grid = grid_parts(T);
+    CK(cudaMemsetAsync(tex_cnt, 0, (T + 1) * 4ull, st));
+    CK(cudaMemsetAsync(cursor, 0, (T + 1) * 4ull, st));
+    k_texels<0><<<warp_grid, kBlock, 0, st>>>(sc, tri_face, owned, grid_off, tex_cnt, nullptr, nullptr, nullptr, nullptr,
+                                              nullptr, nullptr);
+    LAUNCHED("k_texels");
+    k_texels<1><<<warp_grid, kBlock, 0, st>>>(sc, tri_face, owned, grid_off, tex_cnt, nullptr, nullptr, nullptr, nullptr,
+                                              nullptr, nullptr);
+    LAUNCHED("k_texels");
+    s.launches += 2;
     scan_u32(s, tex_cnt, tex_off, T + 1);
     const uint32_t texels_all = read_back(s, tex_off + T);
     uint32_t *tex_xy = P.get<uint32_t>("tex_xy", texels_all);
@@ -2606,8 +2729,8 @@ dl_status run(dl_session &s, dl_progress *progress) {
     uint32_t *tex_tri = P.get<uint32_t>("tex_tri", texels_all);
     uint8_t *buried = P.get<uint8_t>("buried", texels_all);
     if (T) {
-        k_texels<2><<<warp_grid, kBlock, 0, st>>>(sc, tri_face, owned, grid_off, nullptr, tex_off, tex_xy, tex_pos,
-                                                  tex_nrm, tex_tri);
+        k_texels<2><<<warp_grid, kBlock, 0, st>>>(sc, tri_face, owned, grid_off, nullptr, cursor, tex_off, tex_xy,
+                                                  tex_pos, tex_nrm, tex_tri);
         LAUNCHED("k_texels");
         ++s.launches;
     }
@@ -2621,9 +2744,10 @@ dl_status run(dl_session &s, dl_progress *progress) {
     }
     uint32_t *ctex_cnt = P.get<uint32_t>("ctex_cnt", T + 1);
     uint32_t *ctex_off = P.get<uint32_t>("ctex_off", T + 1);
-    CK(cudaMemsetAsync(ctex_cnt + T, 0, 4, st));
+    CK(cudaMemsetAsync(ctex_cnt, 0, (T + 1) * 4ull, st));
+    CK(cudaMemsetAsync(cursor, 0, (T + 1) * 4ull, st));
     if (T) {
-        k_unburied<false><<<warp_grid, kBlock, 0, st>>>(T, tex_off, buried, ctex_cnt, nullptr, nullptr, nullptr,
+        k_unburied<false><<<warp_grid, kBlock, 0, st>>>(T, tex_off, buried, ctex_cnt, nullptr, nullptr, nullptr, nullptr,
                                                         nullptr, nullptr, nullptr, nullptr);
         LAUNCHED("k_unburied");
         ++s.launches;
@@ -2634,7 +2758,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
     float4 *ctex_pos = P.get<float4>("ctex_pos", texels);
     float4 *ctex_nrm = P.get<float4>("ctex_nrm", texels);
     if (T) {
-        k_unburied<true><<<warp_grid, kBlock, 0, st>>>(T, tex_off, buried, nullptr, ctex_off, tex_xy, tex_pos,
+        k_unburied<true><<<warp_grid, kBlock, 0, st>>>(T, tex_off, buried, nullptr, cursor, ctex_off, tex_xy, tex_pos,
                                                        tex_nrm, ctex_xy, ctex_pos, ctex_nrm);
         LAUNCHED("k_unburied");
         ++s.launches;
@@ -2845,12 +2969,14 @@ dl_status run(dl_session &s, dl_progress *progress) {
             LAUNCHED("k_bounce_scatter");
             s.launches += 2;
         }
-        const float *bw = hs.blur_weights;
-        k_bounce_filter<<<(unsigned)entries, 256, 0, st>>>(sc, region_rect, woff, wsize, mapA, bmap, bw[0], bw[1], bw[2],
-                                                           bw[3], bw[4], bw[5], bw[6], hs.blur_weight_sum);
+        BlurWeights bw;
+        std::copy(hs.blur_weights, hs.blur_weights + 7, bw.w);
+        bw.sum = hs.blur_weight_sum;
+        k_bounce_filter<<<dim3((unsigned)entries, grid_parts(entries).y), kTileThreads, 0, st>>>(
+            sc, region_rect, woff, wsize, mapA, bmap, bw);
         LAUNCHED("k_bounce_filter");
         if (bcount) {
-            k_bounce_lit<<<grid_for((size_t)bcount * 32), kBlock, 0, st>>>(sc, ba, tri_crop, region_rect, woff, bmap,
+            k_bounce_lit<<<grid_parts(bcount), kBlock, 0, st>>>(sc, ba, tri_crop, region_rect, woff, bmap,
                                                                            pair_bounce);
             LAUNCHED("k_bounce_lit");
             ++s.launches;
@@ -2867,14 +2993,16 @@ dl_status run(dl_session &s, dl_progress *progress) {
     CK(cudaMemsetAsync(used, 0, entries, st));
     CK(cudaMemsetAsync(kept_cnt, 0, (T + 1) * 4ull, st));
     if (pairs) {
-        k_optimize<<<grid_for((size_t)pairs * 32), kBlock, 0, st>>>(sc, pairs, pair_tri, pair_light, region_rect,
-                                                                    region_off, region_pool, pair_bounce, keep, kept_cnt,
-                                                                    used, s.ctr);
+        CK(cudaMemsetAsync(keep, 0, pairs, st));
+        k_optimize<<<grid_parts(pairs), kBlock, 0, st>>>(sc, pairs, pair_tri, pair_light, region_rect, region_off,
+                                                         region_pool, pair_bounce, keep);
         LAUNCHED("k_optimize");
-        ++s.launches;
+        k_kept<<<grid_for(pairs), kBlock, 0, st>>>(sc, pairs, pair_tri, pair_light, keep, kept_cnt, used, s.ctr);
+        LAUNCHED("k_kept");
+        s.launches += 2;
     }
     if (entries) {
-        k_pad_seams<<<(unsigned)entries, kBlock, 0, st>>>(sc, used, region_rect, region_off, region_pool, visited,
+        k_pad_seams<<<dim3((unsigned)entries, grid_parts(entries).y), kBlock, 0, st>>>(sc, used, region_rect, region_off, region_pool, visited,
                                                           grid_off);
         LAUNCHED("k_pad_seams");
         ++s.launches;
@@ -2914,7 +3042,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
         ++s.launches;
     }
     if (kept) {
-        k_crop<<<grid_for((size_t)kept * 32), kBlock, 0, st>>>(sc, kept, entry_pair, entry_dst, pair_tri, pair_light,
+        k_crop<<<grid_parts(kept), kBlock, 0, st>>>(sc, kept, entry_pair, entry_dst, pair_tri, pair_light,
                                                                tri_crop, region_rect, region_off, region_pool, words);
         LAUNCHED("k_crop");
         ++s.launches;
@@ -2922,7 +3050,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
             k_pack_bounce<<<grid_for(kept), kBlock, 0, st>>>(sc, kept, entry_pair, entry_bdst, pair_tri, pair_light,
                                                              tri_crop, region_rect, woff, bmap, words);
             LAUNCHED("k_pack_bounce");
-            k_pack_bounce8<<<grid_for((size_t)kept * 32), kBlock, 0, st>>>(
+            k_pack_bounce8<<<grid_parts(kept), kBlock, 0, st>>>(
                 sc, kept, entry_pair, entry_bdst, pair_tri, pair_light, tri_crop, region_rect, woff, bmap, words);
             LAUNCHED("k_pack_bounce8");
             s.launches += 2;
@@ -3632,75 +3760,26 @@ void dl_free(void *p) { std::free(p); }
 // separable blur; the body of k_bounce_filter) on one window held in caller-owned device
 // buffers, for callers that cannot allocate device memory — an engine applying the filter from
 // inside its own fixed memory budget, or from code that must not call cudaMalloc (while a
-// stream is being captured, or on a frame thread). The blur's intermediate lives in the
-// fixed array below, which every device that loads the library holds until the process exits.
+// stream is being captured, or on a frame thread). One launch, intermediates in shared memory.
 
 namespace dl {
 
 constexpr uint32_t kNoallocMaxTexels = DL_NOALLOC_MAX_TEXELS;
-static __device__ __align__(256) float g_noalloc_scratch[3 * (size_t)kNoallocMaxTexels];
 
 namespace {
 
 constexpr int kNoallocDevices = 64;
-std::mutex g_noalloc_mutex;
-float *g_noalloc_ptr[kNoallocDevices] = {};
 
-// Dilation (bounce_map.rs:67-87): the first positive texel among itself and its 8 neighbours in
-// a fixed order; outside the window reads 0.
-__global__ void k_noalloc_dilate(const float *in, float *out, uint32_t w, uint32_t h) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w * h) return;
-    int x = (int)(i % w), y = (int)(i / w);
-    const int order[9][2] = {{0, 0}, {-1, -1}, {0, -1}, {1, -1}, {-1, 0}, {1, 0}, {-1, 1}, {0, 1}, {1, 1}};
-    float r = 0.0f, g = 0.0f, b = 0.0f;
-    for (int k = 0; k < 9; ++k) {
-        int xx = x + order[k][0], yy = y + order[k][1];
-        if (xx < 0 || yy < 0 || xx >= (int)w || yy >= (int)h) continue;
-        const float *v = in + ((size_t)yy * w + xx) * 3;
-        if (fmaxf(fmaxf(v[0], v[1]), v[2]) > 0.0f) {
-            r = v[0];
-            g = v[1];
-            b = v[2];
-            break;
-        }
-    }
-    out[(size_t)i * 3] = r;
-    out[(size_t)i * 3 + 1] = g;
-    out[(size_t)i * 3 + 2] = b;
-}
-
-struct BlurWeights {
-    float w[7];
-    float sum;
-};
-
-// One blur pass (bounce_map.rs:92-112): sample coordinates clamped to the map, reads outside
-// the window are 0, sum in tap order, divided by the weights' sum.
-__global__ void k_noalloc_blur(const float *src, float *dst, uint32_t w, uint32_t h, uint32_t x0, uint32_t y0,
-                               uint32_t map_size, int vertical, BlurWeights bw) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w * h) return;
-    int64_t x = x0 + (int64_t)(i % w), y = y0 + (int64_t)(i / w);
-    int64_t last = (int64_t)map_size - 1;
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    for (int k = -3; k <= 3; ++k) {
-        int64_t qx = vertical ? x : min(max(x + k, (int64_t)0), last);
-        int64_t qy = vertical ? min(max(y + k, (int64_t)0), last) : y;
-        float r = 0.0f, g = 0.0f, b = 0.0f;
-        if (qx >= (int64_t)x0 && qy >= (int64_t)y0 && qx < (int64_t)x0 + w && qy < (int64_t)y0 + h) {
-            const float *v = src + ((size_t)(qy - y0) * w + (size_t)(qx - x0)) * 3;
-            r = v[0];
-            g = v[1];
-            b = v[2];
-        }
-        sx = sx + r * bw.w[k + 3];
-        sy = sy + g * bw.w[k + 3];
-        sz = sz + b * bw.w[k + 3];
-    }
-    dst[(size_t)i * 3] = sx / bw.sum;
-    dst[(size_t)i * 3 + 1] = sy / bw.sum;
-    dst[(size_t)i * 3 + 2] = sz / bw.sum;
+// A block filters a tile of the window (filter_tile).
+__global__ void __launch_bounds__(kTileThreads) k_noalloc_filter(const float *in, float *out, int w, int h, int4 clamp,
+                                                                 BlurWeights bw) {
+    __shared__ FilterTile tile;
+    filter_tile(tile, blockIdx.x * kTileW, blockIdx.y * kTileH, w, h, clamp, bw,
+                [&](int x, int y, float v[3]) {
+                    const float *q = in + ((size_t)y * w + x) * 3;
+                    for (int j = 0; j < 3; ++j) v[j] = q[j];
+                },
+                [&](int x, int y, int j, float v) { out[((size_t)y * w + x) * 3 + j] = v; });
 }
 
 // gaussian_weights(7, 5.0) (bounce_map.rs:140-151) in f32, exp rounded once from binary64.
@@ -3761,28 +3840,14 @@ extern "C" dl_status dl_filter_bounce_window_noalloc(const float *in_rgb, float 
                   ", the current device is " + std::to_string(device);
         return DL_UNSUPPORTED;
     }
-    float *scratch = nullptr;
-    {
-        // set-up, once per device, with that device current: the scratch array's device address
-        std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-        if (!g_noalloc_ptr[device]) {
-            e = cudaGetSymbolAddress((void **)&g_noalloc_ptr[device], g_noalloc_scratch);
-            if (e != cudaSuccess) {
-                g_noalloc_ptr[device] = nullptr;
-                g_error = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e);
-                return DL_CUDA_ERROR;
-            }
-        }
-        scratch = g_noalloc_ptr[device];
-    }
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    BlurWeights bw = blur_weights();
-    unsigned blocks = (unsigned)((n + 255) / 256);
-    // dilate into the output, blur across into the scratch, blur down into the output; every
-    // scratch texel is written before it is read, so nothing needs clearing between calls
-    k_noalloc_dilate<<<blocks, 256, 0, st>>>(in_rgb, out_rgb, width, height);
-    k_noalloc_blur<<<blocks, 256, 0, st>>>(out_rgb, scratch, width, height, x0, y0, map_size, 0, bw);
-    k_noalloc_blur<<<blocks, 256, 0, st>>>(scratch, out_rgb, width, height, x0, y0, map_size, 1, bw);
+    static const BlurWeights bw = blur_weights();
+    // the map's first and last column and row in window coordinates, as far as a tap can reach
+    const int far = (int)kNoallocMaxTexels + 64;
+    const int4 clamp = make_int4(-(int)std::min<uint32_t>(x0, 64), (int)std::min<uint32_t>(map_size - 1 - x0, far),
+                                 -(int)std::min<uint32_t>(y0, 64), (int)std::min<uint32_t>(map_size - 1 - y0, far));
+    const dim3 tiles((width + kTileW - 1) / kTileW, (height + kTileH - 1) / kTileH);
+    k_noalloc_filter<<<tiles, kTileThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        in_rgb, out_rgb, (int)width, (int)height, clamp, bw);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_error = std::string("bounce filter launch: ") + cudaGetErrorString(e);

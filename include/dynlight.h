@@ -412,13 +412,8 @@ void dl_free(void *pointer);
  * device (devices 0 to 63, else DL_UNSUPPORTED), enqueued on `stream` (a cudaStream_t, NULL for
  * the legacy default stream).
  *
- * The blur's intermediate lives in one fixed device array of DL_NOALLOC_MAX_TEXELS * 12 bytes
- * (3 MiB) that every device loading the library holds until the process exits. The first call on
- * a device looks up that array's address (cudaGetSymbolAddress) and keeps it; make that call
- * before any stream capture. A process that calls cudaDeviceReset on a device must not call this
- * entry point on that device afterwards: the kept address belongs to the context the reset ended.
- * All calls share the array: calls whose work overlaps on the GPU (concurrent streams, threads)
- * race on it, so serialize them. */
+ * One kernel launch, its intermediates in shared memory: calls on different streams and threads may
+ * overlap, and the first call may be captured like any other. */
 #define DL_NOALLOC_MAX_TEXELS (512u * 512u)
 dl_status dl_filter_bounce_window_noalloc(const float *in_rgb, float *out_rgb, uint32_t width, uint32_t height,
                                           uint32_t x0, uint32_t y0, uint32_t map_size, void *stream);
