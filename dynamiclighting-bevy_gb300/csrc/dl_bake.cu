@@ -2245,18 +2245,30 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 
 // The device pipeline of one bake. Reads back the sizes it needs between stages; everything
 // else stays on the device until dl_session_result.
-// ---- launch-shape autotuner of the batched visibility kernel ---------------------------------
-// Knobs: chunk size (warp-steps per claimed chunk), sky sample lanes (lanes sharing one sky
-// texel), the launch bound's blocks per SM (the register budget: 7, 8, 9, 10 or 12 blocks of 128
-// threads give 72, 64, 56, 48 or 40 registers per thread) and the stack depth (the BVH's depth,
-// rounded up; it sets the shared memory per block and so, with the registers, the resident
-// blocks). Each candidate runs on every k-th chunk of the real queue (k = 8 from 4 M items, 4
-// from 1 M) with scratch counters; its results are the same levels the real pass writes (OR and
-// max), so the trials change no output. Chunk size and lanes are tried at 8 blocks per SM, then
-// the other register budgets with the winning pair (more warps hide more of the traversal's L1
-// and L2 latency, fewer registers spill more: on the outdoor scene 12 blocks ran the visibility
-// stage in 135.7 ms, 9 in 137.8, 10 in 139.4, 8 in 141.9). The fastest shape is cached per
-// process, keyed by the device and the queue's shape.
+// ---- launch shapes of the batched visibility and gather kernels ---------------------------------
+// Knobs: chunk size (warp-steps per claimed chunk), lanes sharing one sky texel's or gathered texel's
+// samples, the launch bound's blocks per SM (the register budget: 7, 8, 9, 10 or 12 blocks of 128
+// threads give 72, 64, 56, 48 or 40 registers per thread; the gather's 6 gives 80) and the stack depth
+// (the BVH's depth, rounded up; it sets the shared memory per block and so, with the registers, the
+// resident blocks). A rule picks the shape:
+// - sky lanes grow with the sample count, 8 from 256 samples, 4 from 128, 2 from 64. Lanes that
+//   share a texel's aligned samples trace neighbouring directions, and few texels with long sample
+//   loops leave the last warps alone. Visibility of a terrain tile (0.5 M items, 256 samples) at 1, 2, 4,
+//   8, 16 lanes: 13.3, 10.7, 9.6, 9.4, 9.6 ms; of foliage (128 samples) 5.6, 3.1, 2.4, 2.3, 2.5 ms;
+//   of a room (64 samples) 0.39, 0.40, 0.43, 0.44, 0.46 ms.
+// - 10 blocks per SM with a sky, 8 without: the tile at 7, 8, 9, 10, 12 takes 10.1, 9.9, 9.6, 9.4, 9.5
+//   ms (sky rays wait on the tree's far nodes, more warps hide it), rooms under panels and tubes 7.0,
+//   6.9, 6.9, 7.0, 8.0 ms.
+// - gathers with a sun take 8 lanes at 9 blocks (tile, 1 to 32 lanes at 9: 11.8, 9.0, 8.1, 7.7, 7.8,
+//   8.2 ms; 6, 8, 9, 10 blocks at 8 lanes: 9.0, 8.0, 7.7, 7.8 ms), local ones alone 2 lanes at 8 (rooms:
+//   8.7, 8.7, 9.2, 10.0, 11.5, 15.9 ms), refined ones 4 lanes (terrain 63.4, 60.7, 59.3, 58.6, 58.3,
+//   58.4 ms, decals 31.2, 29.2, 29.3, 30.4, 32.4, 33.8 ms).
+// From 1 M visibility items (256 K gather items) the rule's neighbours are tried too, each on a small
+// share of the real queue's chunks with scratch counters; their results are the same levels and values
+// that the real pass writes (OR and max, and values that it overwrites), so the trials change no
+// output. Trials stay a small share of the first bake: the wide search this replaces took
+// up to 0.6 s of it and ended within 2 % of the rule. The choice is cached per process, keyed by the
+// device and the queue's shape.
 struct TraceTune {
     uint32_t grab = 1, sky_lanes = 1, minb = 7, stack_depth = kStack, blocks = 1, trials = 0;
     double ms = 0.0;
@@ -2299,21 +2311,23 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
+    const uint32_t n = s.options.sky_samples, sky_lanes = n >= 256 ? 8 : n >= 128 ? 4 : n >= 64 ? 2 : 1;
     std::vector<uint32_t> grabs = c.chunk_texels ? std::vector<uint32_t>{std::max(1u, c.chunk_texels / 32)}
                                                  : std::vector<uint32_t>{1, 2};
     std::vector<uint32_t> lanes = c.sample_lanes ? std::vector<uint32_t>{c.sample_lanes}
-                                  : ta.sky_items  ? std::vector<uint32_t>{1, 2, 4, 8, 16}
-                                                  : std::vector<uint32_t>{1};
-    // the chunk and lane trials run at the first budget; untuned launches take 7 blocks per SM
+                                  : !ta.sky_items ? std::vector<uint32_t>{1}
+                                  : sky_lanes > 1 ? std::vector<uint32_t>{sky_lanes, sky_lanes / 2}
+                                                  : std::vector<uint32_t>{1, 2};
     std::vector<uint32_t> minbs = (count || refine) ? std::vector<uint32_t>{7}
                                   : c.min_blocks    ? std::vector<uint32_t>{c.min_blocks}
-                                                    : std::vector<uint32_t>{8, 7, 9, 10, 12};
-    const uint32_t every = ta.items >= (4u << 20) ? 8 : ta.items >= (1u << 20) ? 4 : 0;
+                                  : ta.sky_items    ? std::vector<uint32_t>{10, 12}
+                                                    : std::vector<uint32_t>{8, 9};
+    const uint32_t every = ta.items >= (4u << 20) ? 32 : ta.items >= (1u << 20) ? 16 : 0;
     const bool tune = !c.no_autotune && every && grabs.size() * lanes.size() * minbs.size() > 1 &&
                       !(progress && progress->cancel);
     best.grab = grabs[0];
     best.sky_lanes = lanes[0];
-    best.minb = (count || refine || !c.min_blocks) ? 7u : c.min_blocks;
+    best.minb = minbs[0];
     if (!tune) {
         best.blocks = blocks_for(best.minb);
         return best;
@@ -2362,8 +2376,8 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
             best.blocks = blocks;
         }
     };
-    for (uint32_t w : lanes)
-        for (uint32_t g : grabs) trial(minbs[0], w, g);
+    for (uint32_t w : lanes) trial(minbs[0], w, grabs[0]);
+    for (size_t k = 1; k < grabs.size(); ++k) trial(minbs[0], best.sky_lanes, grabs[k]);
     const uint32_t w = best.sky_lanes, g = best.grab;
     for (size_t k = 1; k < minbs.size(); ++k) trial(minbs[k], w, g);
     cudaEventDestroy(a);
@@ -2428,18 +2442,21 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
+    bool sun = false;
+    for (const DevLight &l : s.host.lights) sun |= l.shape == DL_SHAPE_SUN && (l.flags & kLightBounce);
     std::vector<uint32_t> lanes = c.sample_lanes ? std::vector<uint32_t>{c.sample_lanes}
-                                                 : std::vector<uint32_t>{1, 4, 8, 16, 32};
-    // register budgets (blocks per SM: 6, 8, 9, 10 give 80, 64, 56, 48 registers per thread); the
-    // lane trials run at the first, the others with the two best lane counts
+                                  : refine        ? std::vector<uint32_t>{4, 8}
+                                  : sun           ? std::vector<uint32_t>{8, 4}
+                                                  : std::vector<uint32_t>{2, 1};
     std::vector<uint32_t> minbs = refine                ? std::vector<uint32_t>{8}
                                   : c.gather_min_blocks ? std::vector<uint32_t>{c.gather_min_blocks}
-                                                        : std::vector<uint32_t>{8, 6, 9, 10};
-    const uint32_t every = ba.items >= (1u << 20) ? 8 : ba.items >= (1u << 18) ? 4 : 0;
+                                  : sun                 ? std::vector<uint32_t>{9, 10}
+                                                        : std::vector<uint32_t>{8, 9};
+    const uint32_t every = ba.items >= (1u << 20) ? 32 : ba.items >= (1u << 18) ? 16 : 0;
     best.lanes = lanes[0];
-    // untuned: 6 blocks per SM; the refined gather always takes 8 (64 registers: 173 ms on the
-    // outdoor scene against 178 ms at 80 registers and 173 ms at 48, its binary64 re-tests spill)
-    best.minb = refine ? 8u : c.gather_min_blocks ? c.gather_min_blocks : 6u;
+    // the refined gather always takes 8 (64 registers: 173 ms on the outdoor scene against 178 ms at
+    // 80 registers and 173 ms at 48, its binary64 re-tests spill)
+    best.minb = minbs[0];
     best.buffered = gather_buffer(s.host, best.lanes);
     best.blocks = blocks_for(best.minb, best.lanes);
     if (c.no_autotune || !every || lanes.size() * minbs.size() == 1 || (progress && progress->cancel))
@@ -2464,55 +2481,32 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     auto t0 = std::chrono::steady_clock::now();
-    // One launch of a candidate shape over the sampled steps (every >= 2) or the whole queue.
-    auto trial = [&](uint32_t minb, uint32_t w, uint32_t sample) {
+    float best_ms = INFINITY;
+    auto trial = [&](uint32_t minb, uint32_t w) {
         const uint32_t blocks = blocks_for(minb, w);
         ba.lanes = w;
         ba.buffered = gather_buffer(s.host, w);
         ba.scratch = gather_scratch(s, blocks, w, ba.buffered);
-        ba.sample_every = sample;
         CK(cudaMemsetAsync(ba.head, 0, sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
-        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.stack_depth, w, ba.buffered), st>>>(s.sc,
-                                                                                                            ba);
+        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.stack_depth, w, ba.buffered), st>>>(s.sc, ba);
         CK(cudaGetLastError());
         CK(cudaEventRecord(b, st));
         CK(cudaEventSynchronize(b));
         float ms = 0.0f;
         CK(cudaEventElapsedTime(&ms, a, b));
         ++best.trials;
-        return ms;
-    };
-    // The sampled trials shortlist two shapes; those two then run over the whole queue, and the
-    // faster wins. A sample has few steps per warp, so its load balance favours the finer
-    // shapes more than the whole pass does (sampled trials alone picked 8 lanes per texel on the
-    // outdoor gather, 3 % slower than the 4 lanes the whole pass prefers). More resident warps
-    // hide more of the traversal's latency and fewer registers spill more: on the outdoor gather
-    // 10 blocks per SM ran in 93.4 ms, 9 in 94.3, 8 in 97.1, 12 (40 registers) in 102.3.
-    struct Candidate {
-        float ms;
-        uint32_t minb, w;
-    };
-    auto by_ms = [](const Candidate &x, const Candidate &y) { return x.ms < y.ms; };
-    std::vector<Candidate> tried;
-    for (uint32_t w : lanes) tried.push_back(Candidate{trial(minbs[0], w, every), minbs[0], w});
-    std::stable_sort(tried.begin(), tried.end(), by_ms);
-    const size_t lane_picks = std::min<size_t>(2, tried.size());
-    for (size_t m = 1; m < minbs.size(); ++m)
-        for (size_t k = 0; k < lane_picks; ++k)
-            tried.push_back(Candidate{trial(minbs[m], tried[k].w, every), minbs[m], tried[k].w});
-    std::stable_sort(tried.begin(), tried.end(), by_ms);
-    float best_ms = INFINITY;
-    for (size_t k = 0; k < std::min<size_t>(2, tried.size()); ++k) {
-        const float ms = trial(tried[k].minb, tried[k].w, 1);
         if (ms < best_ms) {
             best_ms = ms;
-            best.lanes = tried[k].w;
-            best.minb = tried[k].minb;
-            best.blocks = blocks_for(tried[k].minb, tried[k].w);
-            best.buffered = gather_buffer(s.host, tried[k].w);
+            best.lanes = w;
+            best.minb = minb;
+            best.blocks = blocks;
+            best.buffered = ba.buffered;
         }
-    }
+    };
+    for (uint32_t w : lanes) trial(minbs[0], w);
+    const uint32_t w = best.lanes;
+    for (size_t k = 1; k < minbs.size(); ++k) trial(minbs[k], w);
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     best.ms = ms_since(t0);
