@@ -515,6 +515,10 @@ def load_library(path: str = LIBRARY_PATH):
     lib.dl_free.argtypes = [C.c_void_p]
     lib.dl_session_encode_payload.restype = C.c_int
     lib.dl_session_encode_payload.argtypes = [C.c_void_p, P(P(C.c_uint8)), P(C.c_uint64), P(C.c_uint32)]
+    lib.dl_session_payload_build.restype = C.c_int
+    lib.dl_session_payload_build.argtypes = [C.c_void_p, P(C.c_uint64), P(C.c_uint32)]
+    lib.dl_session_payload_read.restype = C.c_int
+    lib.dl_session_payload_read.argtypes = [C.c_void_p, C.c_void_p, C.c_uint64]
     lib.dl_release_memory.restype = None
     lib.dl_release_memory.argtypes = []
     lib.dl_session_occluder_bvh.restype = C.c_int
@@ -530,6 +534,12 @@ def load_library(path: str = LIBRARY_PATH):
     lib.dl_probe_read_bandwidth.argtypes = [C.c_int, C.c_uint32, C.c_uint64, C.c_uint32, P(C.c_double)]
     _LIB = lib
     return lib
+
+
+_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
+_bytes_at = C.pythonapi.PyBytes_AsString
+_bytes_at.restype, _bytes_at.argtypes = C.c_void_p, [C.py_object]
 
 
 def _raise(lib, status):
@@ -605,16 +615,16 @@ class Session:
     def encode_payload(self) -> tuple:
         """The last run's .dynlight payload built on the device and its CRC-32
         (dl_session_encode_payload)."""
-        data = C.POINTER(C.c_uint8)()
-        length = C.c_uint64()
-        crc = C.c_uint32()
-        status = self.lib.dl_session_encode_payload(self.handle, C.byref(data), C.byref(length), C.byref(crc))
+        length, crc = C.c_uint64(), C.c_uint32()
+        status = self.lib.dl_session_payload_build(self.handle, C.byref(length), C.byref(crc))
         if status != 0:
             _raise(self.lib, status)
-        try:
-            return bytes(np.ctypeslib.as_array(data, shape=(length.value,))), crc.value
-        finally:
-            self.lib.dl_free(data)
+        # a bytes object made at its final size and filled in place before anyone else sees it
+        payload = _new_bytes(None, length.value)
+        status = self.lib.dl_session_payload_read(self.handle, _bytes_at(payload), length.value)
+        if status != 0:
+            _raise(self.lib, status)
+        return payload, crc.value
 
     def bounce_map(self, mesh_id: int, slot: int):
         """The last run's filtered bounce map of (mesh id, light slot) before quantization:

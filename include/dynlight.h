@@ -370,6 +370,11 @@ dl_status dl_session_report(const dl_session *session, dl_bake_report *report);
  * dl_encode_payload on dl_session_result's scene. `*bytes` is freed with dl_free; the gzip
  * layer stays with the caller. */
 dl_status dl_session_encode_payload(dl_session *session, uint8_t **bytes, uint64_t *length, uint32_t *crc);
+/* The same in two calls, for callers with memory of their own to put the payload in: build assembles
+ * it on the device and tells its length and CRC-32, read copies it into `bytes` (`length` as build
+ * told it). A later run, build or destroy ends what read can return. */
+dl_status dl_session_payload_build(dl_session *session, uint64_t *length, uint32_t *crc);
+dl_status dl_session_payload_read(dl_session *session, uint8_t *bytes, uint64_t length);
 /* No counterpart in the reference (whose occluder BVH is internal to Occluders,
    src/bake/occluder.rs:63-114): a copy of the session's occluder BVH as the traversal reads it —
    up to `node_cap` 64-byte nodes (child boxes c0, c1, c2 as 12 floats, then the two child
