@@ -255,7 +255,7 @@ template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_burial(DevScene sc, uint32_t texels, const uint32_t *tex_xy,
                                                    const float4 *tex_pos, const uint32_t *tex_tri,
                                                    const float4 *tri_face, uint8_t *buried, Counters *ctr) {
-    __shared__ int stack[kStack * kBlock];
+    extern __shared__ int stack[];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t rays = 0;
     Visits vis{0, 0, 0};
@@ -569,7 +569,7 @@ __global__ void k_item_counts(const uint32_t *order, const uint32_t *pair_tri, c
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_photons(DevScene sc, const uint32_t *cube_lights, uint32_t cubes,
                                                     uint32_t res, Photon *photons, Counters *ctr) {
-    __shared__ int stack[kStack * kBlock];
+    extern __shared__ int stack[];
     uint64_t per = 6ull * res * res;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     Visits vis{0, 0, 0};
@@ -811,7 +811,7 @@ constexpr uint64_t kProbeStream = 0x736b7970726f6265ull;  // PROBE_STREAM (sky_p
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_distance_cubes(DevScene sc, uint32_t lights, uint32_t *out,
                                                            Counters *ctr) {
-    __shared__ int stack[kStack * kBlock];
+    extern __shared__ int stack[];
     const uint32_t per_face = kCubeRes * kCubeRes / 2;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     Visits vis{0, 0, 0};
@@ -845,7 +845,7 @@ struct SunMapArgs {
 __device__ __forceinline__ uint32_t unorm16(float d) { return f2u(roundf(clampf(d, 0.0f, 1.0f) * 65535.0f)); }
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_sun_map(DevScene sc, SunMapArgs a, Counters *ctr) {
-    __shared__ int stack[kStack * kBlock];
+    extern __shared__ int stack[];
     uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
     Visits vis{0, 0, 0};
     if (w < a.words) {
@@ -868,9 +868,11 @@ __global__ void __launch_bounds__(kBlock) k_sun_map(DevScene sc, SunMapArgs a, C
     if (REFINE) add_retests(ctr, vis.retests);
 }
 
-// trace_probe (sky_probes.rs:83-109), one thread per (probe, axis): the sky samples around the
-// axis, each a closest hit (a hit at distance 0 counts as none); the open share and the rays
-// that reached a triangle's back.
+// trace_probe (sky_probes.rs:83-109), kProbeLanes lanes per (probe, axis): the sky samples around
+// the axis, each a closest hit (a hit at distance 0 counts as none); the open share and the rays
+// that reached a triangle's back, both counts, so the lanes' samples add up in any order. One lane a
+// job left the chip a few thousand threads of 64 to 256 rays each: a room's 3087 probes took 394 us,
+// with 8 lanes 117 us.
 struct ProbeArgs {
     f3 origin;
     float spacing;
@@ -879,11 +881,15 @@ struct ProbeArgs {
     float *open;
     uint32_t *back;
 };
+constexpr uint32_t kProbeLanes = 8;
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_sky_probes(DevScene sc, ProbeArgs a, Counters *ctr) {
-    __shared__ int stack[kStack * kBlock];
-    unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    extern __shared__ int stack[];
+    const unsigned long long thread = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x, i = thread / kProbeLanes;
+    const uint32_t sub = (uint32_t)(thread % kProbeLanes);
     Visits vis{0, 0, 0};
+    uint32_t open = 0, back = 0;
+    const uint32_t samples = sc.sky_samples;
     if (i < a.jobs) {
         uint64_t probe = i / 6;
         uint32_t axis = (uint32_t)(i % 6);
@@ -901,8 +907,7 @@ __global__ void __launch_bounds__(kBlock) k_sky_probes(DevScene sc, ProbeArgs a,
         off.y = rng.next_f32();
         f3 side, across;
         ortho_pair(normal, side, across);
-        uint32_t open = 0, back = 0, samples = sc.sky_samples;
-        for (uint32_t taken = 0; taken < samples; ++taken) {
+        for (uint32_t taken = sub; taken < samples; taken += kProbeLanes) {
             f3 dir = cosine_direction_basis(normal, side, across, spread(taken, off, true));
             Hit h;
             bool found = traverse<false, false, REFINE>(sc, position, dir, INFINITY, a.alpha != 0, stack + threadIdx.x,
@@ -911,6 +916,12 @@ __global__ void __launch_bounds__(kBlock) k_sky_probes(DevScene sc, ProbeArgs a,
             if (found && dot(hit_face_normal(sc, h), dir) > 0.0f) ++back;
             if (!found) ++open;
         }
+    }
+    for (uint32_t o = 1; o < kProbeLanes; o <<= 1) {
+        open += __shfl_xor_sync(0xFFFFFFFFu, open, o);
+        back += __shfl_xor_sync(0xFFFFFFFFu, back, o);
+    }
+    if (i < a.jobs && sub == 0) {
         a.open[i] = (float)open / (float)(samples > 1 ? samples : 1);
         a.back[i] = back;
     }
@@ -1848,6 +1859,13 @@ struct dl_session {
 namespace dl {
 namespace {
 
+// Stack entries per thread that the scene's tree needs, rounded up to 4, and the shared memory of a
+// launch whose threads hold one stack each. Sized by the tree (8 to 28 entries on the workloads) instead
+// of by the deepest tree accepted (64, 32 KB a block, at most 7 blocks per SM): the room grid's photon cubes
+// took 7.1 ms and take 5.7 ms, burial of the outdoor level 3.5 ms and 2.6 ms.
+uint32_t stack_depth(const dl_session &s) { return std::max<uint32_t>(8, (s.host.bvh_depth + 3) & ~3u); }
+size_t stack_smem(const dl_session &s) { return (size_t)stack_depth(s) * kBlock * sizeof(int); }
+
 void scan_u32(dl_session &s, const uint32_t *in, uint32_t *out, size_t n) {
     size_t temp = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, temp, in, out, n, s.stream));
@@ -2314,7 +2332,7 @@ std::map<TuneKey, TraceTune> g_tune_cache;
 TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_progress *progress) {
     const dl_bake_config &c = s.config;
     TraceTune best;
-    best.stack_depth = std::max<uint32_t>(8, (s.host.bvh_depth + 3) & ~3u);
+    best.stack_depth = stack_depth(s);
     auto blocks_for = [&](uint32_t minb) {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(count, refine, minb), kBlock,
@@ -2432,7 +2450,7 @@ std::map<TuneKey, GatherTune> g_gather_cache;
 GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refine, dl_progress *progress) {
     const dl_bake_config &c = s.config;
     GatherTune best;
-    best.stack_depth = std::max<uint32_t>(8, (s.host.bvh_depth + 3) & ~3u);
+    best.stack_depth = stack_depth(s);
     auto blocks_for = [&](uint32_t minb, uint32_t w) {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_kernel(refine, minb), kBlock,
@@ -2522,7 +2540,8 @@ void bake_maps(dl_session &s, bool refine) {
     if (h.local_lights) {
         s.cube_word_count = (uint64_t)h.local_lights * 6 * kCubeRes * kCubeRes / 2;
         uint32_t *cubes = P.get<uint32_t>("cube_words", s.cube_word_count);
-        (refine ? k_distance_cubes<true> : k_distance_cubes<false>)<<<grid_for(s.cube_word_count), kBlock, 0, st>>>(
+        (refine ? k_distance_cubes<true>
+                : k_distance_cubes<false>)<<<grid_for(s.cube_word_count), kBlock, stack_smem(s), st>>>(
             s.sc, h.local_lights, cubes, s.ctr);
         LAUNCHED("k_distance_cubes");
         ++s.launches;
@@ -2550,7 +2569,7 @@ void bake_maps(dl_session &s, bool refine) {
             a.words = (uint32_t)(((uint64_t)m.resolution * m.resolution + 1) / 2);
             a.alpha = (l.flags & kLightAlpha) != 0;
             a.out = P.get<uint32_t>("sun_map_" + std::to_string(s.sun_setups.size()), a.words);
-            (refine ? k_sun_map<true> : k_sun_map<false>)<<<grid_for(a.words), kBlock, 0, st>>>(s.sc, a, s.ctr);
+            (refine ? k_sun_map<true> : k_sun_map<false>)<<<grid_for(a.words), kBlock, stack_smem(s), st>>>(s.sc, a, s.ctr);
             LAUNCHED("k_sun_map");
             ++s.launches;
             texels = a.out;
@@ -2570,7 +2589,8 @@ void bake_maps(dl_session &s, bool refine) {
             a.jobs = s.probe_grid.count() * 6;
             a.open = P.get<float>("probe_open", a.jobs);
             a.back = P.get<uint32_t>("probe_back", a.jobs);
-            (refine ? k_sky_probes<true> : k_sky_probes<false>)<<<grid_for(a.jobs), kBlock, 0, st>>>(s.sc, a, s.ctr);
+            (refine ? k_sky_probes<true>
+                    : k_sky_probes<false>)<<<grid_for(a.jobs * kProbeLanes), kBlock, stack_smem(s), st>>>(s.sc, a, s.ctr);
             LAUNCHED("k_sky_probes");
             ++s.launches;
             s.probe_open = a.open;
@@ -2722,7 +2742,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
     CK(cudaEventRecord(s.marks[2], st));
     if (texels_all) {
         auto burial = refine ? k_burial<true> : k_burial<false>;
-        burial<<<grid_for(texels_all), kBlock, 0, st>>>(sc, texels_all, tex_xy, tex_pos, tex_tri, tri_face, buried,
+        burial<<<grid_for(texels_all), kBlock, stack_smem(s), st>>>(sc, texels_all, tex_xy, tex_pos, tex_tri, tri_face, buried,
                                                         s.ctr);
         LAUNCHED("k_burial");
         ++s.launches;
@@ -2873,7 +2893,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
             uint32_t *cube_lights = P.get<uint32_t>("cube_lights", cubes);
             CK(cudaMemcpyAsync(cube_lights, hs.cube_lights.data(), cubes * 4ull, cudaMemcpyHostToDevice, st));
             auto photon = refine_bounce ? k_photons<true> : k_photons<false>;
-            photon<<<grid_for(photons_n), kBlock, 0, st>>>(sc, cube_lights, cubes, res, photons, s.ctr);
+            photon<<<grid_for(photons_n), kBlock, stack_smem(s), st>>>(sc, cube_lights, cubes, res, photons, s.ctr);
             LAUNCHED("k_photons");
             ++s.launches;
         }

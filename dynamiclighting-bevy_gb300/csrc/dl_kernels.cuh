@@ -558,12 +558,11 @@ __device__ __forceinline__ Contribution local_sample(const DevScene &sc, const D
     f3 random = on_unit_sphere(g.rng);
     f3 sample = normalize_or(slerp3(g.direction, random, spread_s), g.direction);
     Photon ph = cube[cube_texel_index(sample, res)];
-    f3 pn{(float)(int8_t)(ph.normal & 0xFF) / 127.0f, (float)(int8_t)((ph.normal >> 8) & 0xFF) / 127.0f,
-          (float)(int8_t)((ph.normal >> 16) & 0xFF) / 127.0f};
+    f3 pn{byte_over((float)(int8_t)(ph.normal & 0xFF), 127.0f, 1.0f / 127.0f),
+          byte_over((float)(int8_t)((ph.normal >> 8) & 0xFF), 127.0f, 1.0f / 127.0f),
+          byte_over((float)(int8_t)((ph.normal >> 16) & 0xFF), 127.0f, 1.0f / 127.0f)};
     pn = normalize_or_zero(pn);
     f3 photon = add(l.position, scale(sample, ph.distance));
-    f3 albedo{(float)(ph.albedo & 0xFF) / 255.0f, (float)((ph.albedo >> 8) & 0xFF) / 255.0f,
-              (float)((ph.albedo >> 16) & 0xFF) / 255.0f};
     f3 to_photon = sub(photon, tr.origin);
     float distance = length(to_photon);
     if (is_zero(pn) || distance <= 0.0f) return c;
@@ -571,7 +570,12 @@ __device__ __forceinline__ Contribution local_sample(const DevScene &sc, const D
     c.rays = 1;
     if (!tr(d, distance)) {
         float weight = fmaxf(dot(normal, d), 0.0f) * fmaxf(dot(pn, neg(d)), 0.0f);
-        c.value = scale(reflected(sc, albedo), weight);
+        f3 albedo{1.0f, 1.0f, 1.0f};
+        if (sc.colored_bounce)
+            albedo = f3{byte_over((float)(ph.albedo & 0xFF), 255.0f, 1.0f / 255.0f),
+                        byte_over((float)((ph.albedo >> 8) & 0xFF), 255.0f, 1.0f / 255.0f),
+                        byte_over((float)((ph.albedo >> 16) & 0xFF), 255.0f, 1.0f / 255.0f)};
+        c.value = scale(albedo, weight);
         c.add = true;
     }
     return c;

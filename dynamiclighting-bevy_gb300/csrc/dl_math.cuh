@@ -149,6 +149,14 @@ DL_HD int f2i8(float f) {
     return (int)f;
 }
 
+// x / n for the whole numbers of a byte and n = 127 or 255, rounded as the division is: a quotient from
+// the rounded reciprocal corrected by its exact remainder (checked over all bytes in
+// tests/native/byte_check.cpp). 3 operations where the division takes about 9.
+DL_HD float byte_over(float x, float n, float reciprocal) {
+    const float q = x * reciprocal;
+    return fmaf(fmaf(-q, n, x), reciprocal, q);
+}
+
 // Orthonormal basis around a unit vector (Duff et al., JCGT 2017), as glam's
 // Vec3::any_orthonormal_pair evaluates it.
 DL_HD void ortho_pair(f3 n, f3 &a, f3 &b) {
