@@ -58,6 +58,29 @@ __device__ __forceinline__ void add_retests(Counters *ctr, unsigned long long n)
     if (lane_id() == 0 && w) atomicAdd(&ctr->retests, w);
 }
 
+// ================================ sample order tables ====================================
+
+// The sample orders of DevScene (`orders`, `order_cells`, `cell_samples`) for n = 16, 32, ...,
+// kMaxOrdered, a thread per sample: the first n points of the (0, 2)-sequence hold one point in each cell of
+// a 2^ceil(m/2) x 2^floor(m/2) grid (n = 2^m), so sample j's rank in the cells' Morton order is the
+// Morton code of its cell: what sky_sample_order and sample_cells (dl_host.hpp) find by sorting. On the
+// host that took 0.7 ms of every session, a fifth of the smallest bake.
+__device__ __forceinline__ uint32_t spread_bits(uint32_t v) {  // bit i of a byte to bit 2i
+    v = (v | v << 4) & 0x0F0Fu;
+    v = (v | v << 2) & 0x3333u;
+    return (v | v << 1) & 0x5555u;
+}
+__global__ void k_sample_tables(uint16_t *orders, uint16_t *cells, uint16_t *samples) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x + 16;
+    if (i >= 2 * kMaxOrdered) return;
+    const uint32_t m = 31 - __clz(i), n = 1u << m, j = i - n, base = n - 16, xb = (m + 1) / 2, yb = m / 2;
+    const uint32_t cx = rev_bits(j) >> (32 - xb), cy = sobol2(j) >> (32 - yb);
+    const uint32_t rank = spread_bits(cx) | spread_bits(cy) << 1;
+    orders[base + rank] = (uint16_t)j;
+    cells[base + rank] = (uint16_t)(cx | cy << 8);
+    samples[base + (cy << xb | cx)] = (uint16_t)j;
+}
+
 // ================================ setup and association ==================================
 
 __global__ void k_setup(DevScene sc, float4 *tri_face, uint4 *tri_crop, uint32_t *tri_count) {
@@ -2091,9 +2114,25 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
         }
     }
     uint32_t V = vbase[M], I = ibase[M], T = tbase[M];
-    // The per-vertex and per-index arrays are flattened by the host's cores into one pinned
-    // staging buffer (reused across sessions through the result-word cache), so that their
-    // uploads run as DMA copies; the buffer goes back once the stream has drained.
+    uint32_t N = (uint32_t)h.occ_mesh.size();
+    // Every array of the scene goes into one pinned staging buffer (reused across sessions through the
+    // result-word cache; it goes back once the stream has drained), the per-vertex and per-index arrays
+    // flattened into it by the host's cores, and from there in one DMA copy into one device allocation.
+    struct Packed {
+        size_t bytes = 0;
+        size_t add(size_t n) {
+            const size_t at = bytes;
+            bytes += (std::max<size_t>(n, 16) + 255) & ~size_t(255);
+            return at;
+        }
+    } pack;
+    const size_t at_occ_mesh = pack.add(N * 4ull), at_occ_tri = pack.add(N * 4ull), at_vbase = pack.add((M + 1) * 4ull),
+                 at_ibase = pack.add((M + 1) * 4ull), at_tbase = pack.add((M + 1) * 4ull), at_res = pack.add(M * 4ull),
+                 at_flags = pack.add(M * 4ull), at_ids = pack.add(M * 8ull), at_albedo = pack.add(M * 12ull),
+                 at_alpha = pack.add(M * 16ull), at_alpha_pool = pack.add(alpha_pool.size()),
+                 at_lights = pack.add(h.lights.size() * sizeof(DevLight)), at_pos = pack.add(V * 12ull),
+                 at_nrm = pack.add(V * 12ull), at_uv1 = pack.add(V * 8ull), at_uv0 = pack.add(V * 8ull),
+                 at_idx = pack.add(I * 4ull), at_tri_mesh = pack.add(T * 4ull);
     struct Staging {
         WordCache::Buffer b;
         cudaStream_t stream;
@@ -2101,10 +2140,12 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
             if (stream) cudaStreamSynchronize(stream);
             word_cache().give(b);
         }
-    } staging{word_cache().take((size_t)V * 10 + I + T + 1), s->stream};
-    float *pos = reinterpret_cast<float *>(staging.b.p), *nrm = pos + (size_t)V * 3, *uv1 = nrm + (size_t)V * 3,
-          *uv0 = uv1 + (size_t)V * 2;
-    uint32_t *idx = reinterpret_cast<uint32_t *>(uv0 + (size_t)V * 2), *tri_mesh = idx + I;
+    } staging{word_cache().take(pack.bytes / 4), s->stream};
+    char *const host_at = reinterpret_cast<char *>(staging.b.p);
+    float *pos = reinterpret_cast<float *>(host_at + at_pos), *nrm = reinterpret_cast<float *>(host_at + at_nrm),
+          *uv1 = reinterpret_cast<float *>(host_at + at_uv1), *uv0 = reinterpret_cast<float *>(host_at + at_uv0);
+    uint32_t *idx = reinterpret_cast<uint32_t *>(host_at + at_idx),
+             *tri_mesh = reinterpret_cast<uint32_t *>(host_at + at_tri_mesh);
     auto flatten = [&](uint32_t m) {
         const dl_mesh &mm = *h.meshes[m];
         std::memcpy(&pos[(size_t)vbase[m] * 3], mm.positions, mm.vertex_count * 12ull);
@@ -2123,7 +2164,9 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
     };
     {
         // meshes split into contiguous runs of about equal vertex and index counts, one per thread
-        const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+        // (starting threads costs more than flattening a small scene)
+        const unsigned cores = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+        const unsigned hw = (uint64_t)V + I < (1u << 17) ? 1u : cores;
         const uint64_t per = ((uint64_t)V + I) / hw + 1;
         std::vector<uint32_t> cut{0};
         uint64_t acc = 0;
@@ -2151,7 +2194,6 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
     }
     s->grid_off[M] = s->grid_words;
     s->mesh_tri_base = tbase;
-    uint32_t N = (uint32_t)h.occ_mesh.size();
 
     uint64_t &bytes = s->scene_bytes;
     auto up = [&](const void *src, size_t n, auto *&dst) {
@@ -2163,23 +2205,45 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
     };
     DevScene &sc = s->sc;
     sc.occluders = N;
-    up(h.occ_mesh.data(), N * 4ull, sc.occ_mesh);
-    up(h.occ_tri.data(), N * 4ull, sc.occ_tri);
+    char *const dev_at = reinterpret_cast<char *>(dev_alloc<uint8_t>(s->owned, s->stream, pack.bytes, bytes, &s->budget));
+    auto put = [&](size_t at, const void *src, size_t n) {
+        if (src && n) std::memcpy(host_at + at, src, n);
+        s->report.h2d_bytes += n;
+    };
+    auto placed = [&](size_t at, auto *&dst) { dst = reinterpret_cast<std::remove_reference_t<decltype(dst)>>(dev_at + at); };
+    put(at_occ_mesh, h.occ_mesh.data(), N * 4ull);
+    put(at_occ_tri, h.occ_tri.data(), N * 4ull);
+    put(at_vbase, vbase.data(), vbase.size() * 4);
+    put(at_ibase, ibase.data(), ibase.size() * 4);
+    put(at_tbase, tbase.data(), tbase.size() * 4);
+    put(at_res, h.resolution.data(), M * 4ull);
+    put(at_flags, flags.data(), M * 4ull);
+    put(at_ids, ids.data(), M * 8ull);
+    put(at_albedo, albedo.data(), M * 12ull);
+    put(at_alpha, alpha.data(), M * 16ull);
+    put(at_alpha_pool, alpha_pool.data(), alpha_pool.size());
+    put(at_lights, h.lights.data(), h.lights.size() * sizeof(DevLight));
+    s->report.h2d_bytes += (uint64_t)V * 40 + I * 4ull + T * 4ull;  // flattened in place
+    CK(cudaMemcpyAsync(dev_at, host_at, pack.bytes, cudaMemcpyHostToDevice, s->stream));
     sc.mesh_count = M;
-    up(vbase.data(), vbase.size() * 4, sc.mesh_vertex_base);
-    up(ibase.data(), ibase.size() * 4, sc.mesh_index_base);
-    up(tbase.data(), tbase.size() * 4, sc.mesh_tri_base);
-    up(h.resolution.data(), M * 4ull, sc.mesh_res);
-    up(flags.data(), M * 4ull, sc.mesh_flags);
-    up(ids.data(), M * 8ull, sc.mesh_id);
-    up(albedo.data(), M * 12ull, sc.mesh_albedo);
-    up(alpha.data(), M * 16ull, sc.mesh_alpha);
-    up(alpha_pool.data(), alpha_pool.size(), sc.alpha_pool);
-    up(pos, (size_t)V * 12, sc.positions);
-    up(nrm, (size_t)V * 12, sc.normals);
-    up(uv1, (size_t)V * 8, sc.uv1);
-    up(uv0, (size_t)V * 8, sc.uv0);
-    up(idx, (size_t)I * 4, sc.indices);
+    placed(at_occ_mesh, sc.occ_mesh);
+    placed(at_occ_tri, sc.occ_tri);
+    placed(at_vbase, sc.mesh_vertex_base);
+    placed(at_ibase, sc.mesh_index_base);
+    placed(at_tbase, sc.mesh_tri_base);
+    placed(at_res, sc.mesh_res);
+    placed(at_flags, sc.mesh_flags);
+    placed(at_ids, sc.mesh_id);
+    placed(at_albedo, sc.mesh_albedo);
+    placed(at_alpha, sc.mesh_alpha);
+    placed(at_alpha_pool, sc.alpha_pool);
+    placed(at_lights, sc.lights);
+    placed(at_pos, sc.positions);
+    placed(at_nrm, sc.normals);
+    placed(at_uv1, sc.uv1);
+    placed(at_uv0, sc.uv0);
+    placed(at_idx, sc.indices);
+    placed(at_tri_mesh, sc.tri_mesh);
     double ms_bvh_device = 0.0;
     if (host_bvh) {
         std::vector<uint32_t> occ_leaf(N);
@@ -2212,7 +2276,7 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
         ms_bvh_device = ms_since(t_bvh);
         s->report.ms_host[1] = ms_bvh_device;
         // the traversal stack holds one entry per level below the root
-        if (db.too_deep || db.depth >= (uint32_t)kStack) {
+        if (db.depth >= (uint32_t)kStack) {
             g_error = "occluder BVH deeper than the traversal stack";
             return DL_UNSUPPORTED;
         }
@@ -2228,31 +2292,27 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
         }
     }
     sc.triangles = T;
-    up(tri_mesh, T * 4ull, sc.tri_mesh);
     sc.light_count = (uint32_t)h.lights.size();
     sc.local_lights = h.local_lights;
-    up(h.lights.data(), h.lights.size() * sizeof(DevLight), sc.lights);
     sc.seed = o->seed;
     sc.area_samples = o->area_light_samples;
     sc.area_min_samples = o->area_light_min_samples;
     sc.sky_samples = o->sky_samples;
-    std::vector<uint16_t> orders, cells, cell_samples;
-    for (uint32_t n = 16; n <= kMaxOrdered; n *= 2) {
-        std::vector<uint16_t> o16 = sky_sample_order(n);
-        orders.insert(orders.end(), o16.begin(), o16.end());
-        SampleCells c = sample_cells(n);
-        cells.insert(cells.end(), c.cells.begin(), c.cells.end());
-        cell_samples.insert(cell_samples.end(), c.samples.begin(), c.samples.end());
-    }
-    up(cells.data(), cells.size() * 2, sc.order_cells);
-    up(cell_samples.data(), cell_samples.size() * 2, sc.cell_samples);
-    std::vector<uint16_t> sky_order = sky_sample_order(o->sky_samples);
-    up(orders.data(), orders.size() * 2, sc.orders);
+    constexpr uint32_t kTable = 2 * kMaxOrdered - 16;
+    uint16_t *tables = dev_alloc<uint16_t>(s->owned, s->stream, 3 * kTable, bytes, &s->budget);
+    k_sample_tables<<<grid_for(kTable), kBlock, 0, s->stream>>>(tables, tables + kTable, tables + 2 * kTable);
+    LAUNCHED("k_sample_tables");
+    sc.orders = tables;
+    sc.order_cells = tables + kTable;
+    sc.cell_samples = tables + 2 * kTable;
     sc.sky_order = nullptr;
-    if (o->sky_samples <= kMaxOrdered && !sky_order.empty()) {
-        sc.sky_order = sc.orders + (o->sky_samples - 16);
-    } else if (!sky_order.empty()) {
-        up(sky_order.data(), sky_order.size() * 2, sc.sky_order);
+    std::vector<uint16_t> sky_order;  // beyond the tables; its upload ends before this returns
+    const uint32_t sky = o->sky_samples;
+    if (sky >= 16 && sky <= kMaxOrdered && !(sky & (sky - 1))) {
+        sc.sky_order = sc.orders + (sky - 16);
+    } else if (sky > kMaxOrdered) {
+        sky_order = sky_sample_order(sky);
+        if (!sky_order.empty()) up(sky_order.data(), sky_order.size() * 2, sc.sky_order);
     }
     sc.colored_bounce = o->colored_bounce;
     sc.refine_eps = s->config.refine_epsilon;

@@ -14,10 +14,10 @@
 //     split      a thread per node: SAH sweep, decision, children (large ones to the next level,
 //                the others to the small list)
 //     partition  per-block left counts, per-node block offsets, stable scatter, copy back
-//   small nodes: a warp builds a whole subtree depth first (bounds by warp reductions, bins by
-//     shared-memory atomics, stable partition by ballots)
-//   layout: subtree sizes bottom-up and depth-first positions top-down, level by level; nodes
-//     written at their positions with padded child boxes; triangles in leaf order.
+//   small nodes: a block builds a whole subtree in shared memory, level by level, a warp per node
+//     (bounds by warp reductions, bins by shared-memory atomics, stable partition by ballots)
+//   layout: subtree sizes by climbing from the lowest nodes, depth-first positions by climbing to the
+//     root; nodes written at their positions with padded child boxes; triangles in leaf order.
 #include "dl_bvh.hpp"
 
 #include <algorithm>
@@ -31,7 +31,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr uint32_t kChunk = 4096;     // positions per block in the large-node kernels
 constexpr uint32_t kSmall = 512;      // nodes up to this size are built whole by one warp
-constexpr int kWarpStack = 96;        // pending nodes of a warp's subtree (depth + 1 at most)
+static_assert(kSmall <= 65536, "a small subtree's positions are 16-bit");
 constexpr int kBinWords = 3 * kBvhBins * 7;  // per (axis, bin): count, lo xyz, hi xyz
 
 #define BK(x)                                                                 \
@@ -57,11 +57,12 @@ struct Task {
     uint32_t node, first, count, depth;
 };
 
-// A node while the tree is built: its box, children (TNode ids) and primitive range.
+// A node while the tree is built: its box, children (TNode ids), primitive range and parent (TNode id
+// << 1 | which child). The array starts zeroed: a TNode that no subtree took is no inner node.
 struct TNode {
     float lo[3], hi[3];
     int32_t kid[2];
-    uint32_t first, count, depth, inner;
+    uint32_t first, count, parent, inner;
 };
 
 struct Split {
@@ -73,7 +74,7 @@ struct State {
     float4 *plo, *phi, *pc;        // per occluder: box and centroid
     uint32_t *idx, *tmp;           // position -> occluder
     TNode *nodes;
-    uint32_t *node_count, *max_depth, *error;
+    uint32_t *node_count, *max_depth;
     Task *small;
     uint32_t *small_count;
 };
@@ -240,23 +241,10 @@ __device__ void bins_decode(const int *w, BvhBins &out) {
         }
 }
 
-// The decision for node `id` (range first/count at depth) with box lo/hi; `binned` false for a
-// leaf before binning, else the best split (cost, axis, bin) and the items left of it. Fills the
-// TNode and, for a split, allocates both children.
-__device__ Split decide_node(const State &st, uint32_t id, uint32_t first, uint32_t count, uint32_t depth,
-                             const float lo[3], const float hi[3], bool binned, float cost, int axis, int bin,
-                             uint32_t left) {
-    TNode &n = st.nodes[id];
-    for (int a = 0; a < 3; ++a) {
-        n.lo[a] = lo[a];
-        n.hi[a] = hi[a];
-    }
-    n.first = first;
-    n.count = count;
-    n.depth = depth;
-    n.inner = 0;
-    n.kid[0] = n.kid[1] = -1;
-    atomicMax(st.max_depth, depth);
+// The decision for a node (`count` items at depth) with box lo/hi; `binned` false for a leaf before
+// binning, else the best split (cost, axis, bin) and the items left of it.
+__device__ __forceinline__ Split decide_split(uint32_t count, uint32_t depth, const float lo[3], const float hi[3],
+                                              bool binned, float cost, int axis, int bin, uint32_t left) {
     Split s{kBvhLeaf, axis, bin, 0};
     if (!binned) return s;
     s.how = bvh_decide(count, depth, lo, hi, cost, axis);
@@ -266,11 +254,25 @@ __device__ Split decide_node(const State &st, uint32_t id, uint32_t first, uint3
         if (left == 0 || left == count) s.how = kBvhByIndex;  // the partition leaves every item in place
     }
     if (s.how == kBvhByIndex) s.left = count / 2;
-    uint32_t k0 = atomicAdd(st.node_count, 2u);
-    n.inner = 1;
-    n.kid[0] = (int32_t)k0;
-    n.kid[1] = (int32_t)(k0 + 1);
     return s;
+}
+// Fills TNode `id`; for a split, k0 and k0 + 1 are its children.
+__device__ __forceinline__ void write_node(const State &st, uint32_t id, uint32_t first, uint32_t count,
+                                           const float lo[3], const float hi[3], bool inner, uint32_t k0) {
+    TNode &n = st.nodes[id];
+    for (int a = 0; a < 3; ++a) {
+        n.lo[a] = lo[a];
+        n.hi[a] = hi[a];
+    }
+    n.first = first;
+    n.count = count;
+    n.inner = inner ? 1u : 0u;
+    n.kid[0] = inner ? (int32_t)k0 : -1;
+    n.kid[1] = inner ? (int32_t)(k0 + 1) : -1;
+    if (inner) {
+        st.nodes[k0].parent = id << 1;
+        st.nodes[k0 + 1].parent = id << 1 | 1u;
+    }
 }
 
 __global__ void k_level_split(State st, Level lv) {
@@ -292,13 +294,14 @@ __global__ void k_level_split(State st, Level lv) {
     bvh_best_split(bins, use, cost, axis, bin);
     uint32_t left = 0;
     for (int j = 0; axis >= 0 && j <= bin; ++j) left += bins.bc[axis][j];
-    Split s = decide_node(st, k.node, k.first, k.count, k.depth, lo, hi, !bvh_leaf_before_bins(k.count, k.depth),
-                          cost, axis, bin, left);
+    Split s = decide_split(k.count, k.depth, lo, hi, !bvh_leaf_before_bins(k.count, k.depth), cost, axis, bin, left);
     lv.split[t] = s;
-    if (s.how == kBvhLeaf) return;
-    const TNode &n = st.nodes[k.node];
-    Task kids[2] = {{(uint32_t)n.kid[0], k.first, s.left, k.depth + 1},
-                    {(uint32_t)n.kid[1], k.first + s.left, k.count - s.left, k.depth + 1}};
+    const bool inner = s.how != kBvhLeaf;
+    const uint32_t k0 = inner ? atomicAdd(st.node_count, 2u) : 0u;
+    write_node(st, k.node, k.first, k.count, lo, hi, inner, k0);
+    atomicMax(st.max_depth, k.depth);
+    if (!inner) return;
+    Task kids[2] = {{k0, k.first, s.left, k.depth + 1}, {k0 + 1, k.first + s.left, k.count - s.left, k.depth + 1}};
     for (const Task &c : kids) {
         if (c.count > kSmall) lv.next[atomicAdd(lv.next_count, 1u)] = c;
         else st.small[atomicAdd(st.small_count, 1u)] = c;
@@ -477,124 +480,214 @@ __device__ void warp_best_split(const int *sb, const bool use[3], float &best_co
     }
 }
 
-constexpr int kSmallWarps = 4;
-
-__global__ void __launch_bounds__(32 * kSmallWarps) k_small(State st, uint32_t count) {
-    __shared__ int sbins[kSmallWarps][kBinWords];
-    __shared__ uint32_t sstack[kSmallWarps][kWarpStack];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t w = blockIdx.x * kSmallWarps + warp;
-    if (w >= count) return;  // warp-uniform
-    int *sb = sbins[warp];
-    uint32_t *stack = sstack[warp];
-    const Task root = st.small[w];
-    // a pending node's range and depth travel in its TNode
-    if (lane == 0) {
-        TNode &n = st.nodes[root.node];
-        n.first = root.first;
-        n.count = root.count;
-        n.depth = root.depth;
-        stack[0] = root.node;
-    }
-    __syncwarp();
-    int sp = 1;
+// A block builds one small subtree, a level at a time, a warp per node. The primitives' boxes and
+// centroids, their order and both levels' nodes stay in shared memory, and the subtree's TNodes (at most
+// twice its primitives, less two) are reserved at once, so that a node costs no round trip to global
+// memory. Bound by a node's latency (some 2 us of reductions, bins and scans in one warp), so nodes run
+// side by side, and small ones, the most, skip the bins' atomics and scans and evaluate every split
+// over the primitives themselves, a lane per (axis, bin). A warp per subtree, depth first, with its state
+// in global memory took 155 us for 72 triangles and 1167 us for subtrees of 512; this takes 50 us and
+// 200 us.
+constexpr int kSmallWarps = 8;
+constexpr uint32_t kDirect = 16;  // primitives up to which a node's splits are evaluated directly
+struct SmallTree {
+    float box[9][kSmall];  // lo xyz, hi xyz, centroid xyz
+    uint32_t item[kSmall];  // occluder
+    uint16_t order[kSmall], tmp[kSmall];  // position -> primitive
+    int bins[kSmallWarps][kBinWords];
+    uint8_t bin[kSmallWarps][3][kDirect];  // a small node's primitives' bins
+    // the level's nodes and the next one's: TNode, first position, count
+    uint32_t node[2][kSmall];
+    uint16_t first[2][kSmall], count[2][kSmall];
+    uint32_t nodes[2];   // their numbers
+    uint32_t next_node;  // the next reserved TNode
+};
+// warp_best_split's answer for a node of at most kDirect primitives, from their boxes and bins: the same
+// unions, counts and costs (minima, maxima and integers, then the same binary32 expression).
+__device__ __forceinline__ void direct_best_split(const SmallTree &t, const uint8_t (*bins)[kDirect], uint32_t first,
+                                                  uint32_t cnt, const bool use[3], float &best_cost, int &axis,
+                                                  int &bin, uint32_t &left) {
     const unsigned all = 0xFFFFFFFFu;
-    while (sp > 0) {
-        uint32_t id = stack[--sp];
-        __syncwarp();
-        const uint32_t first = st.nodes[id].first, cnt = st.nodes[id].count, depth = st.nodes[id].depth;
-        const uint32_t end = first + cnt;
-        int v[12];
-        for (int a = 0; a < 3; ++a) {
-            v[a] = v[6 + a] = ford(INFINITY);
-            v[3 + a] = v[9 + a] = ford(-INFINITY);
+    constexpr int kSplits = kBvhBins - 1;
+    float best = INFINITY;
+    int key = 0x7FFFFFFF;
+    uint32_t best_left = 0;
+    for (int c = threadIdx.x & 31u; c < 3 * kSplits; c += 32) {
+        const int a = c / kSplits, k = c % kSplits;
+        if (!(a == 0 ? use[0] : a == 1 ? use[1] : use[2])) continue;
+        float l[6], r[6];
+        for (int j = 0; j < 3; ++j) {
+            l[j] = r[j] = INFINITY;
+            l[3 + j] = r[3 + j] = -INFINITY;
         }
-        for (uint32_t p = first + lane; p < end; p += 32) {
-            uint32_t i = st.idx[p];
-            float4 lo = st.plo[i], hi = st.phi[i], c = st.pc[i];
+        uint32_t lc = 0;
+        for (uint32_t q = 0; q < cnt; ++q) {
+            const uint32_t i = t.order[first + q];
+            const bool goes = bins[a][q] <= k;
+            lc += goes;
+            for (int j = 0; j < 3; ++j) {
+                const float lo = t.box[j][i], hi = t.box[3 + j][i];
+                l[j] = goes ? bvh_min(l[j], lo) : l[j];
+                l[3 + j] = goes ? bvh_max(l[3 + j], hi) : l[3 + j];
+                r[j] = goes ? r[j] : bvh_min(r[j], lo);
+                r[3 + j] = goes ? r[3 + j] : bvh_max(r[3 + j], hi);
+            }
+        }
+        if (!lc || lc == cnt) continue;
+        const float cost = bvh_half_area(l, l + 3) * (float)lc + bvh_half_area(r, r + 3) * (float)(cnt - lc);
+        if (cost < best) {  // per lane, candidates in (axis, bin) order keep the first
+            best = cost;
+            key = a * kBvhBins + k;
+            best_left = lc;
+        }
+    }
+    for (int d = 16; d >= 1; d >>= 1) {
+        const float ob = __shfl_xor_sync(all, best, d);
+        const int ok = __shfl_xor_sync(all, key, d);
+        const uint32_t ol = __shfl_xor_sync(all, best_left, d);
+        if (ob < best || (ob == best && ok < key)) {
+            best = ob;
+            key = ok;
+            best_left = ol;
+        }
+    }
+    best_cost = best;
+    axis = key == 0x7FFFFFFF ? -1 : key / kBvhBins;
+    bin = key == 0x7FFFFFFF ? 0 : key % kBvhBins;
+    left = key == 0x7FFFFFFF ? 0 : best_left;
+}
+__global__ void __launch_bounds__(32 * kSmallWarps) k_small(State st) {
+    __shared__ SmallTree t;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const unsigned all = 0xFFFFFFFFu, below = (1u << lane) - 1u;
+    const Task root = st.small[blockIdx.x];
+    for (uint32_t p = threadIdx.x; p < root.count; p += blockDim.x) {
+        const uint32_t i = st.idx[root.first + p];
+        const float4 lo = st.plo[i], hi = st.phi[i], c = st.pc[i];
+        for (int a = 0; a < 3; ++a) {
+            t.box[a][p] = comp(lo, a);
+            t.box[3 + a][p] = comp(hi, a);
+            t.box[6 + a][p] = comp(c, a);
+        }
+        t.item[p] = i;
+        t.order[p] = (uint16_t)p;
+    }
+    if (threadIdx.x == 0) {
+        t.next_node = root.count > 1 ? atomicAdd(st.node_count, 2u * root.count - 2u) : 0u;
+        t.node[0][0] = root.node;
+        t.first[0][0] = 0;
+        t.count[0][0] = (uint16_t)root.count;
+        t.nodes[0] = 1;
+        t.nodes[1] = 0;
+    }
+    __syncthreads();
+    int *const bins = t.bins[warp];
+    uint32_t depth = root.depth;
+    for (int cur = 0;; cur ^= 1, ++depth) {
+        const uint32_t level = t.nodes[cur];
+        for (uint32_t k = warp; k < level; k += kSmallWarps) {
+            const uint32_t id = t.node[cur][k], first = t.first[cur][k], cnt = t.count[cur][k], end = first + cnt;
+            int v[12];
             for (int a = 0; a < 3; ++a) {
-                v[a] = min(v[a], ford(comp(lo, a)));
-                v[3 + a] = max(v[3 + a], ford(comp(hi, a)));
-                v[6 + a] = min(v[6 + a], ford(comp(c, a)));
-                v[9 + a] = max(v[9 + a], ford(comp(c, a)));
+                v[a] = v[6 + a] = ford(INFINITY);
+                v[3 + a] = v[9 + a] = ford(-INFINITY);
             }
-        }
-        for (int j = 0; j < 12; ++j) {
-            bool low = j < 3 || (j >= 6 && j < 9);
-            v[j] = low ? __reduce_min_sync(all, v[j]) : __reduce_max_sync(all, v[j]);
-        }
-        float lo[3], hi[3], clo[3], kk[3];
-        bool use[3];
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = funord(v[a]);
-            hi[a] = funord(v[3 + a]);
-        }
-        bin_setup(v, clo, kk, use);
-        const bool binned = !bvh_leaf_before_bins(cnt, depth);
-        if (binned) {
-            for (int j = lane; j < kBinWords; j += 32) {
-                int q = j % 7;
-                sb[j] = q == 0 ? 0 : ford(q <= 3 ? INFINITY : -INFINITY);
+            for (uint32_t p = first + lane; p < end; p += 32) {
+                const uint32_t i = t.order[p];
+                for (int a = 0; a < 3; ++a) {
+                    v[a] = min(v[a], ford(t.box[a][i]));
+                    v[3 + a] = max(v[3 + a], ford(t.box[3 + a][i]));
+                    v[6 + a] = min(v[6 + a], ford(t.box[6 + a][i]));
+                    v[9 + a] = max(v[9 + a], ford(t.box[6 + a][i]));
+                }
             }
-            __syncwarp();
-            for (uint32_t p = first + lane; p < end; p += 32) bin_add(st, st.idx[p], clo, kk, use, sb);
-            __syncwarp();
-        }
-        float cost = INFINITY;
-        int axis = -1, bin = 0;
-        uint32_t left = 0;
-        if (binned) warp_best_split(sb, use, cost, axis, bin, left);
-        Split s{kBvhLeaf, -1, 0, 0};
-        if (lane == 0) s = decide_node(st, id, first, cnt, depth, lo, hi, binned, cost, axis, bin, left);
-        s.how = __shfl_sync(all, s.how, 0);
-        s.axis = __shfl_sync(all, s.axis, 0);
-        s.bin = __shfl_sync(all, s.bin, 0);
-        s.left = __shfl_sync(all, s.left, 0);
-        __syncwarp();
-        if (s.how == kBvhLeaf) continue;
-        if (s.how == kBvhByBin) {
+            for (int j = 0; j < 12; ++j) {
+                bool low = j < 3 || (j >= 6 && j < 9);
+                v[j] = low ? __reduce_min_sync(all, v[j]) : __reduce_max_sync(all, v[j]);
+            }
+            float lo[3], hi[3], clo[3], kk[3];
+            bool use[3];
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = funord(v[a]);
+                hi[a] = funord(v[3 + a]);
+            }
+            bin_setup(v, clo, kk, use);
+            const bool binned = !bvh_leaf_before_bins(cnt, depth);
+            float cost = INFINITY;
+            int axis = -1, bin = 0;
+            uint32_t left = 0;
+            __syncwarp();  // the warp's bins are free again
+            if (binned && cnt <= kDirect) {
+                if (lane < cnt)
+                    for (int a = 0; a < 3; ++a)
+                        if (use[a])
+                            t.bin[warp][a][lane] = (uint8_t)bvh_bin(t.box[6 + a][t.order[first + lane]], clo[a], kk[a]);
+                __syncwarp();
+                direct_best_split(t, t.bin[warp], first, cnt, use, cost, axis, bin, left);
+            } else if (binned) {
+                for (int j = lane; j < kBinWords; j += 32) {
+                    int q = j % 7;
+                    bins[j] = q == 0 ? 0 : ford(q <= 3 ? INFINITY : -INFINITY);
+                }
+                __syncwarp();
+                for (uint32_t p = first + lane; p < end; p += 32) {
+                    const uint32_t i = t.order[p];
+                    for (int a = 0; a < 3; ++a) {
+                        if (!use[a]) continue;
+                        int *w = bins + (a * kBvhBins + bvh_bin(t.box[6 + a][i], clo[a], kk[a])) * 7;
+                        atomicAdd(w, 1);
+                        for (int j = 0; j < 3; ++j) {
+                            atomicMin(w + 1 + j, ford(t.box[j][i]));
+                            atomicMax(w + 4 + j, ford(t.box[3 + j][i]));
+                        }
+                    }
+                }
+                __syncwarp();
+                warp_best_split(bins, use, cost, axis, bin, left);
+            }
+            // every lane holds the same quantities and so the same decision
+            const Split s = decide_split(cnt, depth, lo, hi, binned, cost, axis, bin, left);
+            const bool inner = s.how != kBvhLeaf;
+            if (lane == 0) {
+                uint32_t k0 = 0;
+                if (inner) {
+                    k0 = atomicAdd(&t.next_node, 2u);
+                    const uint32_t slot = atomicAdd(&t.nodes[cur ^ 1], 2u);
+                    t.node[cur ^ 1][slot] = k0;
+                    t.first[cur ^ 1][slot] = (uint16_t)first;
+                    t.count[cur ^ 1][slot] = (uint16_t)s.left;
+                    t.node[cur ^ 1][slot + 1] = k0 + 1;
+                    t.first[cur ^ 1][slot + 1] = (uint16_t)(first + s.left);
+                    t.count[cur ^ 1][slot + 1] = (uint16_t)(cnt - s.left);
+                }
+                write_node(st, id, root.first + first, cnt, lo, hi, inner, k0);
+            }
+            if (!inner || s.how != kBvhByBin) continue;
             // stable partition through tmp, 32 items a round
             uint32_t lefts = 0, rights = 0;
             for (uint32_t base = first; base < end; base += 32) {
-                uint32_t p = base + lane;
-                bool valid = p < end;
-                uint32_t item = valid ? st.idx[p] : 0u;
-                bool left = valid && bvh_bin(comp(st.pc[item], s.axis), clo[s.axis], kk[s.axis]) <= s.bin;
-                unsigned bl = __ballot_sync(all, left), bv = __ballot_sync(all, valid);
-                unsigned below = (1u << lane) - 1u;
-                if (valid) {
-                    if (left) st.tmp[first + lefts + __popc(bl & below)] = item;
-                    else st.tmp[first + s.left + rights + __popc(bv & ~bl & below)] = item;
-                }
+                const uint32_t p = base + lane;
+                const bool valid = p < end;
+                const uint16_t i = valid ? t.order[p] : (uint16_t)0;
+                const bool goes = valid && bvh_bin(t.box[6 + s.axis][i], clo[s.axis], kk[s.axis]) <= s.bin;
+                const unsigned bl = __ballot_sync(all, goes), bv = __ballot_sync(all, valid);
+                if (goes) t.tmp[first + lefts + __popc(bl & below)] = i;
+                else if (valid) t.tmp[first + s.left + rights + __popc(bv & ~bl & below)] = i;
                 lefts += __popc(bl);
                 rights += __popc(bv & ~bl);
             }
             __syncwarp();
-            for (uint32_t p = first + lane; p < end; p += 32) st.idx[p] = st.tmp[p];
+            for (uint32_t p = first + lane; p < end; p += 32) t.order[p] = t.tmp[p];
             __syncwarp();
         }
-        if (lane == 0) {
-            const TNode &n = st.nodes[id];
-            uint32_t k0 = (uint32_t)n.kid[0], k1 = (uint32_t)n.kid[1];
-            TNode &a = st.nodes[k0];
-            a.first = first;
-            a.count = s.left;
-            a.depth = depth + 1;
-            TNode &b = st.nodes[k1];
-            b.first = first + s.left;
-            b.count = cnt - s.left;
-            b.depth = depth + 1;
-            if (sp + 2 <= kWarpStack) {
-                stack[sp] = k1;  // the left child comes off first
-                stack[sp + 1] = k0;
-            } else {
-                atomicExch(st.error, 1u);
-            }
-        }
-        sp += 2;
-        if (sp > kWarpStack) return;  // warp-uniform; the host reports the overflow
-        __syncwarp();
+        __syncthreads();
+        if (t.nodes[cur ^ 1] == 0) break;  // uniform
+        __syncthreads();
+        if (threadIdx.x == 0) t.nodes[cur] = 0;
+        __syncthreads();
     }
+    for (uint32_t p = threadIdx.x; p < root.count; p += blockDim.x) st.idx[root.first + p] = t.item[t.order[p]];
+    if (threadIdx.x == 0) atomicMax(st.max_depth, depth);
 }
 
 // ---- depth-first layout --------------------------------------------------------------------
@@ -603,29 +696,48 @@ struct Layout {
     const TNode *nodes;
     uint32_t total;  // TNodes
     uint32_t *size;  // inner nodes in the subtree of an inner node
-    uint32_t *pos;   // depth-first position of an inner node
+    uint32_t *pos;   // depth-first position of an inner node; before that, children arrived (k_sizes)
 };
 
-__global__ void k_sizes(Layout L, uint32_t depth) {
+// Subtree sizes, children before parents in one launch: a thread starts at every inner node without
+// inner children and climbs; at a node with two of them the second to arrive goes on.
+__global__ void k_sizes(Layout L) {
     uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= L.total) return;
-    const TNode &n = L.nodes[id];
-    if (n.depth != depth || !n.inner) return;
-    uint32_t s = 1;
-    for (int c = 0; c < 2; ++c)
-        if (L.nodes[n.kid[c]].inner) s += L.size[n.kid[c]];
-    L.size[id] = s;
+    if (id >= L.total || !L.nodes[id].inner) return;
+    if (L.nodes[L.nodes[id].kid[0]].inner || L.nodes[L.nodes[id].kid[1]].inner) return;
+    volatile uint32_t *size = L.size;
+    size[id] = 1;
+    while (id != 0) {
+        const uint32_t up = L.nodes[id].parent >> 1;
+        const TNode &n = L.nodes[up];
+        const bool both = L.nodes[n.kid[0]].inner && L.nodes[n.kid[1]].inner;
+        __threadfence();
+        if (both && atomicAdd(L.pos + up, 1u) == 0) return;
+        __threadfence();
+        uint32_t s = 1;
+        for (int c = 0; c < 2; ++c)
+            if (L.nodes[n.kid[c]].inner) s += size[n.kid[c]];
+        size[up] = s;
+        id = up;
+    }
 }
 
-__global__ void k_positions(Layout L, uint32_t depth) {
-    uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= L.total) return;
-    const TNode &n = L.nodes[id];
-    if (n.depth != depth || !n.inner) return;
-    uint32_t p = L.pos[id];
-    const TNode &l = L.nodes[n.kid[0]];
-    if (l.inner) L.pos[n.kid[0]] = p + 1;
-    if (L.nodes[n.kid[1]].inner) L.pos[n.kid[1]] = p + 1 + (l.inner ? L.size[n.kid[0]] : 0u);
+// Depth-first positions, the left subtree before the right one: a node comes one after its parent, plus
+// the left sibling's subtree for a right child. Each thread sums that up to the root.
+__global__ void k_positions(Layout L) {
+    const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
+    if (node >= L.total || !L.nodes[node].inner) return;
+    uint32_t p = 0;
+    for (uint32_t id = node; id != 0;) {
+        const uint32_t parent = L.nodes[id].parent, up = parent >> 1;
+        ++p;
+        if (parent & 1u) {
+            const int32_t left = L.nodes[up].kid[0];
+            if (L.nodes[left].inner) p += L.size[left];
+        }
+        id = up;
+    }
+    L.pos[node] = p;
 }
 
 __device__ __forceinline__ int32_t child_ref(const Layout &L, int32_t kid) {
@@ -717,15 +829,15 @@ void build_bvh_device(const DeviceBvhInput &in, const std::function<void *(size_
     st.pc = sc.get<float4>(n);
     st.idx = sc.get<uint32_t>(n);
     st.tmp = sc.get<uint32_t>(n);
-    const uint32_t cap = 2 * n;  // a binary tree over n leaves of >= 1 primitive has < 2n nodes
+    const uint32_t cap = 2 * n;  // a binary tree over n leaves of >= 1 primitive has < 2n nodes, reserved ones included
     st.nodes = sc.get<TNode>(cap);
-    uint32_t *counters = sc.get<uint32_t>(4);
+    uint32_t *counters = sc.get<uint32_t>(3);
     st.node_count = counters;
     st.max_depth = counters + 1;
-    st.error = counters + 2;
-    st.small_count = counters + 3;
+    st.small_count = counters + 2;
     st.small = sc.get<Task>(n);
-    const uint32_t one[4] = {1, 0, 0, 0};  // the root is TNode 0
+    BK(cudaMemsetAsync(st.nodes, 0, cap * sizeof(TNode), stream));
+    const uint32_t one[3] = {1, 0, 0};  // the root is TNode 0
     BK(cudaMemcpyAsync(counters, one, sizeof one, cudaMemcpyHostToDevice, stream));
     k_prims<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(in, st);
     BLAUNCHED("k_prims (bvh)");
@@ -803,34 +915,28 @@ void build_bvh_device(const DeviceBvhInput &in, const std::function<void *(size_
     uint32_t small = 0;
     BK(cudaMemcpyAsync(&small, st.small_count, 4, cudaMemcpyDeviceToHost, stream));
     BK(cudaStreamSynchronize(stream));
-    if (small)
-        k_small<<<blocks_for(small, kSmallWarps), 32 * kSmallWarps, 0, stream>>>(st, small);
+    if (small) k_small<<<small, 32 * kSmallWarps, 0, stream>>>(st);
     BLAUNCHED("k_small (bvh)");
-    uint32_t c[4];
+    uint32_t c[2];
     BK(cudaMemcpyAsync(c, counters, sizeof c, cudaMemcpyDeviceToHost, stream));
     BK(cudaStreamSynchronize(stream));
-    if (c[2]) {
-        out.too_deep = true;
-        return;
-    }
     const uint32_t total = c[0];
     out.depth = c[1];
 
-    // depth-first layout
-    Layout L{st.nodes, total, sc.get<uint32_t>(total), sc.get<uint32_t>(total)};
+    // depth-first layout; the primitives' boxes are read no more and hold its arrays
+    Layout L{st.nodes, total, reinterpret_cast<uint32_t *>(st.plo), reinterpret_cast<uint32_t *>(st.phi)};
     const uint32_t g = blocks_for(total, kThreads);
-    for (uint32_t d = out.depth; d >= 1; --d) k_sizes<<<g, kThreads, 0, stream>>>(L, d);
-    BK(cudaMemsetAsync(L.pos, 0, 4, stream));  // the root at 0
-    for (uint32_t d = 1; d < out.depth; ++d) k_positions<<<g, kThreads, 0, stream>>>(L, d);
+    BK(cudaMemsetAsync(L.pos, 0, total * 4ull, stream));
+    k_sizes<<<g, kThreads, 0, stream>>>(L);
+    k_positions<<<g, kThreads, 0, stream>>>(L);
     BLAUNCHED("k_sizes/k_positions (bvh)");
-    TNode root;
-    BK(cudaMemcpyAsync(&root, st.nodes, sizeof root, cudaMemcpyDeviceToHost, stream));
-    uint32_t inner = 1;
+    struct {
+        uint32_t inner, size;
+    } root;
+    BK(cudaMemcpyAsync(&root.inner, &st.nodes[0].inner, 4, cudaMemcpyDeviceToHost, stream));
+    BK(cudaMemcpyAsync(&root.size, L.size, 4, cudaMemcpyDeviceToHost, stream));
     BK(cudaStreamSynchronize(stream));
-    if (root.inner) {
-        BK(cudaMemcpyAsync(&inner, L.size, 4, cudaMemcpyDeviceToHost, stream));
-        BK(cudaStreamSynchronize(stream));
-    }
+    const uint32_t inner = root.inner ? root.size : 1;
     out.node_count = inner;
     out.nodes = static_cast<TravNode *>(alloc((size_t)inner * sizeof(TravNode)));
     out.tris = static_cast<float4 *>(alloc((size_t)n * 3 * sizeof(float4)));

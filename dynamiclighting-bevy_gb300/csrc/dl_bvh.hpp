@@ -30,7 +30,6 @@ struct DeviceBvh {
     uint32_t *occ_leaf = nullptr;  // occluder -> its slot in leaf order
     uint32_t node_count = 0;
     uint32_t depth = 0;        // the deepest node's level, the root being 1
-    bool too_deep = false;     // a subtree outgrew the builder's stack (the tree is unusable)
 };
 
 struct DeviceBvhError {
