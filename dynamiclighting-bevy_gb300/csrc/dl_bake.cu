@@ -1160,69 +1160,78 @@ __device__ __forceinline__ uint64_t bounce_words(uint4 crop, uint32_t bits, bool
 }
 
 // pack_bounce / pack_bounce_rgb (bounce_pack.rs:28-71) of one kept entry: the padded crop grid
-// of the filtered map, dithered from the stream [seed, mesh, light, triangle] in texel order.
+// of the filtered map, dithered from the stream [seed, mesh, light, triangle] in texel order. A value
+// takes a draw only when it is lit, so how far the stream has come depends on every value before: a warp
+// takes a round of pixels at once (32, or as many as fill whole words), counts the lit values before
+// each lane's with ballots, and each lane jumps the stream there. A round's pixels fill whole words: a
+// lane per word picks them from their lanes. A thread per entry, drawing one after another, took 749 us
+// for nine rooms (17 lights, colored, 5 bits) and this takes 347 us.
 __global__ void k_pack_bounce(DevScene sc, uint32_t entries, const uint32_t *entry_pair,
                               const unsigned long long *entry_bdst, const uint32_t *pair_tri,
                               const uint32_t *pair_light, const uint4 *tri_crop, const uint32_t *region_rect,
                               const uint32_t *woff, const float4 *map, uint32_t *words) {
-    uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= entries) return;
-    unsigned long long dst = entry_bdst[e];
+    constexpr unsigned all = 0xFFFFFFFFu;
+    const uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = lane_id();
+    if (e >= entries) return;  // uniform across the warp
+    const unsigned long long dst = entry_bdst[e];
     if (dst == ~0ull) return;
-    uint32_t p = entry_pair[e];
-    uint32_t t = pair_tri[p], s = pair_light[p];
-    uint32_t m = sc.tri_mesh[t];
+    const uint32_t p = entry_pair[e], t = pair_tri[p], s = pair_light[p], m = sc.tri_mesh[t];
     const DevLight &l = sc.lights[s];
     if (l.bounce_bits == 8) return;  // undithered: k_pack_bounce8
-    size_t re = (size_t)m * sc.light_count + s;
-    Rect w = bounce_window(region_rect + re * 4, sc.mesh_res[m]);
-    uint32_t ww = w.max_x - w.min_x + 1;
-    uint4 c = tri_crop[t];
-    int gw = (int)(c.z - c.x + 5), gh = (int)(c.w - c.y + 5);
-    uint32_t bits = l.bounce_bits;
+    const size_t re = (size_t)m * sc.light_count + s;
+    const Rect w = bounce_window(region_rect + re * 4, sc.mesh_res[m]);
+    const uint32_t ww = w.max_x - w.min_x + 1, base = woff[re];
+    const uint4 c = tri_crop[t];
+    const uint32_t gw = c.z - c.x + 5, gh = c.w - c.y + 5, bits = l.bounce_bits;
     Pcg rng = stream4(sc.seed, sc.mesh_id[m], l.id, t - sc.mesh_tri_base[m]);
-    bool colored = sc.colored_bounce != 0;
-    uint32_t pixel_bits = colored ? 3 * bits : bits;
-    uint32_t per = 32 / bits;
-    unsigned long long acc = 0;  // bits not yet written
-    uint32_t acc_bits = 0;
+    const bool colored = sc.colored_bounce != 0;
+    // colored: one bit stream of pixels 3 * bits wide; else floor(32 / bits) pixels a word, the
+    // rest of each word zero
+    const uint32_t pixel_bits = colored ? 3 * bits : bits, per = 32 / bits;
+    const uint32_t pixels = colored ? 32 : 32 / per * per, round_words = colored ? 3 * bits : pixels / per;
+    const uint64_t n = (uint64_t)gw * gh;
     uint64_t out = dst;
-    uint64_t n = (uint64_t)gw * gh;
-    for (uint64_t i = 0; i < n; ++i) {
-        int gx = (int)(i % gw), gy = (int)(i / gw);
+    for (uint64_t at = 0; at < n; at += pixels, out += round_words) {
+        const uint64_t i = at + lane;
+        const bool mine = lane < pixels && i < n;
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (gx >= 2 && gy >= 2 && gx < gw - 2 && gy < gh - 2) {
-            uint32_t x = c.x + gx - 2, y = c.y + gy - 2;
-            v = map[woff[re] + (size_t)(y - w.min_y) * ww + (x - w.min_x)];
+        if (mine) {
+            uint32_t gx, gy;
+            grid_xy(i, gw, gx, gy);
+            if (gx >= 2 && gy >= 2 && gx < gw - 2 && gy < gh - 2)
+                v = map[base + (size_t)(c.y + gy - 2 - w.min_y) * ww + (c.x + gx - 2 - w.min_x)];
         }
-        uint32_t pixel;
-        if (colored) {
-            pixel = quantize_bounce(v.x, bits, rng);
-            pixel |= quantize_bounce(v.y, bits, rng) << bits;
-            pixel |= quantize_bounce(v.z, bits, rng) << (2 * bits);
-        } else {
-            pixel = quantize_bounce(v.x, bits, rng);
-        }
-        if (colored) {
-            // one bit stream, pixels 3*bits wide
-            acc |= (unsigned long long)pixel << acc_bits;
-            acc_bits += pixel_bits;
-            while (acc_bits >= 32) {
-                words[out++] = (uint32_t)acc;
-                acc >>= 32;
-                acc_bits -= 32;
-            }
-        } else {
-            // floor(32 / bits) pixels per word, the rest of each word left zero
-            uint32_t j = (uint32_t)(i % per);
-            acc |= (unsigned long long)pixel << (j * bits);
-            if (j == per - 1) {
-                words[out++] = (uint32_t)acc;
-                acc = 0;
+        const unsigned r = __ballot_sync(all, mine && bounce_draws(v.x, bits));
+        const unsigned g = __ballot_sync(all, mine && colored && bounce_draws(v.y, bits));
+        const unsigned b = __ballot_sync(all, mine && colored && bounce_draws(v.z, bits));
+        const unsigned below = (1u << lane) - 1u;
+        uint32_t pixel = 0;
+        if (mine) {
+            Pcg own = rng;
+            own.advance(__popc(r & below) + __popc(g & below) + __popc(b & below));
+            pixel = quantize_bounce(v.x, bits, own);
+            if (colored) {
+                pixel |= quantize_bounce(v.y, bits, own) << bits;
+                pixel |= quantize_bounce(v.z, bits, own) << (2 * bits);
             }
         }
+        rng.advance(__popc(r) + __popc(g) + __popc(b));
+        // lane j < round_words assembles word j
+        const uint64_t left = n - at;
+        const uint32_t have = left < pixels ? (uint32_t)left : pixels;  // pixels of this round
+        const uint32_t used = colored ? (have * pixel_bits + 31) / 32 : (have + per - 1) / per;
+        const uint32_t first = colored ? lane * 32 / pixel_bits : lane * per;
+        const uint32_t most = colored ? 32 / pixel_bits + 2 : per;  // pixels that may touch a word
+        uint32_t word = 0;
+        for (uint32_t k = 0; k < most; ++k) {
+            const uint32_t from = first + k, value = __shfl_sync(all, pixel, from & 31u);
+            if (from >= have) continue;
+            const int shift = colored ? (int)(from * pixel_bits) - (int)(lane * 32) : (int)(k * bits);
+            if (shift >= 32) continue;
+            word |= shift >= 0 ? value << shift : value >> -shift;
+        }
+        if (lane < used) words[out + lane] = word;
     }
-    if (colored ? acc_bits > 0 : (n % per) != 0) words[out++] = (uint32_t)acc;
 }
 
 // pack_bounce(_rgb) for 8-bit bounce (bounce_pack.rs:28-86), which has no dither (its amplitude
@@ -3112,7 +3121,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
         LAUNCHED("k_crop");
         ++s.launches;
         if (bmap) {
-            k_pack_bounce<<<grid_for(kept), kBlock, 0, st>>>(sc, kept, entry_pair, entry_bdst, pair_tri, pair_light,
+            k_pack_bounce<<<grid_for((size_t)kept * 32), kBlock, 0, st>>>(sc, kept, entry_pair, entry_bdst, pair_tri, pair_light,
                                                              tri_crop, region_rect, woff, bmap, words);
             LAUNCHED("k_pack_bounce");
             k_pack_bounce8<<<grid_parts(kept), kBlock, 0, st>>>(

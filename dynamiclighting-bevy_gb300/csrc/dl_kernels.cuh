@@ -639,12 +639,16 @@ __device__ __forceinline__ Contribution sun_sample(const DevScene &sc, const Dev
     return c;
 }
 
-// quantize (bounce_pack.rs:74-86)
+// quantize (bounce_pack.rs:74-86), and whether it takes a draw.
+__device__ __forceinline__ float bounce_color(float value) { return isnan(value) ? 0.0f : clampf(value, 0.0f, 1.0f); }
+__device__ __forceinline__ bool bounce_draws(float value, uint32_t bits) {
+    return bits != 8 && bounce_color(value) > 0.001f;
+}
 __device__ __forceinline__ uint32_t quantize_bounce(float value, uint32_t bits, Pcg &rng) {
     float max = (float)((1u << bits) - 1);
-    float amplitude = bits == 8 ? 0.0f : bits == 6 ? 0.004f : bits == 5 ? 0.008f : 0.02f;
-    float color = isnan(value) ? 0.0f : clampf(value, 0.0f, 1.0f);
-    if (amplitude > 0.0f && color > 0.001f) color = fminf(color + rng.next_f32() * amplitude, 1.0f);
+    float amplitude = bits == 6 ? 0.004f : bits == 5 ? 0.008f : 0.02f;
+    float color = bounce_color(value);
+    if (bounce_draws(value, bits)) color = fminf(color + rng.next_f32() * amplitude, 1.0f);
     return f2u(sqrtf(color) * max);
 }
 
