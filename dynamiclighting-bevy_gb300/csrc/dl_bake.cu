@@ -494,12 +494,13 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, Tra
                     ortho_pair(nrm, side, across);
                     // in the shift-aligned coherent order when the sample count allows it: the
                     // warp's texels (neighbours) then trace their rank-k rays in about one direction
-                    const uint32_t n = sc.sky_samples;
-                    const bool aligned = n >= 16 && n <= kMaxOrdered && !(n & (n - 1));
-                    const uint32_t shift = aligned ? net_shift(n, off) : 0u;
-                    for (uint32_t k = sub; k < n; k += W) {
-                        uint32_t j = aligned ? shifted_sample(sc, n, shift, k) : sc.sky_order ? sc.sky_order[k] : k;
-                        if (!tr(cosine_direction_basis(nrm, side, across, spread(j, off, true)), INFINITY)) ++open;
+                    // (terrain with 200 samples in the net of 256: 22.7 ms, in index order 27.8 ms)
+                    const uint32_t n = sc.sky_samples, net = ordered_net(n, 16, kMaxOrdered);
+                    const uint32_t shift = net ? net_shift(net, off) : 0u, ranks = net ? net : n;
+                    for (uint32_t k = sub; k < ranks; k += W) {
+                        const uint32_t j = net ? shifted_sample(sc, net, shift, k) : sc.sky_order ? sc.sky_order[k] : k;
+                        if (j < n && !tr(cosine_direction_basis(nrm, side, across, spread(j, off, true)), INFINITY))
+                            ++open;
                     }
                 }
                 for (uint32_t o = 1; o < W; o <<= 1) open += __shfl_xor_sync(0xFFFFFFFFu, open, o);
@@ -638,8 +639,8 @@ struct BounceArgs {
 // lanes per (bounce pair, texel) item. Each round, lane k of a group evaluates sample
 // round * lanes + k; the group leader then adds the round's contributions in sample order, so
 // the sum is the reference's sequential one for any group size.
-// Sun gathers with a power-of-two sample count up to `buffered` take their samples in the
-// shift-aligned coherent order instead (shifted_sample): round r of every group in the warp
+// Sun gathers with a sample count that fills a net up to `buffered` (ordered_net) take their samples in
+// the shift-aligned coherent order instead (shifted_sample): round r of every group in the warp
 // traces ranks r * lanes + k, so the warp's texels (neighbours along a triangle) send their rays
 // in about the same directions. A sample whose closest hit faces the sun and is lit by it
 // stores its value, its index and its shadow ray's origin in the next free slot of the group's
@@ -711,18 +712,19 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
             }
         }
         if (!active) samples = 0;
-        const bool aligned = sun && samples >= 32 && samples <= a.buffered && !(samples & (samples - 1));
-        const uint32_t shift = aligned ? net_shift(samples, sg.off) : 0u;
+        const uint32_t net = sun && active && a.buffered ? ordered_net(samples, 32, a.buffered) : 0u;
+        const bool aligned = net != 0;
+        const uint32_t shift = aligned ? net_shift(net, sg.off) : 0u, ranks = aligned ? net : samples;
         FSum3<REFINE> sum;
         uint32_t filled = 0;  // aligned sun gathers: scratch slots filled so far (the same in the group)
-        const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, (samples + W - 1) / W);
+        const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, (ranks + W - 1) / W);
         for (uint32_t r = 0; r < rounds; ++r) {
             const uint32_t k = r * W + sub;
             if (aligned) {
                 SunHit h{f3{0.0f, 0.0f, 0.0f}, f3{0.0f, 0.0f, 0.0f}, false};
-                uint32_t i = 0;
-                if (k < samples) {
-                    i = shifted_sample(sc, samples, shift, k);
+                uint32_t i = samples;
+                if (k < net) i = shifted_sample(sc, net, shift, k);
+                if (i < samples) {
                     h = sun_hit<COUNT, REFINE>(sc, sc.lights[s], origin, normal, sg, i, my, kBlock, &vis);
                     rays += h.pending ? 2 : 1;
                 }
@@ -784,7 +786,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
                     scratch[2 * rank + 1] = v;
                 }
             }
-            for (uint32_t u = 0; u < samples / 32; ++u) open_count += __popc(lit[u] & ~blocked[u]);
+            for (uint32_t u = 0; u < net / 32; ++u) open_count += __popc(lit[u] & ~blocked[u]);
         }
         __syncwarp();
         if (aligned) {
@@ -2498,14 +2500,15 @@ GatherKernel gather_kernel(bool refine, uint32_t minb, bool count = false) {
 size_t gather_smem(uint32_t depth, uint32_t lanes, uint32_t buffered) {
     return (size_t)depth * kBlock * sizeof(int) + (size_t)(kBlock / lanes) * 2 * (buffered / 32) * sizeof(uint32_t);
 }
-// The samples a lane group holds for aligned sun gathers: the largest power-of-two sun bounce
-// sample count from 32 to 256 (0 when there is none).
-uint32_t gather_buffer(const HostScene &h, uint32_t) {
+// The samples a lane group holds for aligned sun gathers: the largest net of a sun's bounce samples,
+// from 32 to 256 (0 when there is none). Under a device-memory cap only counts that are powers of two
+// themselves take the scratch that this needs; others gather without it.
+uint32_t gather_buffer(const dl_session &s) {
     uint32_t most = 0;
-    for (const DevLight &l : h.lights)
+    for (const DevLight &l : s.host.lights)
         if (l.shape == DL_SHAPE_SUN && (l.flags & kLightBounce)) {
-            uint32_t n = l.bounce_samples;
-            if (n >= 32 && n <= 256 && !(n & (n - 1))) most = std::max(most, n);
+            const uint32_t n = l.bounce_samples, net = ordered_net(n, 32, 256);
+            if (net == n || !s.budget.cap) most = std::max(most, net);
         }
     return most;
 }
@@ -2523,7 +2526,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     auto blocks_for = [&](uint32_t minb, uint32_t w) {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_kernel(refine, minb), kBlock,
-                                                         gather_smem(best.stack_depth, w, gather_buffer(s.host, w))));
+                                                         gather_smem(best.stack_depth, w, gather_buffer(s))));
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
@@ -2538,7 +2541,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     // the refined gather always takes 8 (64 registers: 173 ms on the outdoor scene against 178 ms at
     // 80 registers and 173 ms at 48, its binary64 re-tests spill)
     best.minb = minbs[0];
-    best.buffered = gather_buffer(s.host, best.lanes);
+    best.buffered = gather_buffer(s);
     best.blocks = blocks_for(best.minb, best.lanes);
     if (c.no_autotune || !every || minbs.size() == 1 || (progress && progress->cancel))
         return best;

@@ -56,6 +56,14 @@ struct DevScene {
     const uint16_t *order_cells, *cell_samples;
 };
 constexpr uint32_t kMaxOrdered = 4096;
+// The net that n samples are traced in the coherent order of: n itself when it is a power of two, else
+// the next one, as long as n fills five eighths of it (a lane idles where the order's sample is n or
+// more); 0: no such net. The first n points of the sequence are the first n of any larger net.
+__host__ __device__ __forceinline__ uint32_t ordered_net(uint32_t n, uint32_t least, uint32_t most) {
+    uint32_t net = least;
+    while (net < n && net < most) net *= 2;
+    return n <= net && 8ull * n >= 5ull * net ? net : 0;
+}
 // The shift of a net of n samples (n a power of two from 16 to kMaxOrdered) by `off` in whole
 // cells, packed as x | y << 8 | xbits << 16 | ybits << 24.
 __device__ __forceinline__ uint32_t net_shift(uint32_t n, f2 off) {
