@@ -278,7 +278,7 @@ template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_burial(DevScene sc, uint32_t texels, const uint32_t *tex_xy,
                                                    const float4 *tex_pos, const uint32_t *tex_tri,
                                                    const float4 *tri_face, uint8_t *buried, Counters *ctr) {
-    extern __shared__ int stack[];
+    int stack[kStack];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t rays = 0;
     Visits vis{0, 0, 0};
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kBlock) k_burial(DevScene sc, uint32_t texels,
         f3 origin = add(f3{p.x, p.y, p.z}, scale(normal, kRayOffset));
         Pcg rng = stream6(sc.seed, sc.mesh_id[m], kBurialStream, t - sc.mesh_tri_base[m], xy & 0xFFFFu, xy >> 16);
         float turn = rng.next_f32();
-        buried[i] = is_buried<REFINE>(sc, normal, origin, turn, stack + threadIdx.x, kBlock, rays, &vis) ? 1 : 0;
+        buried[i] = is_buried<REFINE>(sc, normal, origin, turn, stack, rays, &vis) ? 1 : 0;
     }
     unsigned r = __reduce_add_sync(0xFFFFFFFFu, rays);
     if (lane_id() == 0 && r) atomicAdd(&ctr->burial_rays, (unsigned long long)r);
@@ -382,7 +382,7 @@ __device__ __forceinline__ void store_texel(const DevScene &sc, const TraceArgs 
 // One (pair, texel) of the visibility loop (mesh_bake.rs:231-248); returns the rays traced.
 template <bool COUNT = false, bool REFINE = false>
 __device__ __forceinline__ uint32_t trace_texel(const DevScene &sc, const TraceArgs &a, uint32_t p, uint32_t k,
-                                                int *stack, int stride, Visits *vis = nullptr) {
+                                                int *stack, Visits *vis = nullptr) {
     uint32_t t = a.pair_tri[p], s = a.pair_light[p];
     uint32_t m = sc.tri_mesh[t];
     uint32_t ci = a.ctex_off[t] + k;
@@ -392,7 +392,7 @@ __device__ __forceinline__ uint32_t trace_texel(const DevScene &sc, const TraceA
     f3 pos{pp.x, pp.y, pp.z}, nrm{nn.x, nn.y, nn.z};
     f3 origin = add(pos, scale(f3{f.x, f.y, f.z}, kRayOffset));
     const DevLight &l = sc.lights[s];
-    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack, stride, vis};
+    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack, vis};
     Vis v = texel_shadow(sc, s, sc.mesh_id[m], x, y, pos, nrm, tr);
     if (!v.some) return 0;
     store_texel(sc, a, m, s, x, y, v.level, l.shadow_bits);
@@ -446,12 +446,10 @@ __device__ __forceinline__ unsigned long long claim(const TraceArgs &a, unsigned
 // run first in a grouped phase: W = sky_lanes lanes share one texel, each tracing every W-th rank
 // of its samples in the shift-aligned coherent order, and the open counts are summed across the
 // group (an integer sum, so the level is the same as one lane tracing them all in index order).
-// MINB is the launch bound's blocks per SM (the register budget). The stack lives in dynamic
-// shared memory.
+// MINB is the launch bound's blocks per SM (the register budget).
 template <bool COUNT, bool REFINE, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, TraceArgs a) {
-    extern __shared__ int stack[];
-    int *my = stack + threadIdx.x;
+    int stack[kStack];
     unsigned lane = lane_id();
     unsigned long long rays = 0;
     Visits vis{0, 0, 0};
@@ -484,7 +482,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, Tra
                     f3 nrm{nn.x, nn.y, nn.z};
                     f3 origin = add(f3{pp.x, pp.y, pp.z}, scale(f3{f.x, f.y, f.z}, kRayOffset));
                     const DevLight &l = sc.lights[s];
-                    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, my, kBlock, &vis};
+                    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack,  &vis};
                     // sky_visibility (sky.rs:30-44), samples sub, sub + W, ...
                     Pcg rng = stream5(sc.seed, sc.mesh_id[m], l.id, x, y);
                     f2 off;
@@ -522,8 +520,8 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, Tra
             unsigned long long item = base + (unsigned long long)g * 32 + lane;
             if (item < a.items) {
                 while ((unsigned long long)a.item_off[cur + 1] <= item) ++cur;
-                rays += trace_texel<COUNT, REFINE>(sc, a, a.order[cur], (uint32_t)(item - a.item_off[cur]), my,
-                                                   kBlock, &vis);
+                rays += trace_texel<COUNT, REFINE>(sc, a, a.order[cur], (uint32_t)(item - a.item_off[cur]), stack,
+                                                    &vis);
             }
         }
     }
@@ -542,8 +540,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, Tra
 // Plain form: one launch per mesh; a warp per triangle, its lights in order, lanes over texels.
 __global__ void __launch_bounds__(kBlock) k_trace_plain(DevScene sc, TraceArgs a, uint32_t first_tri,
                                                          uint32_t tri_count, const uint32_t *tri_pair_off) {
-    __shared__ int stack[kStack * kBlock];
-    int *my = stack + threadIdx.x;
+    int stack[kStack];
     unsigned lane = lane_id();
     unsigned long long rays = 0;
     uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -551,7 +548,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_plain(DevScene sc, TraceArgs a
         uint32_t t = first_tri + w;
         uint32_t n = a.ctex_off[t + 1] - a.ctex_off[t];
         for (uint32_t p = tri_pair_off[t]; p < tri_pair_off[t + 1]; ++p)
-            for (uint32_t k = lane; k < n; k += 32) rays += trace_texel(sc, a, p, k, my, kBlock);
+            for (uint32_t k = lane; k < n; k += 32) rays += trace_texel(sc, a, p, k, stack);
     }
     unsigned long long r = warp_sum(rays);
     if (lane == 0 && r) atomicAdd(&a.ctr->rays, r);
@@ -593,7 +590,7 @@ __global__ void k_item_counts(const uint32_t *order, const uint32_t *pair_tri, c
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_photons(DevScene sc, const uint32_t *cube_lights, uint32_t cubes,
                                                     uint32_t res, Photon *photons, Counters *ctr) {
-    extern __shared__ int stack[];
+    int stack[kStack];
     uint64_t per = 6ull * res * res;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     Visits vis{0, 0, 0};
@@ -602,7 +599,7 @@ __global__ void __launch_bounds__(kBlock) k_photons(DevScene sc, const uint32_t 
         uint32_t rem = (uint32_t)(i % per);
         uint32_t face = rem / (res * res), y = (rem % (res * res)) / res, x = rem % res;
         const DevLight &l = sc.lights[cube_lights[cube]];
-        photons[i] = make_photon<REFINE>(sc, l, cube_texel_direction(face, x, y, res), stack + threadIdx.x, kBlock,
+        photons[i] = make_photon<REFINE>(sc, l, cube_texel_direction(face, x, y, res), stack,
                                          &vis);
     }
     if (REFINE) add_retests(ctr, vis.retests);
@@ -628,7 +625,6 @@ struct BounceArgs {
     Counters *ctr;
     uint32_t lanes;         // lanes sharing one texel's samples (1, 2, 4, 8, 16 or 32)
     uint32_t sample_every;  // tuning trials: one claimed step in `sample_every` (1: all)
-    uint32_t stack_depth;   // shared-memory stack entries per thread
     uint32_t buffered;      // sun samples a lane group can hold for the aligned order (0: none)
     float4 *scratch;        // per lane group (blockIdx * groups + group): 2 * buffered float4
     unsigned long long *head;  // steps claimed so far (32 / lanes items per step)
@@ -650,20 +646,20 @@ struct BounceArgs {
 // (parallel rays towards the sun), marking blocked ones in a second mask; each open sample's
 // value then moves to its rank among the open samples (popcounts of the masks), and the group
 // loads those values W at a time while the leader adds them, in sample order, as the reference
-// does (sun_bounce.rs:70). Dynamic shared memory holds only the traversal stacks and the groups'
-// masks (the per-round contributions go to the leader by shuffles), so that the rest of each SM's
+// does (sun_bounce.rs:70). Dynamic shared memory holds only the groups' masks
+// (the per-round contributions go to the leader by shuffles), so that the rest of each SM's
 // unified L1/shared memory stays L1 cache for the BVH. MINB is the launch bound's blocks per SM
 // (the register budget: 6, 8, 9 and 10 give 80, 64, 56 and 48 registers a thread).
 template <bool COUNT, bool REFINE, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs a) {
-    extern __shared__ int smem[];
-    int *my = smem + threadIdx.x;
+    extern __shared__ uint32_t masks[];
+    int stack[kStack];
     const uint32_t lane = lane_id(), W = a.lanes, sub = lane % W, per_step = 32 / W;
     // this lane group's masks (shared memory: samples whose hit is lit, then those whose shadow
     // ray is blocked) and scratch (global memory) for aligned sun gathers
     const uint32_t group = (threadIdx.x >> 5) * per_step + lane / W, words = a.buffered / 32;
     const unsigned group_lanes = W == 32 ? 0xFFFFFFFFu : ((1u << W) - 1u) << (lane / W * W);
-    uint32_t *lit = reinterpret_cast<uint32_t *>(smem + (size_t)a.stack_depth * kBlock) + (size_t)group * 2 * words;
+    uint32_t *lit = masks + (size_t)group * 2 * words;
     uint32_t *blocked = lit + words;
     float4 *scratch = a.scratch + ((size_t)blockIdx.x * (kBlock / W) + group) * 2 * a.buffered;
     for (uint32_t w = sub; w < 2 * words; w += W) lit[w] = 0u;
@@ -725,7 +721,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
                 uint32_t i = samples;
                 if (k < net) i = shifted_sample(sc, net, shift, k);
                 if (i < samples) {
-                    h = sun_hit<COUNT, REFINE>(sc, sc.lights[s], origin, normal, sg, i, my, kBlock, &vis);
+                    h = sun_hit<COUNT, REFINE>(sc, sc.lights[s], origin, normal, sg, i, stack,  &vis);
                     rays += h.pending ? 2 : 1;
                 }
                 // the group's pending samples of this round take the next slots, in lane order
@@ -743,9 +739,9 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
             if (k < samples) {
                 const DevLight &l = sc.lights[s];
                 if (sun) {
-                    c = sun_sample<COUNT, REFINE>(sc, l, origin, normal, sg, k, my, kBlock, &vis);
+                    c = sun_sample<COUNT, REFINE>(sc, l, origin, normal, sg, k, stack,  &vis);
                 } else {
-                    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, my, kBlock, &vis};
+                    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack,  &vis};
                     c = local_sample(sc, l, a.photons + (size_t)l.cube * 6 * a.res * a.res, a.res, normal, lg, k, tr);
                     lg.rng.advance(2ull * (W - 1));  // to the lane's next sample, k + W
                 }
@@ -767,7 +763,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
             for (uint32_t j = sub; j < filled; j += W) {
                 const float4 q = scratch[2 * j + 1];
                 const uint32_t i = __float_as_uint(scratch[2 * j].w);
-                if (!sun_open<COUNT, REFINE>(sc, sc.lights[s], f3{q.x, q.y, q.z}, my, kBlock, &vis))
+                if (!sun_open<COUNT, REFINE>(sc, sc.lights[s], f3{q.x, q.y, q.z}, stack,  &vis))
                     atomicOr(&blocked[i >> 5], 1u << (i & 31u));
             }
         }
@@ -836,7 +832,7 @@ constexpr uint64_t kProbeStream = 0x736b7970726f6265ull;  // PROBE_STREAM (sky_p
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_distance_cubes(DevScene sc, uint32_t lights, uint32_t *out,
                                                            Counters *ctr) {
-    extern __shared__ int stack[];
+    int stack[kStack];
     const uint32_t per_face = kCubeRes * kCubeRes / 2;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     Visits vis{0, 0, 0};
@@ -849,7 +845,7 @@ __global__ void __launch_bounds__(kBlock) k_distance_cubes(DevScene sc, uint32_t
             f3 dir = cube_texel_direction(face, texel % kCubeRes, texel / kCubeRes, kCubeRes);
             Hit h;
             d[k] = traverse<false, false, REFINE>(sc, L.position, dir, L.radius, (L.flags & kLightAlpha) != 0,
-                                                  stack + threadIdx.x, kBlock, h, &vis)
+                                                  stack, h, &vis)
                        ? h.t
                        : L.radius;
         }
@@ -870,7 +866,7 @@ struct SunMapArgs {
 __device__ __forceinline__ uint32_t unorm16(float d) { return f2u(roundf(clampf(d, 0.0f, 1.0f) * 65535.0f)); }
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_sun_map(DevScene sc, SunMapArgs a, Counters *ctr) {
-    extern __shared__ int stack[];
+    int stack[kStack];
     uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
     Visits vis{0, 0, 0};
     if (w < a.words) {
@@ -883,8 +879,7 @@ __global__ void __launch_bounds__(kBlock) k_sun_map(DevScene sc, SunMapArgs a, C
                 float down = a.bmin.y + ((float)(i / a.res) + 0.5f) * a.texel;
                 f3 origin = add(add(scale(a.side, across), scale(a.up, down)), scale(a.along, a.bmin.z));
                 Hit h;
-                if (traverse<false, false, REFINE>(sc, origin, a.along, a.depth, a.alpha != 0, stack + threadIdx.x,
-                                                   kBlock, h, &vis))
+                if (traverse<false, false, REFINE>(sc, origin, a.along, a.depth, a.alpha != 0, stack, h, &vis))
                     d[k] = h.t / a.depth;
             }
         }
@@ -909,7 +904,7 @@ struct ProbeArgs {
 constexpr uint32_t kProbeLanes = 8;
 template <bool REFINE>
 __global__ void __launch_bounds__(kBlock) k_sky_probes(DevScene sc, ProbeArgs a, Counters *ctr) {
-    extern __shared__ int stack[];
+    int stack[kStack];
     const unsigned long long thread = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x, i = thread / kProbeLanes;
     const uint32_t sub = (uint32_t)(thread % kProbeLanes);
     Visits vis{0, 0, 0};
@@ -935,8 +930,7 @@ __global__ void __launch_bounds__(kBlock) k_sky_probes(DevScene sc, ProbeArgs a,
         for (uint32_t taken = sub; taken < samples; taken += kProbeLanes) {
             f3 dir = cosine_direction_basis(normal, side, across, spread(taken, off, true));
             Hit h;
-            bool found = traverse<false, false, REFINE>(sc, position, dir, INFINITY, a.alpha != 0, stack + threadIdx.x,
-                                                        kBlock, h, &vis) &&
+            bool found = traverse<false, false, REFINE>(sc, position, dir, INFINITY, a.alpha != 0, stack, h, &vis) &&
                          h.t > 0.0f;
             if (found && dot(hit_face_normal(sc, h), dir) > 0.0f) ++back;
             if (!found) ++open;
@@ -1893,12 +1887,9 @@ struct dl_session {
 namespace dl {
 namespace {
 
-// Stack entries per thread that the scene's tree needs, rounded up to 4, and the shared memory of a
-// launch whose threads hold one stack each. Sized by the tree (8 to 28 entries on the workloads) instead
-// of by the deepest tree accepted (64, 32 KB a block, at most 7 blocks per SM): the room grid's photon cubes
-// took 7.1 ms and take 5.7 ms, burial of the outdoor level 3.5 ms and 2.6 ms.
+// Stack entries per thread that the scene's tree needs, rounded up to 4 (what the report names; the
+// stacks themselves are kStack entries of local memory).
 uint32_t stack_depth(const dl_session &s) { return std::max<uint32_t>(8, (s.host.bvh_depth + 3) & ~3u); }
-size_t stack_smem(const dl_session &s) { return (size_t)stack_depth(s) * kBlock * sizeof(int); }
 
 void scan_u32(dl_session &s, const uint32_t *in, uint32_t *out, size_t n) {
     size_t temp = 0;
@@ -2346,9 +2337,7 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 // ---- launch shapes of the batched visibility and gather kernels ---------------------------------
 // Knobs: chunk size (warp-steps per claimed chunk), lanes sharing one sky texel's or gathered texel's
 // samples, the launch bound's blocks per SM (the register budget: 7, 8, 9, 10 or 12 blocks of 128
-// threads give 72, 64, 56, 48 or 40 registers per thread; the gather's 6 gives 80) and the stack depth
-// (the BVH's depth, rounded up; it sets the shared memory per block and so, with the registers, the
-// resident blocks). A rule picks the shape:
+// threads give 72, 64, 56, 48 or 40 registers per thread; the gather's 6 gives 80). A rule picks the shape:
 // - sky lanes grow with the sample count, 8 from 256 samples, 4 from 128, 2 from 64, but at most 4 from
 //   4 M items. Lanes that share a texel's aligned samples trace neighbouring directions, and few texels
 //   with long sample loops leave the last warps alone. Visibility of a terrain tile (0.5 M items, 256
@@ -2406,8 +2395,7 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
     best.stack_depth = stack_depth(s);
     auto blocks_for = [&](uint32_t minb) {
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(count, refine, minb), kBlock,
-                                                         (size_t)best.stack_depth * kBlock * sizeof(int)));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(count, refine, minb), kBlock, 0));
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
@@ -2454,8 +2442,7 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
         const uint32_t blocks = blocks_for(minb);
         CK(cudaMemsetAsync(ta.head, 0, 2 * sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
-        trace_kernel(count, refine, minb)<<<blocks, kBlock, (size_t)best.stack_depth * kBlock * sizeof(int), st>>>(
-            s.sc, ta);
+        trace_kernel(count, refine, minb)<<<blocks, kBlock, 0, st>>>(s.sc, ta);
         CK(cudaGetLastError());
         CK(cudaEventRecord(b, st));
         CK(cudaEventSynchronize(b));
@@ -2482,23 +2469,18 @@ struct GatherTune {
     double ms = 0.0;
 };
 using GatherKernel = void (*)(DevScene, BounceArgs);
-// The gather kernel of a variant, allowed kGatherSmemMax bytes of dynamic shared memory (above
-// the default 48 KB: 16-lane groups of 256 buffered samples need 74 KB with a 64-entry stack).
-constexpr int kGatherSmemMax = 80 * 1024;
 GatherKernel gather_kernel(bool refine, uint32_t minb, bool count = false) {
-    GatherKernel k = count    ? k_gather<true, false, 6>
-                     : refine ? k_gather<false, true, 8>
-                     : minb == 8  ? k_gather<false, false, 8>
-                     : minb == 9  ? k_gather<false, false, 9>
-                     : minb == 10 ? k_gather<false, false, 10>
-                                  : k_gather<false, false, 6>;
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherSmemMax));
-    return k;
+    return count    ? k_gather<true, false, 6>
+           : refine ? k_gather<false, true, 8>
+           : minb == 8  ? k_gather<false, false, 8>
+           : minb == 9  ? k_gather<false, false, 9>
+           : minb == 10 ? k_gather<false, false, 10>
+                        : k_gather<false, false, 6>;
 }
-// Shared memory of a gather launch: stacks and, for aligned sun gathers, two masks of `buffered`
-// bits per lane group (kept small: what the block does not take stays L1 cache for the BVH).
-size_t gather_smem(uint32_t depth, uint32_t lanes, uint32_t buffered) {
-    return (size_t)depth * kBlock * sizeof(int) + (size_t)(kBlock / lanes) * 2 * (buffered / 32) * sizeof(uint32_t);
+// Shared memory of a gather launch: for aligned sun gathers two masks of `buffered` bits per lane
+// group (at most 8 KB).
+size_t gather_smem(uint32_t lanes, uint32_t buffered) {
+    return (size_t)(kBlock / lanes) * 2 * (buffered / 32) * sizeof(uint32_t);
 }
 // The samples a lane group holds for aligned sun gathers: the largest net of a sun's bounce samples,
 // from 32 to 256 (0 when there is none). Under a device-memory cap only counts that are powers of two
@@ -2526,7 +2508,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     auto blocks_for = [&](uint32_t minb, uint32_t w) {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_kernel(refine, minb), kBlock,
-                                                         gather_smem(best.stack_depth, w, gather_buffer(s))));
+                                                         gather_smem(w, gather_buffer(s))));
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
@@ -2560,7 +2542,6 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     cudaStream_t st = s.stream;
     ba.ctr = s.pool.get<Counters>("tune_counters", 1);
     ba.sample_every = every;
-    ba.stack_depth = best.stack_depth;
     cudaEvent_t a, b;
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
@@ -2573,7 +2554,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
         ba.scratch = gather_scratch(s, blocks, best.lanes, ba.buffered);
         CK(cudaMemsetAsync(ba.head, 0, sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
-        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.stack_depth, best.lanes, ba.buffered), st>>>(
+        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.lanes, ba.buffered), st>>>(
             s.sc, ba);
         CK(cudaGetLastError());
         CK(cudaEventRecord(b, st));
@@ -2613,7 +2594,7 @@ void bake_maps(dl_session &s, bool refine) {
         s.cube_word_count = (uint64_t)h.local_lights * 6 * kCubeRes * kCubeRes / 2;
         uint32_t *cubes = P.get<uint32_t>("cube_words", s.cube_word_count);
         (refine ? k_distance_cubes<true>
-                : k_distance_cubes<false>)<<<grid_for(s.cube_word_count), kBlock, stack_smem(s), st>>>(
+                : k_distance_cubes<false>)<<<grid_for(s.cube_word_count), kBlock, 0, st>>>(
             s.sc, h.local_lights, cubes, s.ctr);
         LAUNCHED("k_distance_cubes");
         ++s.launches;
@@ -2641,7 +2622,7 @@ void bake_maps(dl_session &s, bool refine) {
             a.words = (uint32_t)(((uint64_t)m.resolution * m.resolution + 1) / 2);
             a.alpha = (l.flags & kLightAlpha) != 0;
             a.out = P.get<uint32_t>("sun_map_" + std::to_string(s.sun_setups.size()), a.words);
-            (refine ? k_sun_map<true> : k_sun_map<false>)<<<grid_for(a.words), kBlock, stack_smem(s), st>>>(s.sc, a, s.ctr);
+            (refine ? k_sun_map<true> : k_sun_map<false>)<<<grid_for(a.words), kBlock, 0, st>>>(s.sc, a, s.ctr);
             LAUNCHED("k_sun_map");
             ++s.launches;
             texels = a.out;
@@ -2662,7 +2643,7 @@ void bake_maps(dl_session &s, bool refine) {
             a.open = P.get<float>("probe_open", a.jobs);
             a.back = P.get<uint32_t>("probe_back", a.jobs);
             (refine ? k_sky_probes<true>
-                    : k_sky_probes<false>)<<<grid_for(a.jobs * kProbeLanes), kBlock, stack_smem(s), st>>>(s.sc, a, s.ctr);
+                    : k_sky_probes<false>)<<<grid_for(a.jobs * kProbeLanes), kBlock, 0, st>>>(s.sc, a, s.ctr);
             LAUNCHED("k_sky_probes");
             ++s.launches;
             s.probe_open = a.open;
@@ -2814,7 +2795,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
     CK(cudaEventRecord(s.marks[2], st));
     if (texels_all) {
         auto burial = refine ? k_burial<true> : k_burial<false>;
-        burial<<<grid_for(texels_all), kBlock, stack_smem(s), st>>>(sc, texels_all, tex_xy, tex_pos, tex_tri, tri_face, buried,
+        burial<<<grid_for(texels_all), kBlock, 0, st>>>(sc, texels_all, tex_xy, tex_pos, tex_tri, tri_face, buried,
                                                         s.ctr);
         LAUNCHED("k_burial");
         ++s.launches;
@@ -2918,7 +2899,6 @@ dl_status run(dl_session &s, dl_progress *progress) {
         ta.grab = tune.grab;
         ta.sky_lanes = tune.sky_lanes;
         auto trace = trace_kernel(count, refine, tune.minb);
-        const size_t smem = (size_t)tune.stack_depth * kBlock * sizeof(int);
         const unsigned blocks = tune.blocks;
         // The visibility stage runs from a CUDA graph: the memset of the queue heads and the
         // persistent kernel, captured once per queue layout and launch shape and replayed.
@@ -2932,7 +2912,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
             cudaGraph_t g;
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             cudaMemsetAsync(heads, 0, 2 * sizeof(unsigned long long), st);
-            if (items) trace<<<blocks, kBlock, smem, st>>>(sc, ta);
+            if (items) trace<<<blocks, kBlock, 0, st>>>(sc, ta);
             CK(cudaStreamEndCapture(st, &g));
             CK(cudaGraphInstantiate(&s.graph, g, 0));
             cudaGraphDestroy(g);
@@ -2965,7 +2945,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
             uint32_t *cube_lights = P.get<uint32_t>("cube_lights", cubes);
             CK(cudaMemcpyAsync(cube_lights, hs.cube_lights.data(), cubes * 4ull, cudaMemcpyHostToDevice, st));
             auto photon = refine_bounce ? k_photons<true> : k_photons<false>;
-            photon<<<grid_for(photons_n), kBlock, stack_smem(s), st>>>(sc, cube_lights, cubes, res, photons, s.ctr);
+            photon<<<grid_for(photons_n), kBlock, 0, st>>>(sc, cube_lights, cubes, res, photons, s.ctr);
             LAUNCHED("k_photons");
             ++s.launches;
         }
@@ -3009,7 +2989,6 @@ dl_status run(dl_session &s, dl_progress *progress) {
             ba.sample_every = 1;
             GatherTune g = gather_tune(s, ba, bcount, refine_bounce, progress);
             ba.lanes = g.lanes;
-            ba.stack_depth = g.stack_depth;
             ba.buffered = g.buffered;
             ba.scratch = gather_scratch(s, g.blocks, g.lanes, g.buffered);
             s.report.tuned_gather_lanes = g.lanes;
@@ -3021,7 +3000,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
             // the instrumented variant (counting node visits and triangle tests) when asked
             CK(cudaEventRecord(g0, st));
             gather_kernel(refine_bounce, g.minb, s.config.count_visits != 0 && !refine_bounce)<<<
-                g.blocks, kBlock, gather_smem(g.stack_depth, g.lanes, g.buffered), st>>>(sc, ba);
+                g.blocks, kBlock, gather_smem(g.lanes, g.buffered), st>>>(sc, ba);
             LAUNCHED("k_gather");
             CK(cudaEventRecord(g1, st));
             gathered = true;

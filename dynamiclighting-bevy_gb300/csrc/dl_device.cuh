@@ -214,7 +214,12 @@ __device__ __forceinline__ bool tri_test_refined(const DevScene &sc, float4 v0, 
     return tri_test_fp64(sc, __float_as_uint(v0.w), o, d, max, t, u, v);
 }
 
-constexpr int kStack = 64;  // >= BVH depth; the host refuses deeper trees
+// Entries of a traversal stack (>= BVH depth; the host refuses deeper trees). A thread's stack is local
+// memory: a ray holds a few entries of the 8 to 28 that its tree could need, and only the lines in use take
+// room in L1, where shared stacks took their worst case from it for every resident thread (14 KB a block
+// of the outdoor level, 140 KB of the SM's 256). Shared -> local: the outdoor quarter's visibility 24.6 ->
+// 23.5 ms at 10 blocks, the rooms' local gather 24.9 -> 23.7 ms at 8, rooms under panels and tubes 6.4 -> 6.2 ms.
+constexpr int kStack = 64;
 
 // A node's 64 bytes in two 32-byte loads.
 struct NodeData {
@@ -274,16 +279,16 @@ __device__ __forceinline__ bool refined_candidate(const DevScene &sc, f3 o, f3 d
 }
 
 template <bool COUNT>
-__device__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, int stride,
-                              Hit &hit, Visits *vis);
+__device__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, Hit &hit,
+                              Visits *vis);
 
 // Any-hit (ANY) or closest-hit traversal of the BVH2. Child references: >= 0 an inner node,
-// < 0 a leaf ~(first << 3 | count). `stack` points at this thread's first stack slot in shared
-// memory, slots `stride` apart. For closest-hit, `hit` gets the nearest t (ties to the lowest
+// < 0 a leaf ~(first << 3 | count). `stack` is this thread's kStack entries in local
+// memory. For closest-hit, `hit` gets the nearest t (ties to the lowest
 // occluder index, as occluder.rs:205-210) and that test's barycentrics, which equal the ones
 // the reference recomputes with max = infinity.
 template <bool ANY, bool COUNT = false, bool REFINE = false, bool EACH = false>
-__device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, int stride, Hit &hit,
+__device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, Hit &hit,
                          Visits *vis = nullptr) {
     hit.t = INFINITY;
     hit.u = hit.v = 0.0f;
@@ -311,14 +316,14 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
             const int r0 = nd.ref0, r1 = nd.ref1;
             if (h0 && h1) {
                 bool swap = n1 < n0;
-                stack[sp * stride] = swap ? r0 : r1;
+                stack[sp] = swap ? r0 : r1;
                 ++sp;
                 ref = swap ? r1 : r0;
             } else if (h0 || h1) {
                 ref = h0 ? r0 : r1;
             } else {
                 if (sp == 0) goto done;
-                ref = stack[--sp * stride];
+                ref = stack[--sp];
             }
         }
         while (ref < 0) {
@@ -352,7 +357,7 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
                 }
             }
             if (sp == 0) goto done;
-            ref = stack[--sp * stride];
+            ref = stack[--sp];
         }
     }
 done:
@@ -362,22 +367,22 @@ done:
             ++vis->retests;
             if (!tri_test_fp64(sc, hit.occluder, o, d, max, hit.t, hit.u, hit.v) || !isfinite(hit.t)) lost = true;
         }
-        if (!EACH && lost) return traverse_each<COUNT>(sc, o, dir, max, alpha, stack, stride, hit, vis);
+        if (!EACH && lost) return traverse_each<COUNT>(sc, o, dir, max, alpha, stack, hit, vis);
     }
     return found;
 }
 
 template <bool COUNT>
 __device__ __noinline__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack,
-                                           int stride, Hit &hit, Visits *vis) {
-    return traverse<false, COUNT, true, true>(sc, o, dir, max, alpha, stack, stride, hit, vis);
+                                           Hit &hit, Visits *vis) {
+    return traverse<false, COUNT, true, true>(sc, o, dir, max, alpha, stack, hit, vis);
 }
 
 template <bool COUNT = false, bool REFINE = false>
 __device__ __forceinline__ bool occluded(const DevScene &sc, f3 o, f3 d, float max, bool alpha, int *stack,
-                                         int stride, Visits *vis = nullptr) {
+                                         Visits *vis = nullptr) {
     Hit h;
-    return traverse<true, COUNT, REFINE>(sc, o, d, max, alpha, stack, stride, h, vis);
+    return traverse<true, COUNT, REFINE>(sc, o, d, max, alpha, stack, h, vis);
 }
 
 }  // namespace dl

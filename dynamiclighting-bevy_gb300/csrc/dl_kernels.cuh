@@ -183,10 +183,9 @@ struct Tracer {
     f3 origin;
     bool alpha;
     int *stack;
-    int stride;
     Visits *vis;
     __device__ __forceinline__ bool operator()(f3 dir, float dist) const {
-        return occluded<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, stride, vis);
+        return occluded<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
     }
 };
 
@@ -343,7 +342,7 @@ __device__ __forceinline__ Vis texel_shadow(const DevScene &sc, uint32_t slot, u
 // verdict and adds the rays traced to `rays`.
 template <bool REFINE = false>
 __device__ __forceinline__ bool is_buried(const DevScene &sc, f3 normal, f3 origin, float turn, int *stack,
-                                          int stride, uint32_t &rays, Visits *vis = nullptr) {
+                                          uint32_t &rays, Visits *vis = nullptr) {
     f3 tangent, bitangent;
     ortho_pair(normal, tangent, bitangent);
     uint32_t back = 0, front = 0;
@@ -358,7 +357,7 @@ __device__ __forceinline__ bool is_buried(const DevScene &sc, f3 normal, f3 orig
         ++rays;
         Hit h;
         bool backface = false;
-        if (traverse<false, false, REFINE>(sc, origin, dir, INFINITY, false, stack, stride, h, vis)) {
+        if (traverse<false, false, REFINE>(sc, origin, dir, INFINITY, false, stack, h, vis)) {
             // face normal of the hit occluder: cross(b - a, c - a), normalized
             const float4 *tp = sc.tris + (size_t)sc.occ_leaf[h.occluder] * 3;
             float4 e1 = ldg4(tp + 1), e2 = ldg4(tp + 2);
@@ -462,10 +461,10 @@ __device__ __forceinline__ f3 hit_albedo(const DevScene &sc, const Hit &h) {
 
 // photon (bounce.rs:88-115)
 template <bool REFINE = false>
-__device__ __forceinline__ Photon make_photon(const DevScene &sc, const DevLight &l, f3 dir, int *stack, int stride,
+__device__ __forceinline__ Photon make_photon(const DevScene &sc, const DevLight &l, f3 dir, int *stack,
                                               Visits *vis = nullptr) {
     Hit h;
-    if (!traverse<false, false, REFINE>(sc, l.position, dir, l.radius, (l.flags & kLightAlpha) != 0, stack, stride, h,
+    if (!traverse<false, false, REFINE>(sc, l.position, dir, l.radius, (l.flags & kLightAlpha) != 0, stack, h,
                                         vis))
         return Photon{l.radius, 0u, 0u};
     f3 face = hit_face_normal(sc, h);
@@ -602,12 +601,12 @@ struct SunHit {
 };
 template <bool COUNT, bool REFINE>
 __device__ __forceinline__ SunHit sun_hit(const DevScene &sc, const DevLight &l, f3 origin, f3 normal,
-                                          const SunGather &g, uint32_t i, int *stack, int stride, Visits *vis) {
+                                          const SunGather &g, uint32_t i, int *stack, Visits *vis) {
     SunHit r{f3{0.0f, 0.0f, 0.0f}, f3{0.0f, 0.0f, 0.0f}, false};
     bool alpha = (l.flags & kLightAlpha) != 0;
     f3 direction = cosine_direction_basis(normal, g.side, g.across, spread(i, g.off, true));
     Hit h;
-    if (!traverse<false, COUNT, REFINE>(sc, origin, direction, INFINITY, alpha, stack, stride, h, vis)) return r;
+    if (!traverse<false, COUNT, REFINE>(sc, origin, direction, INFINITY, alpha, stack, h, vis)) return r;
     f3 face = hit_face_normal(sc, h);
     if (dot(face, direction) >= 0.0f) return r;
     float lit = dot(hit_surface_normal(sc, h, face), l.toward);
@@ -619,20 +618,20 @@ __device__ __forceinline__ SunHit sun_hit(const DevScene &sc, const DevLight &l,
 }
 // Whether the shadow ray of a pending sun-bounce sample is open (sun_bounce.rs:67).
 template <bool COUNT, bool REFINE>
-__device__ __forceinline__ bool sun_open(const DevScene &sc, const DevLight &l, f3 point, int *stack, int stride,
+__device__ __forceinline__ bool sun_open(const DevScene &sc, const DevLight &l, f3 point, int *stack,
                                          Visits *vis) {
-    return !occluded<COUNT, REFINE>(sc, point, l.toward, INFINITY, (l.flags & kLightAlpha) != 0, stack, stride, vis);
+    return !occluded<COUNT, REFINE>(sc, point, l.toward, INFINITY, (l.flags & kLightAlpha) != 0, stack, vis);
 }
 // Sample i of gather_sun (sun_bounce.rs:53-71).
 template <bool COUNT, bool REFINE>
 __device__ __forceinline__ Contribution sun_sample(const DevScene &sc, const DevLight &l, f3 origin, f3 normal,
-                                                  const SunGather &g, uint32_t i, int *stack, int stride,
+                                                  const SunGather &g, uint32_t i, int *stack,
                                                   Visits *vis) {
     Contribution c{f3{0.0f, 0.0f, 0.0f}, false, 1};
-    SunHit h = sun_hit<COUNT, REFINE>(sc, l, origin, normal, g, i, stack, stride, vis);
+    SunHit h = sun_hit<COUNT, REFINE>(sc, l, origin, normal, g, i, stack, vis);
     if (!h.pending) return c;
     c.rays = 2;
-    if (sun_open<COUNT, REFINE>(sc, l, h.point, stack, stride, vis)) {
+    if (sun_open<COUNT, REFINE>(sc, l, h.point, stack, vis)) {
         c.value = h.value;
         c.add = true;
     }
