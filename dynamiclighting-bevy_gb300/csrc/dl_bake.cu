@@ -2518,7 +2518,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     std::vector<uint32_t> minbs = refine                ? std::vector<uint32_t>{8}
                                   : c.gather_min_blocks ? std::vector<uint32_t>{c.gather_min_blocks}
                                   : sun                 ? std::vector<uint32_t>{9, 10}
-                                                        : std::vector<uint32_t>{8, 9};
+                                                        : std::vector<uint32_t>{9, 8};
     const uint32_t every = ba.items >= (1u << 20) ? 32 : ba.items >= (1u << 18) ? 16 : 0;
     // the refined gather always takes 8 (64 registers: 173 ms on the outdoor scene against 178 ms at
     // 80 registers and 173 ms at 48, its binary64 re-tests spill)

@@ -287,7 +287,7 @@ __device__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool 
 // memory. For closest-hit, `hit` gets the nearest t (ties to the lowest
 // occluder index, as occluder.rs:205-210) and that test's barycentrics, which equal the ones
 // the reference recomputes with max = infinity.
-template <bool ANY, bool COUNT = false, bool REFINE = false, bool EACH = false>
+template <bool ANY, bool COUNT = false, bool REFINE = false, bool EACH = false, int FEW = 0>
 __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, Hit &hit,
                          Visits *vis = nullptr) {
     hit.t = INFINITY;
@@ -303,7 +303,11 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
     int ref = 0;
     // while-while traversal (Aila & Laine 2009): descend inner nodes until a leaf is reached,
     // then test leaves until an inner node comes off the stack, so a warp's lanes run the same
-    // loop body together instead of alternating node and leaf work per lane.
+    // loop body together instead of alternating node and leaf work per lane. With FEW the last lanes still
+    // among inner nodes, when fewer than that, wait for the others' leaves (which shorten those rays'
+    // ranges and bring their lanes back): the outdoor quarter's sun gather 19.6 ms without, 18.5, 18.2, 18.3 ms
+    // at 4, 8, 12. Other closest hits gain nothing (burial in rooms 0.38 -> 0.42 ms, photons 3.32 -> 3.39 ms), and
+    // any-hit rays lose 6 %.
     for (;;) {
         while (ref >= 0) {
             const NodeData nd = load_node(sc.nodes + ref);
@@ -325,6 +329,7 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
                 if (sp == 0) goto done;
                 ref = stack[--sp];
             }
+            if (FEW && __popc(__activemask()) < FEW) break;
         }
         while (ref < 0) {
             uint32_t packed = (uint32_t)(~ref);
@@ -376,6 +381,68 @@ template <bool COUNT>
 __device__ __noinline__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack,
                                            Hit &hit, Visits *vis) {
     return traverse<false, COUNT, true, true>(sc, o, dir, max, alpha, stack, hit, vis);
+}
+
+// Any-hit traversal that holds a ray's first leaf back and goes on among inner nodes until every lane
+// there holds one (speculative traversal, Aila & Laine 2009): more lanes take part in each triangle
+// test, for nodes that a blocked ray did not need. It pays for the local gather's rays, whose
+// directions differ from lane to lane (the room grid's gather 23.3 ms without, 22.0 ms), not for aligned ones (the
+// outdoor quarter's visibility 23.5 -> 24.0 ms) nor for those towards a light (rooms under panels and tubes 6.25 ->
+// 6.4 ms).
+template <bool COUNT, bool REFINE>
+__device__ __forceinline__ bool occluded_postponed(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack,
+                                                   Visits *vis) {
+    if (sc.occluders == 0) return false;
+    constexpr int kNone = 0, kDone = -2147483647 - 1;  // neither is a leaf's reference
+    const f3 d{dir.x + 0.0f, dir.y + 0.0f, dir.z + 0.0f};
+    const RaySlabs slabs = ray_slabs(o, d);
+    const float tmax = fmaxf(max, 0.0f);
+    int sp = 0, ref = 0, leaf = kNone;
+    auto pop = [&]() { return sp ? stack[--sp] : kDone; };
+    auto postpone = [&]() {
+        if (ref < 0 && ref != kDone) {
+            leaf = ref;
+            ref = pop();
+        }
+    };
+    for (;;) {
+        while (ref >= 0) {
+            const NodeData nd = load_node(sc.nodes + ref);
+            if (COUNT) ++vis->nodes;
+            bool h0, h1;
+            float n0, n1;
+            slab_pair(nd.c0, nd.c1, nd.h0, nd.h1, nd.cz, nd.hz, slabs, tmax, h0, h1, n0, n1);
+            const int r0 = nd.ref0, r1 = nd.ref1;
+            if (h0 && h1) {
+                const bool swap = n1 < n0;
+                stack[sp] = swap ? r0 : r1;
+                ++sp;
+                ref = swap ? r1 : r0;
+            } else if (h0 || h1) {
+                ref = h0 ? r0 : r1;
+            } else {
+                ref = pop();
+            }
+            if (leaf == kNone) postpone();
+            if (!__any_sync(__activemask(), leaf == kNone)) break;
+        }
+        while (leaf != kNone) {
+            const uint32_t packed = (uint32_t)(~leaf), first = packed >> 3, count = packed & 7u;
+            for (uint32_t k = 0; k < count; ++k) {
+                const float4 *tp = sc.tris + (size_t)(first + k) * 3;
+                const float4 v0 = ldg4(tp);
+                if (COUNT) ++vis->tris;
+                float t, u, v, err;
+                if ((REFINE ? tri_test_refined(sc, v0, ldg4(tp + 1), ldg4(tp + 2), o, d, max, t, u, v, vis, err)
+                            : tri_test(v0, ldg4(tp + 1), ldg4(tp + 2), o, d, max, t, u, v)) &&
+                    (!alpha || alpha_blocks(sc, __float_as_uint(v0.w), u, v)))
+                    return true;
+            }
+            leaf = kNone;
+            postpone();
+        }
+        if (ref == kDone) return false;
+    }
 }
 
 template <bool COUNT = false, bool REFINE = false>

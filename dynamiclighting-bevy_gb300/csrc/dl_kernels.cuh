@@ -187,6 +187,9 @@ struct Tracer {
     __device__ __forceinline__ bool operator()(f3 dir, float dist) const {
         return occluded<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
     }
+    __device__ __forceinline__ bool postponed(f3 dir, float dist) const {
+        return occluded_postponed<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
+    }
 };
 
 // adaptive_share (area.rs:98-126); `Trace(point, w, unblocked)` is false for a point that sends
@@ -567,7 +570,7 @@ __device__ __forceinline__ Contribution local_sample(const DevScene &sc, const D
     if (is_zero(pn) || distance <= 0.0f) return c;
     f3 d = divs(to_photon, distance);
     c.rays = 1;
-    if (!tr(d, distance)) {
+    if (!tr.postponed(d, distance)) {
         float weight = fmaxf(dot(normal, d), 0.0f) * fmaxf(dot(pn, neg(d)), 0.0f);
         f3 albedo{1.0f, 1.0f, 1.0f};
         if (sc.colored_bounce)
@@ -606,7 +609,7 @@ __device__ __forceinline__ SunHit sun_hit(const DevScene &sc, const DevLight &l,
     bool alpha = (l.flags & kLightAlpha) != 0;
     f3 direction = cosine_direction_basis(normal, g.side, g.across, spread(i, g.off, true));
     Hit h;
-    if (!traverse<false, COUNT, REFINE>(sc, origin, direction, INFINITY, alpha, stack, h, vis)) return r;
+    if (!traverse<false, COUNT, REFINE, false, 8>(sc, origin, direction, INFINITY, alpha, stack, h, vis)) return r;
     f3 face = hit_face_normal(sc, h);
     if (dot(face, direction) >= 0.0f) return r;
     float lit = dot(hit_surface_normal(sc, h, face), l.toward);
