@@ -380,7 +380,7 @@ __device__ __forceinline__ void store_texel(const DevScene &sc, const TraceArgs 
 }
 
 // One (pair, texel) of the visibility loop (mesh_bake.rs:231-248); returns the rays traced.
-template <bool COUNT = false, bool REFINE = false>
+template <bool COUNT = false, bool REFINE = false, NodeLoop LOCAL = NodeLoop::kPlain>
 __device__ __forceinline__ uint32_t trace_texel(const DevScene &sc, const TraceArgs &a, uint32_t p, uint32_t k,
                                                 int *stack, Visits *vis = nullptr) {
     uint32_t t = a.pair_tri[p], s = a.pair_light[p];
@@ -392,7 +392,7 @@ __device__ __forceinline__ uint32_t trace_texel(const DevScene &sc, const TraceA
     f3 pos{pp.x, pp.y, pp.z}, nrm{nn.x, nn.y, nn.z};
     f3 origin = add(pos, scale(f3{f.x, f.y, f.z}, kRayOffset));
     const DevLight &l = sc.lights[s];
-    Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack, vis};
+    Tracer<COUNT, REFINE, LOCAL> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack, vis};
     Vis v = texel_shadow(sc, s, sc.mesh_id[m], x, y, pos, nrm, tr);
     if (!v.some) return 0;
     store_texel(sc, a, m, s, x, y, v.level, l.shadow_bits);
@@ -446,8 +446,10 @@ __device__ __forceinline__ unsigned long long claim(const TraceArgs &a, unsigned
 // run first in a grouped phase: W = sky_lanes lanes share one texel, each tracing every W-th rank
 // of its samples in the shift-aligned coherent order, and the open counts are summed across the
 // group (an integer sum, so the level is the same as one lane tracing them all in index order).
-// MINB is the launch bound's blocks per SM (the register budget).
-template <bool COUNT, bool REFINE, int MINB>
+// MINB is the launch bound's blocks per SM (the register budget). Without SKY there is no grouped phase, and
+// rays towards local lights leave the leaf loop after each leaf (rooms under panels and tubes 6.2 -> 5.5 ms;
+// the same loop beside the grouped phase makes the outdoor quarter 23.6 -> 23.9 ms, so it stays out of there).
+template <bool COUNT, bool REFINE, int MINB, bool SKY = true>
 __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, TraceArgs a) {
     int stack[kStack];
     unsigned lane = lane_id();
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, Tra
     uint32_t grabs = 0;
     const uint32_t W = a.sky_lanes;
     unsigned long long first = 0;
-    if (a.sky_items) {
+    if (SKY && a.sky_items) {
         const uint32_t per_step = 32 / W, sub = lane % W;
         const unsigned long long end = a.sky_items;
         first = end;
@@ -520,8 +522,8 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace_batched(DevScene sc, Tra
             unsigned long long item = base + (unsigned long long)g * 32 + lane;
             if (item < a.items) {
                 while ((unsigned long long)a.item_off[cur + 1] <= item) ++cur;
-                rays += trace_texel<COUNT, REFINE>(sc, a, a.order[cur], (uint32_t)(item - a.item_off[cur]), stack,
-                                                    &vis);
+                rays += trace_texel<COUNT, REFINE, SKY ? NodeLoop::kPlain : NodeLoop::kOneLeaf>(
+                    sc, a, a.order[cur], (uint32_t)(item - a.item_off[cur]), stack, &vis);
             }
         }
     }
@@ -2346,10 +2348,12 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 //   samples) 0.39, 0.40, 0.43, 0.44, 0.46 ms.
 // - 10 blocks per SM with a sky, 8 without: the tile at 7, 8, 9, 10, 12 takes 10.1, 9.9, 9.6, 9.4, 9.5
 //   ms (sky rays wait on the tree's far nodes, more warps hide it), rooms under panels and tubes 7.0,
-//   6.9, 6.9, 7.0, 8.0 ms. Chunks of 32 items (the level: 64 take 1 % longer).
-// - gathers with a sun take 9 blocks and 8 lanes, from 1 M items 4 (tile, 1 to 32 lanes at 9 blocks:
+//   6.9, 6.9, 7.0, 8.0 ms (now 5.5, 5.6, 5.7 ms at 8, 9, 10). Chunks of 32 items (the level: 64 take 1 %
+//   longer).
+// - gathers with a sun take 10 blocks (the outdoor quarter 17.5 ms, at 9 17.7 ms) and 8 lanes, from 1 M items 4 (tile, 1 to 32 lanes at 9 blocks:
 //   11.8, 9.0, 8.1, 7.7, 7.8, 8.2 ms; 6, 8, 9, 10 blocks at 8 lanes: 9.0, 8.0, 7.7, 7.8 ms; the level at
-//   2, 4, 8 lanes: 84.3, 84.8, 87.2 ms), local ones alone 2 lanes at 8 (rooms: 8.7, 8.7, 9.2, 10.0, 11.5,
+//   2, 4, 8 lanes: 84.3, 84.8, 87.2 ms), local ones alone 2 lanes at 9 (rooms 22.0 ms,
+//   22.3 at 8; by lanes 8.7, 8.7, 9.2, 10.0, 11.5,
 //   15.9 ms), refined ones 4 lanes (terrain 63.4, 60.7, 59.3, 58.6, 58.3, 58.4 ms, decals 31.2, 29.2,
 //   29.3, 30.4, 32.4, 33.8 ms).
 // From 1 M visibility items (256 K gather items) neighbouring register budgets are tried too, each on a
@@ -2364,9 +2368,12 @@ struct TraceTune {
 };
 using TraceKernel = void (*)(DevScene, TraceArgs);
 
-TraceKernel trace_kernel(bool count, bool refine, uint32_t minb) {
+TraceKernel trace_kernel(bool count, bool refine, uint32_t minb, bool sky) {
     if (count) return refine ? k_trace_batched<true, true, 7> : k_trace_batched<true, false, 7>;
     if (refine) return k_trace_batched<false, true, 7>;
+    if (!sky && minb == 8) return k_trace_batched<false, false, 8, false>;
+    if (!sky && minb == 9) return k_trace_batched<false, false, 9, false>;
+    if (!sky && minb == 10) return k_trace_batched<false, false, 10, false>;
     switch (minb) {
         case 8: return k_trace_batched<false, false, 8>;
         case 9: return k_trace_batched<false, false, 9>;
@@ -2395,7 +2402,7 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
     best.stack_depth = stack_depth(s);
     auto blocks_for = [&](uint32_t minb) {
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(count, refine, minb), kBlock, 0));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(count, refine, minb, ta.sky_items != 0), kBlock, 0));
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
@@ -2442,7 +2449,7 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
         const uint32_t blocks = blocks_for(minb);
         CK(cudaMemsetAsync(ta.head, 0, 2 * sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
-        trace_kernel(count, refine, minb)<<<blocks, kBlock, 0, st>>>(s.sc, ta);
+        trace_kernel(count, refine, minb, ta.sky_items != 0)<<<blocks, kBlock, 0, st>>>(s.sc, ta);
         CK(cudaGetLastError());
         CK(cudaEventRecord(b, st));
         CK(cudaEventSynchronize(b));
@@ -2517,7 +2524,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     best.lanes = c.sample_lanes ? c.sample_lanes : refine || (sun && ba.items >= (1u << 20)) ? 4u : sun ? 8u : 2u;
     std::vector<uint32_t> minbs = refine                ? std::vector<uint32_t>{8}
                                   : c.gather_min_blocks ? std::vector<uint32_t>{c.gather_min_blocks}
-                                  : sun                 ? std::vector<uint32_t>{9, 10}
+                                  : sun                 ? std::vector<uint32_t>{10, 9}
                                                         : std::vector<uint32_t>{9, 8};
     const uint32_t every = ba.items >= (1u << 20) ? 32 : ba.items >= (1u << 18) ? 16 : 0;
     // the refined gather always takes 8 (64 registers: 173 ms on the outdoor scene against 178 ms at
@@ -2898,7 +2905,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
         s.report.ms_tune = tune.ms;
         ta.grab = tune.grab;
         ta.sky_lanes = tune.sky_lanes;
-        auto trace = trace_kernel(count, refine, tune.minb);
+        auto trace = trace_kernel(count, refine, tune.minb, ta.sky_items != 0);
         const unsigned blocks = tune.blocks;
         // The visibility stage runs from a CUDA graph: the memset of the queue heads and the
         // persistent kernel, captured once per queue layout and launch shape and replayed.

@@ -278,6 +278,14 @@ __device__ __forceinline__ bool refined_candidate(const DevScene &sc, f3 o, f3 d
     return t < hit.t || (t == hit.t && occ < hit.occluder);
 }
 
+// How a warp's lanes leave the traversal's two loops. Most of its idle lanes wait at their border (14 of 32
+// threads active). kFew: the last lanes still among inner nodes, when fewer than 8, wait for the others'
+// leaves, which shorten those rays' ranges and bring their lanes back: the outdoor quarter's sun gather 19.6 ms
+// plain, 18.5, 18.2, 18.3 ms at 4, 8, 12; other closest hits gain nothing (burial in rooms 0.38 -> 0.42 ms,
+// photons 3.32 -> 3.39 ms), any-hit rays lose 6 %. kOneLeaf: back to inner nodes after one leaf: the sun gather's shadow
+// rays (its 18.2 -> 17.7 ms) and rays towards local lights; the sky's and the sun's lose 2 to 10 %.
+enum class NodeLoop { kPlain, kFew, kOneLeaf };
+
 template <bool COUNT>
 __device__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, Hit &hit,
                               Visits *vis);
@@ -287,7 +295,7 @@ __device__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool 
 // memory. For closest-hit, `hit` gets the nearest t (ties to the lowest
 // occluder index, as occluder.rs:205-210) and that test's barycentrics, which equal the ones
 // the reference recomputes with max = infinity.
-template <bool ANY, bool COUNT = false, bool REFINE = false, bool EACH = false, int FEW = 0>
+template <bool ANY, bool COUNT = false, bool REFINE = false, bool EACH = false, NodeLoop LOOP = NodeLoop::kPlain>
 __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack, Hit &hit,
                          Visits *vis = nullptr) {
     hit.t = INFINITY;
@@ -303,11 +311,7 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
     int ref = 0;
     // while-while traversal (Aila & Laine 2009): descend inner nodes until a leaf is reached,
     // then test leaves until an inner node comes off the stack, so a warp's lanes run the same
-    // loop body together instead of alternating node and leaf work per lane. With FEW the last lanes still
-    // among inner nodes, when fewer than that, wait for the others' leaves (which shorten those rays'
-    // ranges and bring their lanes back): the outdoor quarter's sun gather 19.6 ms without, 18.5, 18.2, 18.3 ms
-    // at 4, 8, 12. Other closest hits gain nothing (burial in rooms 0.38 -> 0.42 ms, photons 3.32 -> 3.39 ms), and
-    // any-hit rays lose 6 %.
+    // loop body together instead of alternating node and leaf work per lane (NodeLoop varies it).
     for (;;) {
         while (ref >= 0) {
             const NodeData nd = load_node(sc.nodes + ref);
@@ -329,9 +333,9 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
                 if (sp == 0) goto done;
                 ref = stack[--sp];
             }
-            if (FEW && __popc(__activemask()) < FEW) break;
+            if (LOOP == NodeLoop::kFew && __popc(__activemask()) < 8) break;
         }
-        while (ref < 0) {
+        if (ref < 0) do {
             uint32_t packed = (uint32_t)(~ref);
             uint32_t first = packed >> 3, count = packed & 7u;
             for (uint32_t k = 0; k < count; ++k) {
@@ -363,7 +367,7 @@ __device__ bool traverse(const DevScene &sc, f3 o, f3 dir, float max, bool alpha
             }
             if (sp == 0) goto done;
             ref = stack[--sp];
-        }
+        } while (LOOP != NodeLoop::kOneLeaf && ref < 0);
     }
 done:
     if (!ANY && REFINE) {
@@ -445,11 +449,11 @@ __device__ __forceinline__ bool occluded_postponed(const DevScene &sc, f3 o, f3 
     }
 }
 
-template <bool COUNT = false, bool REFINE = false>
+template <bool COUNT = false, bool REFINE = false, NodeLoop LOOP = NodeLoop::kPlain>
 __device__ __forceinline__ bool occluded(const DevScene &sc, f3 o, f3 d, float max, bool alpha, int *stack,
                                          Visits *vis = nullptr) {
     Hit h;
-    return traverse<true, COUNT, REFINE>(sc, o, d, max, alpha, stack, h, vis);
+    return traverse<true, COUNT, REFINE, false, LOOP>(sc, o, d, max, alpha, stack, h, vis);
 }
 
 }  // namespace dl

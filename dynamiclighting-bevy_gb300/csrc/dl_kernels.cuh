@@ -176,7 +176,7 @@ struct Vis {
 
 // A shadow-ray tracer from one origin; REFINE selects the refined form's triangle test and
 // compensated sums in the visibility functions that use it.
-template <bool COUNT = false, bool REFINE = false>
+template <bool COUNT = false, bool REFINE = false, NodeLoop LOCAL = NodeLoop::kPlain>
 struct Tracer {
     static constexpr bool kRefine = REFINE;
     const DevScene &sc;
@@ -186,6 +186,10 @@ struct Tracer {
     Visits *vis;
     __device__ __forceinline__ bool operator()(f3 dir, float dist) const {
         return occluded<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
+    }
+    // for rays towards a local light
+    __device__ __forceinline__ bool toward_light(f3 dir, float dist) const {
+        return occluded<COUNT, REFINE, LOCAL>(sc, origin, dir, dist, alpha, stack, vis);
     }
     __device__ __forceinline__ bool postponed(f3 dir, float dist) const {
         return occluded_postponed<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
@@ -239,7 +243,7 @@ __device__ __forceinline__ Vis point_vis(const DevLight &l, f3 pos, f3 nrm, cons
     if (d == 0.0f) return Vis{true, 1, 0};
     f3 dir = divs(to, d);
     if (dot(nrm, dir) <= kNdotlTolerance) return Vis{false, 0, 0};
-    return Vis{true, tr(dir, d) ? 0u : 1u, 1};
+    return Vis{true, tr.toward_light(dir, d) ? 0u : 1u, 1};
 }
 
 // texel_visibility (area.rs:61-90) with toward (area.rs:130-146)
@@ -267,7 +271,7 @@ __device__ __forceinline__ Vis area_vis(const DevScene &sc, const DevLight &l, f
         if (!(receiver > 0.0f && emitter > 0.0f)) return false;
         w = receiver * emitter / dsq;
         rays += 1;
-        unblocked = !tr(dir, fmaxf(dist - kEndGap, 0.0f));
+        unblocked = !tr.toward_light(dir, fmaxf(dist - kEndGap, 0.0f));
         return true;
     };
     f2 off;
@@ -609,7 +613,7 @@ __device__ __forceinline__ SunHit sun_hit(const DevScene &sc, const DevLight &l,
     bool alpha = (l.flags & kLightAlpha) != 0;
     f3 direction = cosine_direction_basis(normal, g.side, g.across, spread(i, g.off, true));
     Hit h;
-    if (!traverse<false, COUNT, REFINE, false, 8>(sc, origin, direction, INFINITY, alpha, stack, h, vis)) return r;
+    if (!traverse<false, COUNT, REFINE, false, NodeLoop::kFew>(sc, origin, direction, INFINITY, alpha, stack, h, vis)) return r;
     f3 face = hit_face_normal(sc, h);
     if (dot(face, direction) >= 0.0f) return r;
     float lit = dot(hit_surface_normal(sc, h, face), l.toward);
@@ -623,7 +627,8 @@ __device__ __forceinline__ SunHit sun_hit(const DevScene &sc, const DevLight &l,
 template <bool COUNT, bool REFINE>
 __device__ __forceinline__ bool sun_open(const DevScene &sc, const DevLight &l, f3 point, int *stack,
                                          Visits *vis) {
-    return !occluded<COUNT, REFINE>(sc, point, l.toward, INFINITY, (l.flags & kLightAlpha) != 0, stack, vis);
+    return !occluded<COUNT, REFINE, NodeLoop::kOneLeaf>(sc, point, l.toward, INFINITY, (l.flags & kLightAlpha) != 0,
+                                                       stack, vis);
 }
 // Sample i of gather_sun (sun_bounce.rs:53-71).
 template <bool COUNT, bool REFINE>

@@ -36,3 +36,13 @@ def test_few_and_many_leaves_match_the_oracle(faces, cells, alpha, form):
         inp, opts, mode=mode, eps=dl.DEFAULT_REFINE_EPSILON)["scene"]
     for lanes in (0, 1, 32):
         assert_same(dl.bake(inp, opts, form=form, sample_lanes=lanes), want)
+
+
+def test_kernels_without_a_sky_phase_match_the_oracle():
+    # points, panels and tubes without a sky take k_trace_batched's form without the grouped phase where one is
+    # built for the register budget (8, 9 and 10 blocks), the general one otherwise
+    inp, opts = scenes.soft_rooms(rooms=1, boxes_per_room=6, lights=6)
+    opts.pixel_density = 6.0
+    want, _, _ = oracle.bake(inp, opts)
+    for blocks in (0, 7, 8, 9, 10, 12):
+        assert_same(dl.bake(inp, opts, min_blocks=blocks), want)
