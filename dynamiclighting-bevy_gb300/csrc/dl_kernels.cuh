@@ -176,9 +176,10 @@ struct Vis {
 
 // A shadow-ray tracer from one origin; REFINE selects the refined form's triangle test and
 // compensated sums in the visibility functions that use it.
-template <bool COUNT = false, bool REFINE = false, NodeLoop LOCAL = NodeLoop::kPlain>
+template <bool COUNT = false, bool REFINE = false, bool QUEUED = false>
 struct Tracer {
     static constexpr bool kRefine = REFINE;
+    static constexpr bool kQueued = QUEUED;  // the batched queue's items behind the sky's
     const DevScene &sc;
     f3 origin;
     bool alpha;
@@ -189,7 +190,7 @@ struct Tracer {
     }
     // for rays towards a local light
     __device__ __forceinline__ bool toward_light(f3 dir, float dist) const {
-        return occluded<COUNT, REFINE, LOCAL>(sc, origin, dir, dist, alpha, stack, vis);
+        return occluded<COUNT, REFINE, QUEUED ? NodeLoop::kOneLeaf : NodeLoop::kPlain>(sc, origin, dir, dist, alpha, stack, vis);
     }
     __device__ __forceinline__ bool postponed(f3 dir, float dist) const {
         return occluded_postponed<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
@@ -341,7 +342,8 @@ __device__ __forceinline__ Vis texel_shadow(const DevScene &sc, uint32_t slot, u
     if (l.shape == DL_SHAPE_POINT) return point_vis(l, pos, nrm, tr);
     Pcg rng = stream5(sc.seed, mesh_id, l.id, x, y);
     if (l.shape == DL_SHAPE_SUN) return sun_vis(sc, l, nrm, rng, tr);
-    if (l.shape == DL_SHAPE_SKY) return sky_vis(sc, l, nrm, rng, tr);
+    if constexpr (!TR::kQueued)
+        if (l.shape == DL_SHAPE_SKY) return sky_vis(sc, l, nrm, rng, tr);
     return area_vis(sc, l, pos, nrm, rng, tr);
 }
 

@@ -38,11 +38,24 @@ def test_few_and_many_leaves_match_the_oracle(faces, cells, alpha, form):
         assert_same(dl.bake(inp, opts, form=form, sample_lanes=lanes), want)
 
 
-def test_kernels_without_a_sky_phase_match_the_oracle():
-    # points, panels and tubes without a sky take k_trace_batched's form without the grouped phase where one is
-    # built for the register budget (8, 9 and 10 blocks), the general one otherwise
+def test_local_lights_alone_match_the_oracle():
+    # points, panels and tubes: rays that return to the nodes after each leaf, for every register budget
     inp, opts = scenes.soft_rooms(rooms=1, boxes_per_room=6, lights=6)
     opts.pixel_density = 6.0
     want, _, _ = oracle.bake(inp, opts)
     for blocks in (0, 7, 8, 9, 10, 12):
         assert_same(dl.bake(inp, opts, min_blocks=blocks), want)
+
+
+def test_the_queues_two_kernels_match_the_oracle():
+    # a sky alone, a sky with sun, points and panels behind it, and those alone, for every register budget
+    inp, opts = scenes.outdoor(grid=17, chunks=2, boxes=5, point_lights=2, sky_samples=24, bounce_samples=20)
+    opts.pixel_density = 2.0
+    skies = [light for light in inp.lights if light.shape.kind == dl.SKY]
+    others = [light for light in inp.lights if light.shape.kind != dl.SKY]
+    assert skies and others
+    for lights in (skies, skies + others, others):
+        case = dl.BakeInput(inp.meshes, lights)
+        want, _, _ = oracle.bake(case, opts)
+        for blocks in (0, 7, 8, 9, 10, 12):
+            assert_same(dl.bake(case, opts, min_blocks=blocks), want)
