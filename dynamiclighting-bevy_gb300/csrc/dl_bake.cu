@@ -668,8 +668,10 @@ struct BounceArgs {
 // does (sun_bounce.rs:70). Dynamic shared memory holds only the groups' masks
 // (the per-round contributions go to the leader by shuffles), so that the rest of each SM's
 // unified L1/shared memory stays L1 cache for the BVH. MINB is the launch bound's blocks per SM
-// (the register budget: 6, 8, 9 and 10 give 80, 64, 56 and 48 registers a thread).
-template <bool COUNT, bool REFINE, int MINB>
+// (the register budget: 6, 8, 9 and 10 give 80, 64, 56 and 48 registers a thread). Without SUNS the sun's half is
+// left out (no sun in the scene gathers): 200 bytes of spills at 9 blocks instead of 292, the rooms' gather
+// 22.0 -> 21.5 ms. A form without the local half measured the same as this one.
+template <bool COUNT, bool REFINE, int MINB, bool SUNS = true>
 __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs a) {
     extern __shared__ uint32_t masks[];
     int stack[kStack];
@@ -718,7 +720,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
             origin = add(pos, scale(normal, kRayOffset));
             const DevLight &l = sc.lights[s];
             samples = l.bounce_samples;
-            sun = l.shape == DL_SHAPE_SUN;
+            sun = SUNS && l.shape == DL_SHAPE_SUN;
             if (sun) {
                 sun_setup(sc, l, sc.mesh_id[m], xy & 0xFFFFu, xy >> 16, normal, sg);
                 active = true;
@@ -728,7 +730,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
         }
         if (!active) samples = 0;
         const uint32_t net = sun && active && a.buffered ? ordered_net(samples, 32, a.buffered) : 0u;
-        const bool aligned = net != 0;
+        const bool aligned = SUNS && net != 0;
         const uint32_t shift = aligned ? net_shift(net, sg.off) : 0u, ranks = aligned ? net : samples;
         FSum3<REFINE> sum;
         uint32_t filled = 0;  // aligned sun gathers: scratch slots filled so far (the same in the group)
@@ -757,7 +759,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs
             Contribution c{f3{0.0f, 0.0f, 0.0f}, false, 0};
             if (k < samples) {
                 const DevLight &l = sc.lights[s];
-                if (sun) {
+                if (SUNS && sun) {
                     c = sun_sample<COUNT, REFINE>(sc, l, origin, normal, sg, k, stack,  &vis);
                 } else {
                     Tracer<COUNT, REFINE> tr{sc, origin, (l.flags & kLightAlpha) != 0, stack, &vis};
@@ -2369,7 +2371,8 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 //   19.7 ms). Chunks of 32 items (the level: 64 take 1 % longer).
 // - gathers with a sun take 10 blocks (the outdoor quarter 17.5 ms, at 9 17.7 ms) and 8 lanes, from 1 M
 //   items 4 (tile, 1 to 32 lanes: 11.8, 9.0, 8.1, 7.7, 7.8, 8.2 ms; the level at 2, 4, 8 lanes: 84.3, 84.8,
-//   87.2 ms), local ones alone 9 (rooms 22.0 ms, at 8 22.3 ms) and 2 lanes (8.7, 8.7, 9.2, 10.0, 11.5,
+//   87.2 ms), local ones alone 9 (rooms at 6, 8, 9, 10, 12: 24.1,
+//   21.7, 21.5, 21.4, 22.5 ms) and 2 lanes (8.7, 8.7, 9.2, 10.0, 11.5,
 //   15.9 ms), refined ones 4 lanes at 8 (terrain 63.4, 60.7, 59.3, 58.6, 58.3, 58.4 ms, decals 31.2, 29.2,
 //   29.3, 30.4, 32.4, 33.8 ms).
 // From 1 M visibility items (256 K gather items) neighbouring register budgets are tried too, each on a
@@ -2512,13 +2515,22 @@ struct GatherTune {
     double ms = 0.0;
 };
 using GatherKernel = void (*)(DevScene, BounceArgs);
-GatherKernel gather_kernel(bool refine, uint32_t minb, bool count = false) {
-    return count    ? k_gather<true, false, 6>
-           : refine ? k_gather<false, true, 8>
-           : minb == 8  ? k_gather<false, false, 8>
+// `suns`: whether the scene gathers a sun's bounce.
+GatherKernel gather_kernel(bool refine, uint32_t minb, bool suns, bool count = false) {
+    if (count) return k_gather<true, false, 6>;
+    if (refine) return k_gather<false, true, 8>;
+    if (!suns && minb == 8) return k_gather<false, false, 8, false>;
+    if (!suns && minb == 9) return k_gather<false, false, 9, false>;
+    if (!suns && minb == 10) return k_gather<false, false, 10, false>;
+    return minb == 8    ? k_gather<false, false, 8>
            : minb == 9  ? k_gather<false, false, 9>
            : minb == 10 ? k_gather<false, false, 10>
                         : k_gather<false, false, 6>;
+}
+bool gathers_suns(const dl_session &s) {
+    for (const DevLight &l : s.host.lights)
+        if (l.shape == DL_SHAPE_SUN && (l.flags & kLightBounce)) return true;
+    return false;
 }
 // Shared memory of a gather launch: for aligned sun gathers two masks of `buffered` bits per lane
 // group (at most 8 KB).
@@ -2546,22 +2558,21 @@ std::map<TuneKey, GatherTune> g_gather_cache;
 
 GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refine, dl_progress *progress) {
     const dl_bake_config &c = s.config;
+    const bool sun = gathers_suns(s);
     GatherTune best;
     best.stack_depth = stack_depth(s);
     auto blocks_for = [&](uint32_t minb, uint32_t w) {
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_kernel(refine, minb), kBlock,
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_kernel(refine, minb, sun), kBlock,
                                                          gather_smem(w, gather_buffer(s))));
         if (c.blocks_per_sm) per_sm = std::min(per_sm, (int)c.blocks_per_sm);
         return (uint32_t)std::max(1, per_sm) * (uint32_t)s.sms;
     };
-    bool sun = false;
-    for (const DevLight &l : s.host.lights) sun |= l.shape == DL_SHAPE_SUN && (l.flags & kLightBounce);
     best.lanes = c.sample_lanes ? c.sample_lanes : refine || (sun && ba.items >= (1u << 20)) ? 4u : sun ? 8u : 2u;
     std::vector<uint32_t> minbs = refine                ? std::vector<uint32_t>{8}
                                   : c.gather_min_blocks ? std::vector<uint32_t>{c.gather_min_blocks}
                                   : sun                 ? std::vector<uint32_t>{10, 9}
-                                                        : std::vector<uint32_t>{9, 8};
+                                                        : std::vector<uint32_t>{9, 10};
     const uint32_t every = ba.items >= (1u << 20) ? 32 : ba.items >= (1u << 18) ? 16 : 0;
     // the refined gather always takes 8 (64 registers: 173 ms on the outdoor scene against 178 ms at
     // 80 registers and 173 ms at 48, its binary64 re-tests spill)
@@ -2597,7 +2608,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
         ba.scratch = gather_scratch(s, blocks, best.lanes, ba.buffered);
         CK(cudaMemsetAsync(ba.head, 0, sizeof(unsigned long long), st));
         CK(cudaEventRecord(a, st));
-        gather_kernel(refine, minb)<<<blocks, kBlock, gather_smem(best.lanes, ba.buffered), st>>>(
+        gather_kernel(refine, minb, sun)<<<blocks, kBlock, gather_smem(best.lanes, ba.buffered), st>>>(
             s.sc, ba);
         CK(cudaGetLastError());
         CK(cudaEventRecord(b, st));
@@ -3058,7 +3069,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
             CK(cudaMemsetAsync(ba.head, 0, sizeof(unsigned long long), st));
             // the instrumented variant (counting node visits and triangle tests) when asked
             CK(cudaEventRecord(g0, st));
-            gather_kernel(refine_bounce, g.minb, s.config.count_visits != 0 && !refine_bounce)<<<
+            gather_kernel(refine_bounce, g.minb, gathers_suns(s), s.config.count_visits != 0 && !refine_bounce)<<<
                 g.blocks, kBlock, gather_smem(g.lanes, g.buffered), st>>>(sc, ba);
             LAUNCHED("k_gather");
             CK(cudaEventRecord(g1, st));

@@ -34,8 +34,8 @@ def test_few_and_many_leaves_match_the_oracle(faces, cells, alpha, form):
     mode = oracle.REFINED_BOUNCE if form == "bounce_refined" else None
     want = oracle.bake(inp, opts)[0] if mode is None else oracle.bake_ex(
         inp, opts, mode=mode, eps=dl.DEFAULT_REFINE_EPSILON)["scene"]
-    for lanes in (0, 1, 32):
-        assert_same(dl.bake(inp, opts, form=form, sample_lanes=lanes), want)
+    for lanes, blocks in ((0, 0), (1, 6), (32, 8), (2, 9), (4, 10)):
+        assert_same(dl.bake(inp, opts, form=form, sample_lanes=lanes, gather_min_blocks=blocks), want)
 
 
 def test_local_lights_alone_match_the_oracle():
@@ -59,3 +59,5 @@ def test_the_queues_two_kernels_match_the_oracle():
         want, _, _ = oracle.bake(case, opts)
         for blocks in (0, 7, 8, 9, 10, 12):
             assert_same(dl.bake(case, opts, min_blocks=blocks), want)
+        for blocks in (6, 8, 9, 10):
+            assert_same(dl.bake(case, opts, gather_min_blocks=blocks), want)
