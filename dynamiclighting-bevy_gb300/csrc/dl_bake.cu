@@ -6,7 +6,7 @@
 //   texels     per triangle: owned grid, centered + touched texels (texels.rs, mesh_texels.rs)
 //   burial     per texel: <= 8 closest-hit rays (mesh_texels.rs:57-88,111-135)
 //   visibility per (pair, texel): point/area/sun/sky shadow rays (mesh_bake.rs:203-267)
-//              batched: one persistent kernel over a device work queue, from a CUDA graph;
+//              batched: persistent kernels over a device work queue;
 //              plain: one launch per mesh, a warp per triangle, lanes over texels
 //   optimize   per triangle: drop lights with no lit texel nearby (shadows.rs:54-73)
 //   seams      per region: pad unvisited texels (seams.rs:15-39)
@@ -573,22 +573,34 @@ __global__ void __launch_bounds__(kBlock) k_trace_plain(DevScene sc, TraceArgs a
     if (lane == 0 && r) atomicAdd(&a.ctr->rays, r);
 }
 
-// Queue construction: pairs in class order (sky, soft, hard) and their item prefix sums.
-__global__ void k_pair_class(DevScene sc, const uint32_t *pair_light, uint32_t pairs, uint32_t cls, uint32_t *flag) {
+// Queue construction: pairs in class order (sky, soft, hard) and their item prefix sums. One scan of
+// packed counts (sky pairs in the low word, soft ones in the high word) places all three classes.
+__global__ void k_pair_class(DevScene sc, const uint32_t *pair_light, uint32_t pairs, unsigned long long *flag) {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p > pairs) return;
-    if (p == pairs) {
-        flag[p] = 0;
-        return;
+    unsigned long long f = 0;
+    if (p < pairs) {
+        const DevLight &l = sc.lights[pair_light[p]];
+        f = l.shape == DL_SHAPE_SKY ? 1ull : l.shadow_bits > 1 ? 1ull << 32 : 0ull;
     }
-    const DevLight &l = sc.lights[pair_light[p]];
-    uint32_t c = l.shape == DL_SHAPE_SKY ? 0 : (l.shadow_bits > 1 ? 1 : 2);
-    flag[p] = c == cls;
+    flag[p] = f;
 }
-__global__ void k_pair_scatter(const uint32_t *flag, const uint32_t *pos, uint32_t pairs, uint32_t base,
-                               uint32_t *order) {
+__global__ void k_pair_scatter(const unsigned long long *flag, const unsigned long long *pos, uint32_t pairs,
+                               uint32_t *order, uint32_t *sky_pairs) {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < pairs && flag[p]) order[base + pos[p]] = p;
+    const unsigned long long total = pos[pairs];
+    const uint32_t skies = (uint32_t)total, softs = (uint32_t)(total >> 32);
+    if (p == 0) *sky_pairs = skies;
+    if (p >= pairs) return;
+    const unsigned long long f = flag[p], at = pos[p];
+    const uint32_t sky = (uint32_t)at, soft = (uint32_t)(at >> 32);
+    order[f == 1 ? sky : f ? skies + soft : skies + softs + (p - sky - soft)] = p;
+}
+// The queue's items and, of them, the sky's (sizes[1], sizes[2]) from the sky pairs' count in sizes[0].
+__global__ void k_queue_sizes(const uint32_t *item_off, uint32_t pairs, uint32_t *sizes) {
+    const uint32_t items = item_off[pairs], sky_items = item_off[sizes[0]];
+    sizes[2] = items;
+    sizes[3] = sky_items;
 }
 __global__ void k_item_counts(const uint32_t *order, const uint32_t *pair_tri, const uint32_t *ctex_off,
                               uint32_t pairs, uint32_t *cnt) {
@@ -625,6 +637,10 @@ __global__ void __launch_bounds__(kBlock) k_photons(DevScene sc, const uint32_t 
 }
 
 // Pairs whose light bakes bounce, in pair order.
+__global__ void k_pair_compact(const uint32_t *flag, const uint32_t *pos, uint32_t pairs, uint32_t *out) {
+    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < pairs && flag[p]) out[pos[p]] = p;
+}
 __global__ void k_bounce_flag(DevScene sc, const uint32_t *pair_light, uint32_t pairs, uint32_t *flag) {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p > pairs) return;
@@ -1806,7 +1822,6 @@ struct Pool {
     cudaStream_t stream = nullptr;
     DeviceBudget *budget = nullptr;
     uint64_t bytes = 0;
-    uint64_t generation = 0;  // bumped whenever a buffer moves
     template <class T>
     T *get(const std::string &name, size_t count) {
         size_t b = std::max<size_t>(count * sizeof(T), 16);
@@ -1821,7 +1836,6 @@ struct Pool {
         void *p = dev_malloc(b, stream, budget);
         bufs[name] = {p, b};
         bytes += b;
-        ++generation;
         return static_cast<T *>(p);
     }
     // Frees every buffer on the stream; the session calls it before destroying its stream.
@@ -1878,22 +1892,21 @@ struct dl_session {
     ProbeGridSetup probe_grid;
     const float *probe_open = nullptr;
     const uint32_t *probe_back = nullptr;
-    // batched-form graph over the visibility stage, rebuilt when the queue changes
     cudaEvent_t marks[9] = {};  // stage boundaries of the last run
-    cudaGraphExec_t graph = nullptr;
-    uint64_t graph_generation = ~0ull;
-    unsigned long long graph_items = 0;
-    unsigned graph_blocks = 0;
-    uint64_t graph_shape = 0;
+    // the visibility stage's second kernel runs beside the first (made by the first run that has both)
+    cudaStream_t branch = nullptr;
+    cudaEvent_t forks[2] = {};
     // the payload of the last payload_build (device, in the pool) and the readers' streams
     const uint32_t *payload_dev = nullptr;
     uint64_t payload_words = 0;
     std::vector<cudaStream_t> readers;
     ~dl_session() {
         for (cudaStream_t r : readers) cudaStreamDestroy(r);
-        if (graph) cudaGraphExecDestroy(graph);
         for (auto &e : marks)
             if (e) cudaEventDestroy(e);
+        for (auto &e : forks)
+            if (e) cudaEventDestroy(e);
+        if (branch) cudaStreamDestroy(branch);
         if (stream) {
             // back to the stream-ordered pool (kept for the next session), in stream order
             pool.release();
@@ -2910,29 +2923,26 @@ dl_status run(dl_session &s, dl_progress *progress) {
     } else {
         // queue: pairs ordered sky, soft, hard; item prefix sums over their texel counts
         uint32_t *order = P.get<uint32_t>("order", pairs + 1);
-        uint32_t *flag = P.get<uint32_t>("flag", pairs + 1);
-        uint32_t *fpos = P.get<uint32_t>("fpos", pairs + 1);
-        uint32_t base = 0, sky_pairs = 0;
-        for (uint32_t c = 0; c < 3; ++c) {
-            k_pair_class<<<grid_for(pairs + 1), kBlock, 0, st>>>(sc, pair_light, pairs, c, flag);
-            LAUNCHED("k_pair_class");
-            scan_u32(s, flag, fpos, pairs + 1);
-            k_pair_scatter<<<grid_for(pairs), kBlock, 0, st>>>(flag, fpos, pairs, base, order);
-            LAUNCHED("k_pair_scatter");
-            s.launches += 2;
-            base += read_back(s, fpos + pairs);
-            if (c == 0) sky_pairs = base;
-        }
-        uint32_t *icnt = P.get<uint32_t>("icnt", pairs + 1);
-        uint32_t *item_off = P.get<uint32_t>("item_off", pairs + 1);
+        // packed class flags and their scan, then (in the same room) item counts and their prefix sums
+        unsigned long long *flag = P.get<unsigned long long>("queue", 2 * ((size_t)pairs + 1));
+        unsigned long long *fpos = flag + pairs + 1;
+        uint32_t *icnt = reinterpret_cast<uint32_t *>(flag), *item_off = reinterpret_cast<uint32_t *>(fpos);
+        unsigned long long *heads = P.get<unsigned long long>("heads", 2);
+        uint32_t *sizes = reinterpret_cast<uint32_t *>(heads);  // until the queue is drained
+        k_pair_class<<<grid_for(pairs + 1), kBlock, 0, st>>>(sc, pair_light, pairs, flag);
+        LAUNCHED("k_pair_class");
+        scan_u64(s, flag, fpos, pairs + 1);
+        k_pair_scatter<<<grid_for(pairs), kBlock, 0, st>>>(flag, fpos, pairs, order, sizes);
+        LAUNCHED("k_pair_scatter");
         k_item_counts<<<grid_for(pairs + 1), kBlock, 0, st>>>(order, pair_tri, ctex_off, pairs, icnt);
         LAUNCHED("k_item_counts");
-        ++s.launches;
         scan_u32(s, icnt, item_off, pairs + 1);
-        const uint32_t items = read_back(s, item_off + pairs);
-        const uint32_t sky_items = sky_pairs ? read_back(s, item_off + sky_pairs) : 0;
+        k_queue_sizes<<<1, 1, 0, st>>>(item_off, pairs, sizes);
+        LAUNCHED("k_queue_sizes");
+        s.launches += 4;
+        const unsigned long long queued = read_back(s, heads + 1);
+        const uint32_t items = (uint32_t)queued, sky_items = (uint32_t)(queued >> 32);
         s.report.work_items = items;
-        unsigned long long *heads = P.get<unsigned long long>("heads", 2);
         ta.order = order;
         ta.item_off = item_off;
         ta.pairs = pairs;
@@ -2952,47 +2962,28 @@ dl_status run(dl_session &s, dl_progress *progress) {
         s.report.ms_tune = tune.ms;
         ta.grab = tune.grab;
         ta.sky_lanes = tune.sky_lanes;
-        const unsigned blocks = tune.sky_blocks << 16 | tune.rest_blocks;
-        // The visibility stage runs from a CUDA graph: the memset of the queue heads and the
-        // persistent kernel, captured once per queue layout and launch shape and replayed.
-        const uint64_t shape = ((uint64_t)tune.grab << 40) ^ ((uint64_t)tune.sky_lanes << 32) ^
-                               ((uint64_t)tune.minb << 24) ^ ((uint64_t)tune.stack_depth << 16) ^ (count ? 1 : 0) ^
-                               (refine ? 2 : 0);
-        if (!s.graph || s.graph_generation != P.generation || s.graph_items != items || s.graph_blocks != blocks ||
-            s.graph_shape != shape) {
-            if (s.graph) cudaGraphExecDestroy(s.graph);
-            s.graph = nullptr;
-            cudaGraph_t g;
-            CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            cudaMemsetAsync(heads, 0, 2 * sizeof(unsigned long long), st);
-            // the two kernels claim from heads of their own, so they are branches of the graph: blocks of
-            // one take the SMs that the other's last blocks leave (the outdoor quarter 24.1 -> 23.4 ms)
-            const bool fork = tune.sky && tune.rest;
-            cudaEvent_t before = nullptr, after = nullptr;
-            if (fork) {
-                cudaEventCreateWithFlags(&before, cudaEventDisableTiming);
-                cudaEventCreateWithFlags(&after, cudaEventDisableTiming);
-                cudaEventRecord(before, st);
-                cudaStreamWaitEvent(s.side, before, 0);
-            }
-            if (tune.sky) tune.sky<<<tune.sky_blocks, kBlock, 0, st>>>(sc, ta);
-            if (tune.rest) tune.rest<<<tune.rest_blocks, kBlock, 0, fork ? s.side : st>>>(sc, ta);
-            if (fork) {
-                cudaEventRecord(after, s.side);
-                cudaStreamWaitEvent(st, after, 0);
-                cudaEventDestroy(before);
-                cudaEventDestroy(after);
-            }
-            CK(cudaStreamEndCapture(st, &g));
-            CK(cudaGraphInstantiate(&s.graph, g, 0));
-            cudaGraphDestroy(g);
-            s.graph_generation = P.generation;
-            s.graph_items = items;
-            s.graph_blocks = blocks;
-            s.graph_shape = shape;
-        }
         CK(cudaEventRecord(v0, st));
-        CK(cudaGraphLaunch(s.graph, st));
+        CK(cudaMemsetAsync(heads, 0, 2 * sizeof(unsigned long long), st));
+        // The two kernels claim from heads of their own, so they run side by side: blocks of one take the
+        // SMs that the other's last blocks leave (the outdoor quarter 24.1 -> 23.4 ms, foliage 2.58 -> 1.95 ms).
+        // Launched directly: a graph of these nodes saves nothing and cost a one-off bake its instantiation.
+        const bool fork = tune.sky && tune.rest;
+        if (fork) {
+            if (!s.branch) {
+                CK(cudaStreamCreateWithFlags(&s.branch, cudaStreamNonBlocking));
+                for (auto &e : s.forks) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            }
+            CK(cudaEventRecord(s.forks[0], st));
+            CK(cudaStreamWaitEvent(s.branch, s.forks[0], 0));
+        }
+        if (tune.sky) tune.sky<<<tune.sky_blocks, kBlock, 0, st>>>(sc, ta);
+        if (tune.rest) tune.rest<<<tune.rest_blocks, kBlock, 0, fork ? s.branch : st>>>(sc, ta);
+        const cudaError_t launched = cudaGetLastError();
+        if (fork) {
+            CK(cudaEventRecord(s.forks[1], s.branch));
+            CK(cudaStreamWaitEvent(st, s.forks[1], 0));
+        }
+        CK(launched);
         s.launches += (tune.sky != nullptr) + (tune.rest != nullptr);
         CK(cudaEventRecord(v1, st));
     }
@@ -3027,8 +3018,8 @@ dl_status run(dl_session &s, dl_progress *progress) {
         scan_u32(s, bflag, bpos, pairs + 1);
         const uint32_t bcount = read_back(s, bpos + pairs);
         uint32_t *bpairs = P.get<uint32_t>("bpairs", bcount + 1);
-        k_pair_scatter<<<grid_for(pairs), kBlock, 0, st>>>(bflag, bpos, pairs, 0, bpairs);
-        LAUNCHED("k_pair_scatter");
+        k_pair_compact<<<grid_for(pairs), kBlock, 0, st>>>(bflag, bpos, pairs, bpairs);
+        LAUNCHED("k_pair_compact");
         uint32_t *bcnt = P.get<uint32_t>("bcnt", bcount + 1);
         uint32_t *bitem_off = P.get<uint32_t>("bitem_off", bcount + 1);
         k_item_counts<<<grid_for(bcount + 1), kBlock, 0, st>>>(bpairs, pair_tri, ctex_off, bcount, bcnt);

@@ -151,8 +151,8 @@ typedef struct dl_progress {
    with compensated (Kahan) sums. Its bytes may differ from the other forms where those change a
    level. */
 enum {
-    DL_FORM_BATCHED = 0, /* every (triangle, light) pair through one persistent kernel fed by a
-                            device work queue, launched from a CUDA graph */
+    DL_FORM_BATCHED = 0, /* every (triangle, light) pair through persistent kernels fed by a
+                            device work queue */
     DL_FORM_PLAIN = 1,   /* one launch per mesh, a warp per triangle looping over its lights and
                             texels: the reference's loop order on the GPU */
     DL_FORM_REFINED = 2, /* the batched form with binary64 edge re-tests and compensated sums */
