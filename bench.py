@@ -327,8 +327,8 @@ def main():
             "bound": "l2", "kernel": "k_gather", "achieved": g_achieved, "peak": l2_gbs.value, "unit": "GB/s",
             "frac": g_achieved / l2_gbs.value if l2_gbs.value else None,
             "peak_source": "the same L2 read bandwidth measurement",
-            "limiter": "instruction issue (ncu on the quarter-size outdoor case: issue slots 71 % busy, "
-                       "SIMT efficiency 40 %, L2 throughput 8.4 % of peak)",
+            "limiter": "instruction issue and L1 return (ncu on the quarter-size outdoor case: issue slots 70 % "
+                       "busy, L1 data pipe 72 %, SIMT efficiency 44 %, L2 throughput 9 % of peak)",
             "algorithmic_bytes_per_launch": int(g_bytes), "ms": gms, "traffic": g_traffic,
             "bytes_per_unit": "64 per node visit + 48 per triangle test + 52 per (bounce pair, texel) item",
             "node_visits": int(crep.gather_node_visits), "tri_tests": int(crep.gather_tri_tests),
@@ -420,8 +420,8 @@ def main():
                                     "buffer streamed 100 times with L1-bypassing loads (dl_probe_read_bandwidth)",
                      "l1_read_gbs": l1_gbs.value, "hbm_gbs": hbm, "hbm_source": f"{peak_kind} (MEASURED_PEAKS.json)",
                      "traffic": traffic, "traffic_frac_of_algorithmic": traffic / alg_bytes if traffic else None,
-                     "limiter": "instruction issue (ncu on the quarter-size outdoor case: issue slots 74 % busy, "
-                                "SIMT efficiency 54 %, L2 throughput 3.9 % of peak)",
+                     "limiter": "instruction issue and L1 return (ncu on the quarter-size outdoor case: issue slots "
+                                "76 % busy, L1 data pipe 72 %, SIMT efficiency 47 %, L2 throughput 6 % of peak)",
                      "algorithmic_bytes_per_launch": int(alg_bytes),
                      "bytes_per_unit": "64 per node visit + 48 per triangle test + 76 per (pair, texel) item",
                      "node_visits": int(crep.node_visits), "tri_tests": int(crep.tri_tests),

@@ -227,7 +227,9 @@ DL_HD void sincos_d(double x, double &s, double &c) {
 // double-float binary32 arithmetic (error-free sums and FMA products; Dekker 1971, Knuth TAOCP
 // 4.2.2) to within 2^-40 of the true value, and the result is kept only when the rounding test
 // of Ziv's strategy (Ziv 1991) proves it is the correctly rounded binary32 value; otherwise the
-// binary64 path below decides. Either way the value equals what the binary64 path returns.
+// binary64 path below decides. Either way the value equals what the binary64 path returns. The baker's
+// sines and cosines take the table path further down; the series over the whole octant, its rounding test
+// and its pi/2 are what tests/native/sincos_check.cpp holds against binary64.
 struct FF {
     float h, l;
 };

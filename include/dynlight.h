@@ -146,10 +146,10 @@ typedef struct dl_progress {
 /* How the bake runs. BATCHED and PLAIN give identical bytes, bit-exact with the reference's
    binary32 arithmetic. REFINED is the batched form with three precision changes: ray/triangle
    tests whose binary32 barycentrics, determinant or hit distance fall within `refine_epsilon` of
-   a boundary are re-tested in binary64; closest hits are chosen by the candidates' binary64
-   distances (with their barycentrics); soft-visibility weights and bounce gathers are summed
-   with compensated (Kahan) sums. Its bytes may differ from the other forms where those change a
-   level. */
+   a boundary are re-tested in binary64; closest hits are the ones that the candidates' binary64
+   distances would choose (with the winner's binary64 distance and barycentrics); soft-visibility
+   weights and bounce gathers are summed with compensated (Kahan) sums. Its bytes may differ from
+   the other forms where those change a level. */
 enum {
     DL_FORM_BATCHED = 0, /* every (triangle, light) pair through persistent kernels fed by a
                             device work queue */
@@ -167,17 +167,17 @@ typedef struct dl_bake_config {
     uint32_t form;             /* DL_FORM_* */
     uint32_t device;           /* CUDA device ordinal */
     uint32_t block_threads;    /* 0: tuned default */
-    uint32_t chunk_texels;     /* (pair, texel) items a warp claims from the queue at once, 0: tuned */
+    uint32_t chunk_texels;     /* (pair, texel) items a warp claims from the queue at once, 0: by rule */
     uint32_t sample_lanes;     /* lanes sharing one texel's sky samples and bounce-gather samples
-                                  (1, 2, 4, 8, 16 or 32), 0: tuned */
+                                  (1, 2, 4, 8, 16 or 32), 0: by rule */
     uint32_t blocks_per_sm;    /* upper bound of persistent blocks per SM, 0: as many as fit */
     uint32_t count_visits;     /* 1: run the instrumented visibility kernel that counts BVH node
                                   visits and triangle tests (for roofline accounting; slower) */
     float refine_epsilon;      /* DL_FORM_REFINED: re-test margin (barycentric units; times
                                   max(1, ray length) for distances), 0: 1e-4 */
     uint32_t no_autotune;      /* 1: never time candidate launch shapes; unset knobs take defaults.
-                                  0: knobs left 0 are picked by timing trials on the first run of a
-                                  scene shape (cached per process) */
+                                  0: large queues also time neighbouring register budgets on the first
+                                  run of a scene shape (cached per process) */
     uint32_t host_bvh;         /* 1: build the occluder BVH on the host's cores and upload it;
                                   0: build it on the device (the same tree, in milliseconds) */
     uint32_t max_device_mib;   /* cap on the device memory one bake (session) may hold, in MiB:
@@ -186,10 +186,11 @@ typedef struct dl_bake_config {
                                   frees what the bake held. 0: no cap */
     uint32_t min_blocks;       /* register budget of the bit-exact visibility kernel, as the
                                   blocks of 128 threads per SM it is compiled to fit: 7, 8, 9, 10
-                                  or 12 (72, 64, 56, 48 or 40 registers per thread), 0: tuned.
-                                  The refined and counting kernels have one budget (7) */
+                                  or 12 (72, 64, 56, 48 or 40 registers per thread), 0: by rule (and
+                                  trials). The refined and counting kernels have one budget each */
     uint32_t gather_min_blocks; /* the same for the bit-exact bounce gather: 6, 8, 9 or 10 (80,
-                                  64, 56 or 48 registers), 0: tuned; the refined gather has one (8) */
+                                  64, 56 or 48 registers), 0: by rule (and trials); the refined gather has
+                                  one (8) */
     uint32_t reserved[1];
 } dl_bake_config;
 
@@ -220,8 +221,10 @@ typedef struct dl_bake_report {
     double ms_host[4];        /* host time of session creation: validation + sorting + lights,
                                  occluder BVH build, flattening + uploads, unused */
     uint64_t retests;         /* DL_FORM_REFINED: ray/triangle tests re-run in binary64 (tests
-                                 near a boundary, and every closest-hit candidate) */
-    /* launch shape of the batched visibility kernel (picked by the autotuner or the config) */
+                                 near a boundary, closest-hit candidates whose order binary32
+                                 leaves open, and each closest hit) */
+    /* launch shape of the batched visibility (rule, trials or config): the sky's kernel where the
+       scene has one */
     uint32_t tuned_chunk_texels, tuned_sample_lanes, tuned_blocks_per_sm, tuned_stack_depth;
     uint32_t tuned_min_blocks;  /* launch bound: blocks per SM the registers were sized for */
     uint32_t tune_trials;       /* candidate shapes timed in this run (0: defaults or cached) */
