@@ -447,7 +447,7 @@ __device__ __forceinline__ unsigned long long claim(const TraceArgs &a, unsigned
 // of its samples in the shift-aligned coherent order, and the open counts are summed across the
 // group (an integer sum, so the level is the same as one lane tracing them all in index order).
 // MINB is the launch bound's blocks per SM (the register budget). Apart from the other lights' code the sky's
-// loop needs 40 registers at 12 blocks with a quarter of the spills (the outdoor quarter's visibility 23.5 ms in one
+// loop needs 40 registers at 12 blocks with a quarter of the spills (a 77 k triangle terrain's visibility 23.5 ms in one
 // kernel at 10, 23.1 ms in two).
 template <bool COUNT, bool REFINE, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_trace_sky(DevScene sc, TraceArgs a) {
@@ -2373,21 +2373,20 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 // samples, the launch bound's blocks per SM (the register budget: 7, 8, 9, 10 or 12 blocks of 128
 // threads give 72, 64, 56, 48 or 40 registers per thread; the gather's 6 gives 80). A rule picks the shape:
 // - sky lanes grow with the sample count, 8 from 256 samples, 4 from 128, 2 from 64, but at most 4 from
-//   4 M items. Lanes that share a texel's aligned samples trace neighbouring directions, and few texels
+//   1 M items. Lanes that share a texel's aligned samples trace neighbouring directions, and few texels
 //   with long sample loops leave the last warps alone. Visibility of a terrain tile (0.5 M items, 256
-//   samples) at 1, 2, 4, 8, 16 lanes: 13.3, 10.7, 9.6, 9.4, 9.6 ms; of the outdoor level (9.4 M) at 2,
-//   4, 8: 126.4, 123.7, 127.7 ms; of foliage (128 samples) 5.6, 3.1, 2.4, 2.3, 2.5 ms; of a room (64
-//   samples) 0.39, 0.40, 0.43, 0.44, 0.46 ms.
-// - 12 blocks per SM for the sky (the outdoor quarter at 9, 10, 12, 14: 23.5, 23.4, 23.1, 26.9 ms; sky rays
+//   samples) at 1, 2, 4, 8, 16 lanes: 11.8, 9.7, 8.6, 8.4, 8.6 ms; of the outdoor quarter (2.6 M) 42.1, 38.1,
+//   37.0, 38.4, 40.0 ms; of terrain with 200 samples (1.6 M) 25.2, 22.4, 21.3, 21.9, 22.6 ms; of foliage (128
+//   samples) 4.5, 2.8, 1.9, 2.0, 2.1 ms; of a room (64 samples) 0.38, 0.35, 0.35, 0.36, 0.36 ms.
+// - 12 blocks per SM for the sky (a 77 k triangle terrain at 9, 10, 12, 14: 23.5, 23.4, 23.1, 26.9 ms; sky rays
 //   wait on the tree's far nodes, more warps hide it), 8 for the rest (rooms under panels and tubes at 8, 9,
 //   10: 5.5, 5.6, 5.7 ms), 8 and 7 in the refined form (decals at 7, 8, 9, 10 for the sky: 18.4, 18.1, 19.0,
 //   19.7 ms). Chunks of 32 items (the level: 64 take 1 % longer).
-// - gathers with a sun take 10 blocks (the outdoor quarter 17.5 ms, at 9 17.7 ms) and 8 lanes, from 1 M
-//   items 4 (tile, 1 to 32 lanes: 11.8, 9.0, 8.1, 7.7, 7.8, 8.2 ms; the level at 2, 4, 8 lanes: 84.3, 84.8,
-//   87.2 ms), local ones alone 9 (rooms at 6, 8, 9, 10, 12: 24.1,
-//   21.7, 21.5, 21.4, 22.5 ms) and 2 lanes (8.7, 8.7, 9.2, 10.0, 11.5,
-//   15.9 ms), refined ones 4 lanes at 8 (terrain 63.4, 60.7, 59.3, 58.6, 58.3, 58.4 ms, decals 31.2, 29.2,
-//   29.3, 30.4, 32.4, 33.8 ms).
+// - gathers with a sun take 10 blocks (a terrain of 77 k triangles 17.5 ms, at 9 17.7 ms) and 8 lanes, from 1 M
+//   items 4 (tile, 1 to 16 lanes: 10.2, 8.0, 7.2, 6.8, 7.0 ms; the quarter 30.3, 27.0, 26.8, 27.1, 29.5 ms),
+//   local ones alone 9 (rooms at 6, 8, 9, 10, 12: 24.1, 21.7, 21.5, 21.4, 22.5 ms) and 2 lanes (6.3, 6.2, 6.3,
+//   6.6, 7.5 ms), refined ones 8 and 4 lanes (terrain 26.1, 23.1, 22.6, 23.3, 25.7 ms, decals 16.1, 14.6,
+//   14.4, 15.4, 16.9 ms).
 // From 1 M visibility items (256 K gather items) neighbouring register budgets are tried too, each on a
 // small share of the real queue's chunks with scratch counters; their results are the same levels and
 // values that the real pass writes (OR and max, and values that it overwrites), so the trials change no
@@ -2459,10 +2458,11 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
         best.rest_blocks = best.rest ? blocks_of(best.rest) : 0;
     };
     const uint32_t n = s.options.sky_samples;
-    const uint32_t sky_lanes = n >= 256 && ta.items < (4u << 20) ? 8 : n >= 128 ? 4 : n >= 64 ? 2 : 1;
+    const uint32_t sky_lanes = n >= 256 && ta.items < (1u << 20) ? 8 : n >= 128 ? 4 : n >= 64 ? 2 : 1;
     best.grab = c.chunk_texels ? std::max(1u, c.chunk_texels / 32) : 1u;
     best.sky_lanes = c.sample_lanes ? c.sample_lanes : ta.sky_items ? sky_lanes : 1u;
-    std::vector<uint32_t> minbs = (count || refine) ? std::vector<uint32_t>{7}
+    std::vector<uint32_t> minbs = count             ? std::vector<uint32_t>{7}
+                                  : refine          ? std::vector<uint32_t>{ta.sky_items ? 8u : 7u}
                                   : c.min_blocks    ? std::vector<uint32_t>{c.min_blocks}
                                   : ta.sky_items    ? std::vector<uint32_t>{12, 10}
                                                     : std::vector<uint32_t>{8, 9, 10};
@@ -2965,7 +2965,7 @@ dl_status run(dl_session &s, dl_progress *progress) {
         CK(cudaEventRecord(v0, st));
         CK(cudaMemsetAsync(heads, 0, 2 * sizeof(unsigned long long), st));
         // The two kernels claim from heads of their own, so they run side by side: blocks of one take the
-        // SMs that the other's last blocks leave (the outdoor quarter 24.1 -> 23.4 ms, foliage 2.58 -> 1.95 ms).
+        // SMs that the other's last blocks leave (a 77 k triangle terrain 24.1 -> 23.4 ms, foliage 2.58 -> 1.95 ms).
         // Launched directly: a graph of these nodes saves nothing and cost a one-off bake its instantiation.
         const bool fork = tune.sky && tune.rest;
         if (fork) {

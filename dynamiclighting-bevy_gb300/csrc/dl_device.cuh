@@ -217,7 +217,7 @@ __device__ __forceinline__ bool tri_test_refined(const DevScene &sc, float4 v0, 
 // Entries of a traversal stack (>= BVH depth; the host refuses deeper trees). A thread's stack is local
 // memory: a ray holds a few entries of the 8 to 28 that its tree could need, and only the lines in use take
 // room in L1, where shared stacks took their worst case from it for every resident thread (14 KB a block
-// of the outdoor level, 140 KB of the SM's 256). Shared -> local: the outdoor quarter's visibility 24.6 ->
+// of the outdoor level, 140 KB of the SM's 256). Shared -> local: a 77 k triangle terrain's visibility 24.6 ->
 // 23.5 ms at 10 blocks, the rooms' local gather 24.9 -> 23.7 ms at 8, rooms under panels and tubes 6.4 -> 6.2 ms.
 constexpr int kStack = 64;
 
@@ -280,7 +280,7 @@ __device__ __forceinline__ bool refined_candidate(const DevScene &sc, f3 o, f3 d
 
 // How a warp's lanes leave the traversal's two loops. Most of its idle lanes wait at their border (14 of 32
 // threads active). kFew: the last lanes still among inner nodes, when fewer than 8, wait for the others'
-// leaves, which shorten those rays' ranges and bring their lanes back: the outdoor quarter's sun gather 19.6 ms
+// leaves, which shorten those rays' ranges and bring their lanes back: a 77 k triangle terrain's sun gather 19.6 ms
 // plain, 18.5, 18.2, 18.3 ms at 4, 8, 12; other closest hits gain nothing (burial in rooms 0.38 -> 0.42 ms,
 // photons 3.32 -> 3.39 ms), any-hit rays lose 6 %. kOneLeaf: back to inner nodes after one leaf: the sun gather's shadow
 // rays (its 18.2 -> 17.7 ms) and rays towards local lights; the sky's and the sun's lose 2 to 10 %.
@@ -390,8 +390,8 @@ __device__ __noinline__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, flo
 // Any-hit traversal that holds a ray's first leaf back and goes on among inner nodes until every lane
 // there holds one (speculative traversal, Aila & Laine 2009): more lanes take part in each triangle
 // test, for nodes that a blocked ray did not need. It pays for the local gather's rays, whose
-// directions differ from lane to lane (the room grid's gather 23.3 ms without, 22.0 ms), not for aligned ones (the
-// outdoor quarter's visibility 23.5 -> 24.0 ms) nor for those towards a light (rooms under panels and tubes 6.25 ->
+// directions differ from lane to lane (the room grid's gather 23.3 ms without, 22.0 ms), not for aligned ones (a 77 k triangle
+// terrain's visibility 23.5 -> 24.0 ms) nor for those towards a light (rooms under panels and tubes 6.25 ->
 // 6.4 ms).
 template <bool COUNT, bool REFINE>
 __device__ __forceinline__ bool occluded_postponed(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack,
