@@ -536,10 +536,10 @@ def load_library(path: str = LIBRARY_PATH):
     return lib
 
 
-_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.restype, _new_bytes.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
-_bytes_at = C.pythonapi.PyBytes_AsString
-_bytes_at.restype, _bytes_at.argtypes = C.c_void_p, [C.py_object]
+# The interpreter's functions through prototypes of this module's own: those of ctypes.pythonapi are one
+# object each for the whole process, which any module may give other types.
+_new_bytes = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+_bytes_at = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
 
 
 def _raise(lib, status):
