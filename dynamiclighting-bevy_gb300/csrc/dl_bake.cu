@@ -685,8 +685,8 @@ struct BounceArgs {
 // (the per-round contributions go to the leader by shuffles), so that the rest of each SM's
 // unified L1/shared memory stays L1 cache for the BVH. MINB is the launch bound's blocks per SM
 // (the register budget: 6, 8, 9 and 10 give 80, 64, 56 and 48 registers a thread). Without SUNS the sun's half is
-// left out (no sun in the scene gathers): 200 bytes of spills at 9 blocks instead of 292, the rooms' gather
-// 22.0 -> 21.5 ms. A form without the local half measured the same as this one.
+// left out (no sun in the scene gathers): 136 bytes of spill stores at 9 blocks instead of 296, nine rooms' gather
+// 22.0 -> 21.5 ms (with an earlier traversal loop; 12.5 ms now). A form without the local half measured the same as this one.
 template <bool COUNT, bool REFINE, int MINB, bool SUNS = true>
 __global__ void __launch_bounds__(kBlock, MINB) k_gather(DevScene sc, BounceArgs a) {
     extern __shared__ uint32_t masks[];
@@ -2384,8 +2384,8 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 //   19.7 ms). Chunks of 32 items (the level: 64 take 1 % longer).
 // - gathers with a sun take 10 blocks (a terrain of 77 k triangles 17.5 ms, at 9 17.7 ms) and 8 lanes, from 1 M
 //   items 4 (tile, 1 to 16 lanes: 10.2, 8.0, 7.2, 6.8, 7.0 ms; the quarter 30.3, 27.0, 26.8, 27.1, 29.5 ms),
-//   local ones alone 9 (rooms at 6, 8, 9, 10, 12: 24.1, 21.7, 21.5, 21.4, 22.5 ms) and 2 lanes (6.3, 6.2, 6.3,
-//   6.6, 7.5 ms), refined ones 8 and 4 lanes (terrain 26.1, 23.1, 22.6, 23.3, 25.7 ms, decals 16.1, 14.6,
+//   local ones alone 9 (nine rooms with 2 lanes at 6, 8, 9, 10: 14.0, 12.6, 12.5, 12.3 ms) and 2 lanes (at 9
+//   blocks 1, 2, 4, 8: 13.0, 12.5, 12.3, 12.8 ms), refined ones 8 and 4 lanes (terrain 26.1, 23.1, 22.6, 23.3, 25.7 ms, decals 16.1, 14.6,
 //   14.4, 15.4, 16.9 ms).
 // From 1 M visibility items (256 K gather items) neighbouring register budgets are tried too, each on a
 // small share of the real queue's chunks with scratch counters; their results are the same levels and

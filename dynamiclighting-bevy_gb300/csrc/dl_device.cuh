@@ -283,7 +283,9 @@ __device__ __forceinline__ bool refined_candidate(const DevScene &sc, f3 o, f3 d
 // leaves, which shorten those rays' ranges and bring their lanes back: a 77 k triangle terrain's sun gather 19.6 ms
 // plain, 18.5, 18.2, 18.3 ms at 4, 8, 12; other closest hits gain nothing (burial in rooms 0.38 -> 0.42 ms,
 // photons 3.32 -> 3.39 ms), any-hit rays lose 6 %. kOneLeaf: back to inner nodes after one leaf: the sun gather's shadow
-// rays (its 18.2 -> 17.7 ms) and rays towards local lights; the sky's and the sun's lose 2 to 10 %.
+// rays (its 18.2 -> 17.7 ms), rays towards local lights and the local gather's, whose directions differ from lane to
+// lane (36 rooms' 48.8 -> 41.7 ms; holding a first leaf back until every lane has one, with votes among lanes named
+// beforehand, 48.1 ms); the sky's and the sun's lose 2 to 10 %.
 enum class NodeLoop { kPlain, kFew, kOneLeaf };
 
 template <bool COUNT>
@@ -385,68 +387,6 @@ template <bool COUNT>
 __device__ __noinline__ bool traverse_each(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack,
                                            Hit &hit, Visits *vis) {
     return traverse<false, COUNT, true, true>(sc, o, dir, max, alpha, stack, hit, vis);
-}
-
-// Any-hit traversal that holds a ray's first leaf back and goes on among inner nodes until every lane
-// there holds one (speculative traversal, Aila & Laine 2009): more lanes take part in each triangle
-// test, for nodes that a blocked ray did not need. It pays for the local gather's rays, whose
-// directions differ from lane to lane (the room grid's gather 23.3 ms without, 22.0 ms), not for aligned ones (a 77 k triangle
-// terrain's visibility 23.5 -> 24.0 ms) nor for those towards a light (rooms under panels and tubes 6.25 ->
-// 6.4 ms).
-template <bool COUNT, bool REFINE>
-__device__ __forceinline__ bool occluded_postponed(const DevScene &sc, f3 o, f3 dir, float max, bool alpha, int *stack,
-                                                   Visits *vis) {
-    if (sc.occluders == 0) return false;
-    constexpr int kNone = 0, kDone = -2147483647 - 1;  // neither is a leaf's reference
-    const f3 d{dir.x + 0.0f, dir.y + 0.0f, dir.z + 0.0f};
-    const RaySlabs slabs = ray_slabs(o, d);
-    const float tmax = fmaxf(max, 0.0f);
-    int sp = 0, ref = 0, leaf = kNone;
-    auto pop = [&]() { return sp ? stack[--sp] : kDone; };
-    auto postpone = [&]() {
-        if (ref < 0 && ref != kDone) {
-            leaf = ref;
-            ref = pop();
-        }
-    };
-    for (;;) {
-        while (ref >= 0) {
-            const NodeData nd = load_node(sc.nodes + ref);
-            if (COUNT) ++vis->nodes;
-            bool h0, h1;
-            float n0, n1;
-            slab_pair(nd.c0, nd.c1, nd.h0, nd.h1, nd.cz, nd.hz, slabs, tmax, h0, h1, n0, n1);
-            const int r0 = nd.ref0, r1 = nd.ref1;
-            if (h0 && h1) {
-                const bool swap = n1 < n0;
-                stack[sp] = swap ? r0 : r1;
-                ++sp;
-                ref = swap ? r1 : r0;
-            } else if (h0 || h1) {
-                ref = h0 ? r0 : r1;
-            } else {
-                ref = pop();
-            }
-            if (leaf == kNone) postpone();
-            if (!__any_sync(__activemask(), leaf == kNone)) break;
-        }
-        while (leaf != kNone) {
-            const uint32_t packed = (uint32_t)(~leaf), first = packed >> 3, count = packed & 7u;
-            for (uint32_t k = 0; k < count; ++k) {
-                const float4 *tp = sc.tris + (size_t)(first + k) * 3;
-                const float4 v0 = ldg4(tp);
-                if (COUNT) ++vis->tris;
-                float t, u, v, err;
-                if ((REFINE ? tri_test_refined(sc, v0, ldg4(tp + 1), ldg4(tp + 2), o, d, max, t, u, v, vis, err)
-                            : tri_test(v0, ldg4(tp + 1), ldg4(tp + 2), o, d, max, t, u, v)) &&
-                    (!alpha || alpha_blocks(sc, __float_as_uint(v0.w), u, v)))
-                    return true;
-            }
-            leaf = kNone;
-            postpone();
-        }
-        if (ref == kDone) return false;
-    }
 }
 
 template <bool COUNT = false, bool REFINE = false, NodeLoop LOOP = NodeLoop::kPlain>

@@ -192,8 +192,9 @@ struct Tracer {
     __device__ __forceinline__ bool toward_light(f3 dir, float dist) const {
         return occluded<COUNT, REFINE, QUEUED ? NodeLoop::kOneLeaf : NodeLoop::kPlain>(sc, origin, dir, dist, alpha, stack, vis);
     }
-    __device__ __forceinline__ bool postponed(f3 dir, float dist) const {
-        return occluded_postponed<COUNT, REFINE>(sc, origin, dir, dist, alpha, stack, vis);
+    // for the local gather's rays
+    __device__ __forceinline__ bool one_leaf(f3 dir, float dist) const {
+        return occluded<COUNT, REFINE, NodeLoop::kOneLeaf>(sc, origin, dir, dist, alpha, stack, vis);
     }
 };
 
@@ -576,7 +577,7 @@ __device__ __forceinline__ Contribution local_sample(const DevScene &sc, const D
     if (is_zero(pn) || distance <= 0.0f) return c;
     f3 d = divs(to_photon, distance);
     c.rays = 1;
-    if (!tr.postponed(d, distance)) {
+    if (!tr.one_leaf(d, distance)) {
         float weight = fmaxf(dot(normal, d), 0.0f) * fmaxf(dot(pn, neg(d)), 0.0f);
         f3 albedo{1.0f, 1.0f, 1.0f};
         if (sc.colored_bounce)
