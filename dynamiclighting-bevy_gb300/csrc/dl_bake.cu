@@ -2392,7 +2392,9 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
 // values that the real pass writes (OR and max, and values that it overwrites), so the trials change no
 // output. Lanes and chunks are left to the rule: on a small share the finer shapes look better than they
 // are. The wide search that this replaces took up to 0.6 s of a first bake and ended within 2 % of
-// the rule. The choice is cached per process, keyed by the device and the queue's shape.
+// the rule. The register budget that the trials picked, and nothing else, is kept per process, keyed by the device,
+// the queue's shape and the lanes, chunk and buffer that they ran with: the rest follows from each bake's
+// own samples, lights and memory cap.
 using TraceKernel = void (*)(DevScene, TraceArgs);
 struct TraceTune {
     uint32_t grab = 1, sky_lanes = 1, minb = 7, rest_minb = 7, stack_depth = kStack, trials = 0;
@@ -2428,15 +2430,21 @@ TraceKernel trace_kernel(bool count, bool refine, uint32_t minb) {
 struct TuneKey {
     int device;
     uint64_t items, sky_items, pairs, occluders, nodes;
-    uint32_t depth, flags, fixed, fixed_minb;
+    uint32_t flags, blocks_per_sm, lanes, grab, buffered;
     bool operator<(const TuneKey &o) const {
-        return std::tie(device, items, sky_items, pairs, occluders, nodes, depth, flags, fixed, fixed_minb) <
-               std::tie(o.device, o.items, o.sky_items, o.pairs, o.occluders, o.nodes, o.depth, o.flags, o.fixed,
-                        o.fixed_minb);
+        return std::tie(device, items, sky_items, pairs, occluders, nodes, flags, blocks_per_sm, lanes, grab, buffered) <
+               std::tie(o.device, o.items, o.sky_items, o.pairs, o.occluders, o.nodes, o.flags, o.blocks_per_sm, o.lanes,
+                        o.grab, o.buffered);
     }
 };
 std::mutex g_tune_lock;
-std::map<TuneKey, TraceTune> g_tune_cache;
+std::map<TuneKey, uint32_t> g_tune_cache, g_gather_cache;  // the register budget (launch bound)
+// The budget kept for a key, 0 when there is none.
+uint32_t cached_budget(const std::map<TuneKey, uint32_t> &cache, const TuneKey &key) {
+    std::lock_guard<std::mutex> guard(g_tune_lock);
+    const auto it = cache.find(key);
+    return it == cache.end() ? 0u : it->second;
+}
 
 TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_progress *progress) {
     const dl_bake_config &c = s.config;
@@ -2470,18 +2478,11 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
     const bool tune = !c.no_autotune && every && minbs.size() > 1 && !(progress && progress->cancel);
     shape_for(minbs[0]);
     if (!tune) return best;
-    TuneKey key{s.device, ta.items, ta.sky_items, ta.pairs, s.host.occ_mesh.size(), s.host.bvh_node_count,
-                best.stack_depth, (count ? 1u : 0u) | (refine ? 2u : 0u),
-                c.chunk_texels | (c.sample_lanes << 16) | (c.blocks_per_sm << 24), c.min_blocks};
-    {
-        std::lock_guard<std::mutex> guard(g_tune_lock);
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) {
-            TraceTune hit = it->second;
-            hit.trials = 0;
-            hit.ms = 0.0;
-            return hit;
-        }
+    const TuneKey key{s.device, ta.items, ta.sky_items, ta.pairs, s.host.occ_mesh.size(), s.host.bvh_node_count,
+                      0, c.blocks_per_sm, best.sky_lanes, best.grab, 0};
+    if (const uint32_t kept = cached_budget(g_tune_cache, key)) {
+        shape_for(kept);
+        return best;
     }
     cudaStream_t st = s.stream;
     Counters *scratch = s.pool.get<Counters>("tune_counters", 1);
@@ -2518,13 +2519,13 @@ TraceTune trace_tune(dl_session &s, TraceArgs ta, bool refine, bool count, dl_pr
     cudaEventDestroy(b);
     best.ms = ms_since(t0);
     std::lock_guard<std::mutex> guard(g_tune_lock);
-    g_tune_cache[key] = best;
+    g_tune_cache[key] = fastest;
     return best;
 }
 
 // The gather's shape, the same way.
 struct GatherTune {
-    uint32_t lanes = 1, minb = 6, stack_depth = kStack, blocks = 1, trials = 0, buffered = 0;
+    uint32_t lanes = 1, minb = 6, blocks = 1, trials = 0, buffered = 0;
     double ms = 0.0;
 };
 using GatherKernel = void (*)(DevScene, BounceArgs);
@@ -2567,13 +2568,11 @@ uint32_t gather_buffer(const dl_session &s) {
 float4 *gather_scratch(dl_session &s, uint32_t blocks, uint32_t lanes, uint32_t buffered) {
     return s.pool.get<float4>("gather_scratch", (size_t)blocks * (kBlock / lanes) * 2 * buffered);
 }
-std::map<TuneKey, GatherTune> g_gather_cache;
 
 GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refine, dl_progress *progress) {
     const dl_bake_config &c = s.config;
     const bool sun = gathers_suns(s);
     GatherTune best;
-    best.stack_depth = stack_depth(s);
     auto blocks_for = [&](uint32_t minb, uint32_t w) {
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gather_kernel(refine, minb, sun), kBlock,
@@ -2594,17 +2593,12 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     best.blocks = blocks_for(best.minb, best.lanes);
     if (c.no_autotune || !every || minbs.size() == 1 || (progress && progress->cancel))
         return best;
-    TuneKey key{s.device, ba.items, bpairs, 0, s.host.occ_mesh.size(), s.host.bvh_node_count, best.stack_depth,
-                refine ? 2u : 0u, c.blocks_per_sm | (c.sample_lanes << 16), c.gather_min_blocks};
-    {
-        std::lock_guard<std::mutex> guard(g_tune_lock);
-        auto it = g_gather_cache.find(key);
-        if (it != g_gather_cache.end()) {
-            GatherTune hit = it->second;
-            hit.trials = 0;
-            hit.ms = 0.0;
-            return hit;
-        }
+    const TuneKey key{s.device, ba.items, 0, bpairs, s.host.occ_mesh.size(), s.host.bvh_node_count,
+                      sun ? 1u : 0u, c.blocks_per_sm, best.lanes, 0, best.buffered};
+    if (const uint32_t kept = cached_budget(g_gather_cache, key)) {
+        best.minb = kept;
+        best.blocks = blocks_for(kept, best.lanes);
+        return best;
     }
     cudaStream_t st = s.stream;
     ba.ctr = s.pool.get<Counters>("tune_counters", 1);
@@ -2639,7 +2633,7 @@ GatherTune gather_tune(dl_session &s, BounceArgs ba, uint32_t bpairs, bool refin
     cudaEventDestroy(b);
     best.ms = ms_since(t0);
     std::lock_guard<std::mutex> guard(g_tune_lock);
-    g_gather_cache[key] = best;
+    g_gather_cache[key] = best.minb;
     return best;
 }
 
