@@ -2289,12 +2289,7 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
             occ_leaf[occ] = k;
         }
         std::vector<TravNode> nodes(h.nodes.size());
-        for (size_t i = 0; i < nodes.size(); ++i) {
-            const BvhNode &b = h.nodes[i];
-            const float lo0[3] = {b.c0[0], b.c0[2], b.c2[0]}, hi0[3] = {b.c0[1], b.c0[3], b.c2[1]};
-            const float lo1[3] = {b.c1[0], b.c1[2], b.c2[2]}, hi1[3] = {b.c1[1], b.c1[3], b.c2[3]};
-            nodes[i] = trav_node(lo0, hi0, lo1, hi1, b.ref[0], b.ref[1]);
-        }
+        for (size_t i = 0; i < nodes.size(); ++i) nodes[i] = traversal_node(h.nodes[i]);
         up(nodes.data(), nodes.size() * sizeof(TravNode), sc.nodes);
         up(h.tris.data(), h.tris.size() * 4, sc.tris);
         up(occ_leaf.data(), N * 4ull, sc.occ_leaf);
@@ -3581,15 +3576,13 @@ void payload_read(dl_session &s, uint8_t *dst) {
 // The occluder BVH's nodes with their boxes as planes, for dl_session_occluder_bvh. The device
 // holds centres and half extents, from which the planes do not follow exactly; they are minima and
 // maxima over the triangles below (padded), so they are taken again from the resident triangles,
-// children before parents (a node's index is below its children's).
-std::vector<BvhNode> plane_nodes(dl_session &s) {
+// children before parents (a node's index is below its children's). `dev`: the device's nodes.
+std::vector<BvhNode> plane_nodes(dl_session &s, const std::vector<TravNode> &dev) {
     const DevScene &sc = s.sc;
     const HostScene &h = s.host;
     const uint32_t count = h.bvh_node_count, M = sc.mesh_count;
-    std::vector<TravNode> dev(count);
     std::vector<float> tris((size_t)sc.occluders * 12);
     std::vector<uint32_t> vbase(M + 1), ibase(M + 1);
-    CK(cudaMemcpy(dev.data(), sc.nodes, count * sizeof(TravNode), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(tris.data(), sc.tris, tris.size() * 4, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(vbase.data(), sc.mesh_vertex_base, (M + 1) * 4ull, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(ibase.data(), sc.mesh_index_base, (M + 1) * 4ull, cudaMemcpyDeviceToHost));
@@ -3829,9 +3822,16 @@ dl_status dl_session_occluder_bvh(dl_session *s, void *nodes, uint64_t node_cap,
     DL_GUARD({
         CK(cudaSetDevice(s->device));
         uint64_t n = std::min<uint64_t>(node_cap, h.bvh_node_count);
-        if (n && !h.nodes.empty()) std::memcpy(nodes, h.nodes.data(), n * sizeof(BvhNode));
-        else if (n) {
-            const std::vector<BvhNode> boxes = plane_nodes(*s);
+        if (n) {
+            // the boxes come from the host; the device's nodes have to be the ones that they make
+            std::vector<TravNode> dev(h.bvh_node_count);
+            CK(cudaMemcpy(dev.data(), s->sc.nodes, dev.size() * sizeof(TravNode), cudaMemcpyDeviceToHost));
+            const std::vector<BvhNode> boxes = h.nodes.empty() ? plane_nodes(*s, dev) : h.nodes;
+            const size_t bad = first_unlike(boxes.data(), dev.data(), dev.size());
+            if (bad < dev.size()) {
+                g_error = "occluder BVH node " + std::to_string(bad) + " of the device does not hold its triangles' boxes";
+                return DL_CUDA_ERROR;
+            }
             std::memcpy(nodes, boxes.data(), n * sizeof(BvhNode));
         }
         uint64_t t = std::min<uint64_t>(tri_cap, s->sc.occluders);

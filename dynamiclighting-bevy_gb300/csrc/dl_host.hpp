@@ -5,11 +5,13 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <vector>
 
 #include "../../include/dynlight.h"
 #include "dl_math.cuh"
+#include "dl_slab.hpp"
 
 namespace dl {
 
@@ -55,6 +57,25 @@ struct BvhNode {
     int32_t ref[2];
     uint32_t count[2];
 };
+// The node that the traversal reads for it.
+inline TravNode traversal_node(const BvhNode &b) {
+    const float lo0[3] = {b.c0[0], b.c0[2], b.c2[0]}, hi0[3] = {b.c0[1], b.c0[3], b.c2[1]};
+    const float lo1[3] = {b.c1[0], b.c1[2], b.c2[2]}, hi1[3] = {b.c1[1], b.c1[3], b.c2[3]};
+    return trav_node(lo0, hi0, lo1, hi1, b.ref[0], b.ref[1]);
+}
+// The first of `count` nodes whose traversal node is not the one given, bit for bit (any NaN for a NaN: a
+// coordinate beyond binary32's range leaves one, whose bits differ between host and device); `count`: none.
+inline size_t first_unlike(const BvhNode *boxes, const TravNode *held, size_t count) {
+    auto same = [](float x, float y) { return std::memcmp(&x, &y, 4) == 0 || (x != x && y != y); };
+    for (size_t i = 0; i < count; ++i) {
+        const TravNode want = traversal_node(boxes[i]), &got = held[i];
+        bool all = want.ref[0] == got.ref[0] && want.ref[1] == got.ref[1];
+        for (int k = 0; k < 4; ++k)
+            all = all && same(want.cxy[k], got.cxy[k]) && same(want.hxy[k], got.hxy[k]) && same(want.z[k], got.z[k]);
+        if (!all) return i;
+    }
+    return count;
+}
 
 struct HostScene {
     std::vector<const dl_mesh *> meshes;      // sorted by id

@@ -379,10 +379,11 @@ dl_status dl_session_encode_payload(dl_session *session, uint8_t **bytes, uint64
 dl_status dl_session_payload_build(dl_session *session, uint64_t *length, uint32_t *crc);
 dl_status dl_session_payload_read(dl_session *session, uint8_t *bytes, uint64_t length);
 /* No counterpart in the reference (whose occluder BVH is internal to Occluders,
-   src/bake/occluder.rs:63-114): a copy of the session's occluder BVH as the traversal reads it —
-   up to `node_cap` 64-byte nodes (child boxes c0, c1, c2 as 12 floats, then the two child
-   references as int32: >= 0 an inner node, < 0 a leaf ~(first << 3 | count), ~0 empty, then two
-   zero words) and up to `tri_cap` triangles in leaf order (12 floats: v0 with the occluder index's
+   src/bake/occluder.rs:63-114): the session's occluder BVH — up to `node_cap` 64-byte nodes (child
+   boxes c0, c1, c2 as 12 floats, then the two child references as int32: >= 0 an inner node, < 0 a
+   leaf ~(first << 3 | count), ~0 empty, then two zero words; the device holds each box as centre
+   and half extent, and the call fails with DL_CUDA_ERROR unless every node it holds is, bit for bit,
+   the one that these boxes and references make) and up to `tri_cap` triangles in leaf order (12 floats: v0 with the occluder index's
    bits in the fourth, e1 and e2 with a zero fourth). `*node_count` and `*depth` (the deepest
    level, the root being 1) are set either way. For tests and tools. */
 dl_status dl_session_occluder_bvh(dl_session *session, void *nodes, uint64_t node_cap, float *triangles,
