@@ -316,8 +316,10 @@ constexpr float kPio2F3 = 6.223371969669989e-14f;  // 0x1.184698p-44
 // sin and cos of k pi/128 + r, |r| <= pi/256, from a table of sin and cos at the 256 multiples of
 // pi/128 (as binary32 pairs) and short series in r (table-driven reduction, Tang 1989, with Gal's idea of
 // keeping the table's low words): sin = S + C sin r - S (1 - cos r), cos = C - S sin r - C (1 - cos r).
-// The series' terms beyond r and r^2/2 are below 2^-21 of the result, so plain binary32 carries them to
-// 2^-37.5 of it; everything else is summed without error or in the low words. About 90 operations for
+// The series' terms beyond r and r^2/2 are below 2^-15 of the result and carried in plain binary32, everything
+// else without error or in the low words. The sums are within 2^-36.92 of the value over every argument up to 16
+// (tests/native/sincos_table_check.cpp, all of them once, a sample in every run), where the rounding test allows
+// 2^-36; it leaves one argument in 2000 to the binary64 path. About 90 operations for
 // both against 250 for the double-float series above, which it replaces; the same rounding test follows.
 // On the device the rooms' local gather (two sines, a cosine and three more sines a sample) went from
 // 67.3 ms to 55.7 ms, the outdoor visibility stage (one of each a ray) from 123.6 ms to 119.5 ms.
@@ -372,8 +374,9 @@ DL_HD SinCosEntry sincos_entry(int k) {
     return kSinCosHost.at[k & 255];
 #endif
 }
-// pi/128 as C1 + C2 + C3 in binary32. C1 is a multiple of 2^-29, as every |x| < 16 that is not itself
-// below the first half step is, so x - k C1 is exact in one multiply-add.
+// pi/128 as C1 + C2 + C3 in binary32. x - k C1 is exact in one multiply-add: for |x| >= 2^-6 both are multiples of
+// 2^-29 and their difference is below 2^-6; below that k is 0, or 1 with x between C1 / 2 and C1, whose
+// difference is exact too (Sterbenz).
 constexpr float kStepC1 = 0.024543693f;     // 0x1.921fb6p-6
 constexpr float kStepC2 = -6.8299044e-10f;  // -0x1.777a5cp-31
 constexpr float kStepC3 = -2.679882e-17f;   // -0x1.ee59dap-56
