@@ -2956,7 +2956,8 @@ dl_status run(dl_session &s, dl_progress *progress) {
         // The two kernels claim from heads of their own, so they run side by side: blocks of one take the
         // SMs that the other's last blocks leave (a 77 k triangle terrain 24.1 -> 23.4 ms, foliage 2.58 -> 1.95 ms).
         // Launched directly: a graph of these nodes saves nothing and cost a one-off bake its instantiation.
-        const bool fork = tune.sky && tune.rest;
+        // One after the other where a caller bounds the persistent blocks per SM: the bound holds for both together.
+        const bool fork = tune.sky && tune.rest && !s.config.blocks_per_sm;
         if (fork) {
             if (!s.branch) {
                 CK(cudaStreamCreateWithFlags(&s.branch, cudaStreamNonBlocking));
