@@ -60,25 +60,16 @@ __device__ __forceinline__ void add_retests(Counters *ctr, unsigned long long n)
 
 // ================================ sample order tables ====================================
 
-// The sample orders of DevScene (`orders`, `order_cells`, `cell_samples`) for n = 16, 32, ...,
-// kMaxOrdered, a thread per sample: the first n points of the (0, 2)-sequence hold one point in each cell of
-// a 2^ceil(m/2) x 2^floor(m/2) grid (n = 2^m), so sample j's rank in the cells' Morton order is the
-// Morton code of its cell: what sky_sample_order and sample_cells (dl_host.hpp) find by sorting. On the
-// host that took 0.7 ms of every session, a fifth of the smallest bake.
-__device__ __forceinline__ uint32_t spread_bits(uint32_t v) {  // bit i of a byte to bit 2i
-    v = (v | v << 4) & 0x0F0Fu;
-    v = (v | v << 2) & 0x3333u;
-    return (v | v << 1) & 0x5555u;
-}
-__global__ void k_sample_tables(uint16_t *orders, uint16_t *cells, uint16_t *samples) {
+// The tables of shifted_sample (DevScene's `order_cells`, `cell_samples`) for n = 16, 32, ..., kMaxOrdered, a
+// thread per sample: what sample_cells (dl_host.hpp) finds by sorting. On the host that took 0.7 ms of every
+// session, a fifth of the smallest bake.
+__global__ void k_sample_tables(uint16_t *cells, uint16_t *samples) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x + 16;
     if (i >= 2 * kMaxOrdered) return;
-    const uint32_t m = 31 - __clz(i), n = 1u << m, j = i - n, base = n - 16, xb = (m + 1) / 2, yb = m / 2;
-    const uint32_t cx = rev_bits(j) >> (32 - xb), cy = sobol2(j) >> (32 - yb);
-    const uint32_t rank = spread_bits(cx) | spread_bits(cy) << 1;
-    orders[base + rank] = (uint16_t)j;
-    cells[base + rank] = (uint16_t)(cx | cy << 8);
-    samples[base + (cy << xb | cx)] = (uint16_t)j;
+    const uint32_t m = 31 - __clz(i), n = 1u << m, j = i - n, base = n - 16;
+    const NetCell c = net_cell(j, m);
+    cells[base + c.rank] = (uint16_t)(c.x | c.y << 8);
+    samples[base + (c.y << ((m + 1) / 2) | c.x)] = (uint16_t)j;
 }
 
 // ================================ setup and association ==================================
@@ -2330,19 +2321,15 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
     sc.area_min_samples = o->area_light_min_samples;
     sc.sky_samples = o->sky_samples;
     constexpr uint32_t kTable = 2 * kMaxOrdered - 16;
-    uint16_t *tables = dev_alloc<uint16_t>(s->owned, s->stream, 3 * kTable, bytes, &s->budget);
-    k_sample_tables<<<grid_for(kTable), kBlock, 0, s->stream>>>(tables, tables + kTable, tables + 2 * kTable);
+    uint16_t *tables = dev_alloc<uint16_t>(s->owned, s->stream, 2 * kTable, bytes, &s->budget);
+    k_sample_tables<<<grid_for(kTable), kBlock, 0, s->stream>>>(tables, tables + kTable);
     LAUNCHED("k_sample_tables");
-    sc.orders = tables;
-    sc.order_cells = tables + kTable;
-    sc.cell_samples = tables + 2 * kTable;
+    sc.order_cells = tables;
+    sc.cell_samples = tables + kTable;
     sc.sky_order = nullptr;
-    std::vector<uint16_t> sky_order;  // beyond the tables; its upload ends before this returns
-    const uint32_t sky = o->sky_samples;
-    if (sky >= 16 && sky <= kMaxOrdered && !(sky & (sky - 1))) {
-        sc.sky_order = sc.orders + (sky - 16);
-    } else if (sky > kMaxOrdered) {
-        sky_order = sky_sample_order(sky);
+    std::vector<uint16_t> sky_order;  // for counts beyond the tables; its upload ends before this returns
+    if (o->sky_samples > kMaxOrdered) {
+        sky_order = sky_sample_order(o->sky_samples);
         if (!sky_order.empty()) up(sky_order.data(), sky_order.size() * 2, sc.sky_order);
     }
     sc.colored_bounce = o->colored_bounce;

@@ -48,11 +48,9 @@ struct DevScene {
     uint32_t colored_bounce;
     // refined form: the epsilon of the binary64 re-test and its square
     float refine_eps, refine_eps2;
-    // coherent sample orders (sky_sample_order) for n = 16, 32, ..., kMaxOrdered back to back
-    // (the table of n starts at n - 16); sky_order is the sky's, or null
-    const uint16_t *orders;
+    // the coherent order (sky_sample_order) of a sky count beyond kMaxOrdered, or null
     const uint16_t *sky_order;
-    // sample_cells (dl_host.hpp) for the same n, laid out like `orders`
+    // sample_cells (dl_host.hpp) for n = 16, 32, ..., kMaxOrdered back to back (n's start at n - 16)
     const uint16_t *order_cells, *cell_samples;
 };
 constexpr uint32_t kMaxOrdered = 4096;

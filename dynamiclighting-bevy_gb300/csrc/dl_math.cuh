@@ -578,6 +578,20 @@ DL_HD uint32_t sobol2(uint32_t index) {
     x ^= (x >> 16) & 0x0000FFFFu;
     return rev_bits(x);
 }
+// Sample j of the net of the sequence's first 2^m points (m from 4 to 16): its cell in a grid of 2^ceil(m/2) x
+// 2^floor(m/2), which holds no other of them, and the cell's rank in the grid's Morton order.
+struct NetCell {
+    uint32_t x, y, rank;
+};
+DL_HD uint32_t spread_bits(uint32_t v) {  // bit i of a byte to bit 2i
+    v = (v | v << 4) & 0x0F0Fu;
+    v = (v | v << 2) & 0x3333u;
+    return (v | v << 1) & 0x5555u;
+}
+DL_HD NetCell net_cell(uint32_t j, uint32_t m) {
+    const uint32_t x = rev_bits(j) >> (32 - (m + 1) / 2), y = sobol2(j) >> (32 - m / 2);
+    return NetCell{x, y, spread_bits(x) | spread_bits(y) << 1};
+}
 DL_HD float unit24(uint32_t bits) { return (float)(bits >> 8) / 16777216.0f; }
 DL_HD f2 spread(uint32_t index, f2 off, bool rect) {
     float across = unit24(rev_bits(index));
