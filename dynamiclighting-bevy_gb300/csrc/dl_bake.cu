@@ -2191,9 +2191,10 @@ dl_status create(const dl_bake_input *in, const dl_bake_options *o, const dl_bak
     };
     {
         // meshes split into contiguous runs of about equal vertex and index counts, one per thread
-        // (starting threads costs more than flattening a small scene)
+        // (starting threads costs more than flattening a small scene: upload with one thread and with 16, at 356 K
+        // vertices and indices 0.28 and 0.44 ms, at 722 K 0.50 and 0.50 ms, at 1.04 M 0.69 and 0.54 ms)
         const unsigned cores = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-        const unsigned hw = (uint64_t)V + I < (1u << 17) ? 1u : cores;
+        const unsigned hw = (uint64_t)V + I < (3u << 18) ? 1u : cores;
         const uint64_t per = ((uint64_t)V + I) / hw + 1;
         std::vector<uint32_t> cut{0};
         uint64_t acc = 0;
