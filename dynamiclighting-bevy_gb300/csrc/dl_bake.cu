@@ -1,6 +1,6 @@
 // The bake pipeline on one GPU and the C ABI (include/dynlight.h).
 //
-// Stages, all on one stream, each a kernel over the whole scene (every mesh at once):
+// Stages, on one stream (the queue's two kernels on two), each a kernel over the whole scene (every mesh at once):
 //   setup      per triangle: face normal, crop rect, light association (mesh_bake.rs:141-173)
 //   regions    per (mesh, light): union of crop rects -> one shadow grid (mesh_bake.rs:175-192)
 //   texels     per triangle: owned grid, centered + touched texels (texels.rs, mesh_texels.rs)
@@ -587,7 +587,7 @@ __global__ void k_pair_scatter(const unsigned long long *flag, const unsigned lo
     const uint32_t sky = (uint32_t)at, soft = (uint32_t)(at >> 32);
     order[f == 1 ? sky : f ? skies + soft : skies + softs + (p - sky - soft)] = p;
 }
-// The queue's items and, of them, the sky's (sizes[1], sizes[2]) from the sky pairs' count in sizes[0].
+// The queue's items and, of them, the sky's (sizes[2], sizes[3]) from the sky pairs' count in sizes[0].
 __global__ void k_queue_sizes(const uint32_t *item_off, uint32_t pairs, uint32_t *sizes) {
     const uint32_t items = item_off[pairs], sky_items = item_off[sizes[0]];
     sizes[2] = items;
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(kBlock) k_sun_map(DevScene sc, SunMapArgs a, C
 // the axis, each a closest hit (a hit at distance 0 counts as none); the open share and the rays
 // that reached a triangle's back, both counts, so the lanes' samples add up in any order. One lane a
 // job left the chip a few thousand threads of 64 to 256 rays each: a room's 3087 probes took 394 us,
-// with 8 lanes 117 us.
+// with 8 lanes 117 us (all maps of that room with 4, 8, 16 lanes: 193, 163, 157 us).
 struct ProbeArgs {
     f3 origin;
     float spacing;
@@ -1940,7 +1940,8 @@ T read_back(dl_session &s, const T *p) {
 unsigned grid_for(size_t n, unsigned block = kBlock) { return (unsigned)std::max<size_t>(1, (n + block - 1) / block); }
 // Grid of `jobs` jobs of `threads` threads each, with parts (second dimension) while the jobs alone
 // leave the chip short of warps: up to kParts, aiming at kPartThreads threads (a few times what
-// the SMs hold: parts of jobs that turn out small end at once).
+// the SMs hold: parts of jobs that turn out small end at once). The stages that use it, at 2^18, 2^20, 2^22: a
+// room under every light 0.41, 0.38, 0.38 ms, a terrain tile 0.86, 0.88, 0.98 ms, foliage 0.50, 0.53, 0.67 ms.
 // Most (mesh, light) entries have no region: for them the parts are counted as if a warp took an entry.
 constexpr size_t kParts = 64, kPartThreads = 1u << 20;
 dim3 grid_parts(size_t jobs, unsigned threads = 32, unsigned block = kBlock) {
@@ -2546,8 +2547,7 @@ uint32_t gather_buffer(const dl_session &s) {
         }
     return most;
 }
-// The lane groups' scratch of a gather launch (2 float4 per held sample per group), from the
-// session's pool: the largest launch (one lane per group) sizes it once.
+// The lane groups' scratch of a gather launch (2 float4 per held sample per group), from the session's pool.
 float4 *gather_scratch(dl_session &s, uint32_t blocks, uint32_t lanes, uint32_t buffered) {
     return s.pool.get<float4>("gather_scratch", (size_t)blocks * (kBlock / lanes) * 2 * buffered);
 }
@@ -3494,8 +3494,10 @@ void payload_build(dl_session &s, HostResult &r, uint64_t &length, uint32_t &crc
 // Copies the built payload into `dst` (pageable host memory, in general not touched before). The
 // host's cores share it, each in pieces through its own pinned buffer: the SMs write a piece over
 // the CPU-GPU link while the core copies the previous one on. Bound by the cores' page faults and
-// copies; one core behind the driver's staging copy, and a second copy into the caller's object, took
-// 71 ms for the outdoor level's 505 MB, this takes 14 ms (terrain), rooms 4.3 ms and 0.9 ms (20 MB).
+// copies (the link alone moves the level's 505 MB in 2.6 ms); one core behind the driver's staging copy, and a
+// second copy into the caller's object, took 71 ms for them, this takes 12 to 14 ms, 2.5 ms for the rooms' 68 MB
+// (was 12 ms), 0.7 ms for 20 MB. kPiece also sets how many cores take part; at 128 K, 512 K, 2 M words: 505 MB
+// 12.0, 11.7, 12.0 ms, 68 MB 2.4, 2.4, 2.6 ms, 20 MB 1.2, 0.7, 1.1 ms.
 void payload_read(dl_session &s, uint8_t *dst) {
     constexpr uint64_t kPiece = 512 * 1024;  // words
     const uint64_t words = s.payload_words;
@@ -3990,7 +3992,7 @@ constexpr uint32_t kNoallocMaxTexels = DL_NOALLOC_MAX_TEXELS;
 
 namespace {
 
-constexpr int kNoallocDevices = 64;
+constexpr int kNoallocDevices = 64;  // devices beyond are refused, as they always were
 
 // A block filters a tile of the window (filter_tile).
 __global__ void __launch_bounds__(kTileThreads) k_noalloc_filter(const float *in, float *out, int w, int h, int4 clamp,

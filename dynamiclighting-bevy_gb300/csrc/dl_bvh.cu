@@ -30,7 +30,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kChunk = 4096;     // positions per block in the large-node kernels
-constexpr uint32_t kSmall = 512;      // nodes up to this size are built whole by one warp
+constexpr uint32_t kSmall = 512;      // nodes up to this size are built whole by one block
 static_assert(kSmall <= 65536, "a small subtree's positions are 16-bit");
 constexpr int kBinWords = 3 * kBvhBins * 7;  // per (axis, bin): count, lo xyz, hi xyz
 
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kThreads) k_level_copy(State st, Level lv) {
     for (uint32_t p = b + threadIdx.x; p < e; p += blockDim.x) st.idx[p] = st.tmp[p];
 }
 
-// ---- small nodes: a warp per subtree -------------------------------------------------------
+// ---- small nodes: a block per subtree ------------------------------------------------------
 
 // bvh_best_split over the bins images `sb` by a whole warp: lane k < kBvhBins of each used axis
 // holds bin k, shuffle scans give the exact unions left of and right of every split, and the
@@ -489,7 +489,9 @@ __device__ void warp_best_split(const int *sb, const bool use[3], float &best_co
 // in global memory took 155 us for 72 triangles and 1167 us for subtrees of 512; this takes 50 us and
 // 200 us.
 constexpr int kSmallWarps = 8;
-constexpr uint32_t kDirect = 16;  // primitives up to which a node's splits are evaluated directly
+// Primitives up to which a node's splits are evaluated directly. The whole build with 2 (never), 8, 16, 32: outdoor
+// level 2.66, 2.58, 2.57, 2.61 ms, terrain tile 1.10, 1.08, 1.07, 1.08 ms, rooms 1.28, 1.27, 1.26, 1.27 ms.
+constexpr uint32_t kDirect = 16;
 struct SmallTree {
     float box[9][kSmall];  // lo xyz, hi xyz, centroid xyz
     uint32_t item[kSmall];  // occluder

@@ -56,7 +56,10 @@ struct DevScene {
 constexpr uint32_t kMaxOrdered = 4096;
 // The net that n samples are traced in the coherent order of: n itself when it is a power of two, else
 // the next one, as long as n fills five eighths of it (a lane idles where the order's sample is n or
-// more); 0: no such net. The first n points of the sequence are the first n of any larger net.
+// more); 0: no such net. The first n points of the sequence are the first n of any larger net. Where the line
+// lies, on a 77 k triangle terrain: sky samples 144, 160, 176, 192 in the net of 256 20.3, 20.7, 21.1, 21.6 ms, in
+// index order 19.3, 21.3, 23.3, 25.3 ms; sun bounces of 72, 80, 88, 96 in the net of 128 14.4, 14.9, 15.4, 15.9 ms, in
+// index order 14.3, 15.9, 17.5, 19.1 ms.
 __host__ __device__ __forceinline__ uint32_t ordered_net(uint32_t n, uint32_t least, uint32_t most) {
     uint32_t net = least;
     while (net < n && net < most) net *= 2;

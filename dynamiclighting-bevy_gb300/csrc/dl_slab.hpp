@@ -3,7 +3,7 @@
 // A box is stored as centre and half extent per axis. On one axis the ray meets the slab around
 // t_c = (c - o) / d at t_c -+ h / |d|, so near and far come out of two multiply-adds with no
 // minimum and maximum of the two planes' distances: a node's test is 9 packed (two at a time)
-// multiply-adds and 8 three-input minima and maxima, where the plane form needs 12 multiply-adds
+// multiply-adds, 4 three-input and 4 two-input minima and maxima, where the plane form needs 12 multiply-adds
 // and 24 minima and maxima. The traversal is bound by instruction issue and, within that, by the
 // integer/comparison pipe, which runs minima and maxima at half the multiply-adds' rate (ncu on the
 // quarter-size outdoor case with the plane form: issue slots 83 % busy, that pipe 55 %, the

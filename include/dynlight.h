@@ -170,7 +170,8 @@ typedef struct dl_bake_config {
     uint32_t chunk_texels;     /* (pair, texel) items a warp claims from the queue at once, 0: by rule */
     uint32_t sample_lanes;     /* lanes sharing one texel's sky samples and bounce-gather samples
                                   (1, 2, 4, 8, 16 or 32), 0: by rule */
-    uint32_t blocks_per_sm;    /* upper bound of persistent blocks per SM, 0: as many as fit */
+    uint32_t blocks_per_sm;    /* upper bound of persistent blocks per SM, 0: as many as fit (with a
+                                  bound the visibility's two kernels run one after the other) */
     uint32_t count_visits;     /* 1: run the instrumented visibility kernel that counts BVH node
                                   visits and triangle tests (for roofline accounting; slower) */
     float refine_epsilon;      /* DL_FORM_REFINED: re-test margin (barycentric units; times
@@ -183,7 +184,10 @@ typedef struct dl_bake_config {
     uint32_t max_device_mib;   /* cap on the device memory one bake (session) may hold, in MiB:
                                   scene, BVH and its build scratch, every stage's buffers. An
                                   allocation past it fails the call with DL_OUT_OF_MEMORY and
-                                  frees what the bake held. 0: no cap */
+                                  frees what the bake held. 0: no cap. Not in it: what the CUDA
+                                  context holds, among it the kernels' local memory (traversal
+                                  stacks of 256 bytes and spills for every thread that the GPU
+                                  can hold, 80 MB and more on a GB300, taken at their first launch) */
     uint32_t min_blocks;       /* register budget of the bit-exact visibility kernel, as the
                                   blocks of 128 threads per SM it is compiled to fit: 7, 8, 9, 10
                                   or 12 (72, 64, 56, 48 or 40 registers per thread), 0: by rule (and
@@ -225,7 +229,8 @@ typedef struct dl_bake_report {
                                  leaves open, and each closest hit) */
     /* launch shape of the batched visibility (rule, trials or config): the sky's kernel where the
        scene has one */
-    uint32_t tuned_chunk_texels, tuned_sample_lanes, tuned_blocks_per_sm, tuned_stack_depth;
+    uint32_t tuned_chunk_texels, tuned_sample_lanes, tuned_blocks_per_sm;
+    uint32_t tuned_stack_depth; /* stack entries that the tree needs, rounded up to 4 (at least 8) */
     uint32_t tuned_min_blocks;  /* launch bound: blocks per SM the registers were sized for */
     uint32_t tune_trials;       /* candidate shapes timed in this run (0: defaults or cached) */
     double ms_tune;             /* host time of those trials */
