@@ -421,7 +421,7 @@ def main():
                      "l1_read_gbs": l1_gbs.value, "hbm_gbs": hbm, "hbm_source": f"{peak_kind} (MEASURED_PEAKS.json)",
                      "traffic": traffic, "traffic_frac_of_algorithmic": traffic / alg_bytes if traffic else None,
                      "limiter": "instruction issue and L1 return (ncu on the quarter-size outdoor case: issue slots "
-                                "76 % busy, L1 data pipe 72 %, SIMT efficiency 47 %, L2 throughput 6 % of peak)",
+                                "76 % busy, L1 data pipe 72 %, SIMT efficiency 49 %, L2 throughput 5 % of peak)",
                      "algorithmic_bytes_per_launch": int(alg_bytes),
                      "bytes_per_unit": "64 per node visit + 48 per triangle test + 76 per (pair, texel) item",
                      "node_visits": int(crep.node_visits), "tri_tests": int(crep.tri_tests),
